@@ -267,11 +267,48 @@ template <typename T> struct ZParams {
   const typename Vec2<T>::type *stab;  // [m][nrad] (value, slope) of beta/eps0 s_i, or null
   const typename Cx<T>::type *L;       // [N2][N1][Nhp] long-range field / h^3, or null
   const typename Cx<T>::type *chi3;    // chi - 1 on the k grid [m(m+1)/2][N2][N1][Nhp], or null
+  const T *kt;                         // chi - 1 on the octant of the k grid (k_octant) [m(m+1)/2][oct], or null
+  const T *ks;                         // beta/eps0 s_i on the octant [m][oct], or null
+  long long oct;                       // (N1/2 + 1) (N2/2 + 1) oct_row(g)
   int nrad;
   double dkr;                          // pi / rmax
   T a[kMaxSites];                      // c_j -= a_j L      (no-renorm: beta q_j)
   T bconst[kMaxSites];                 // t_i -= bconst_i L (no-renorm: beta q_i)
 };
+
+// Row stride of the octant tables: whole 8-column blocks, so that a tile's
+// rows are 32-byte aligned and need no bounds check (the padding holds 0).
+__host__ __device__ __forceinline__ int oct_row(const Geo &g) { return (g.Nh + 7) & ~7; }
+
+// A radial table on the k grid: out[q][|ky|][|kz|][kx] = table q at |k|, by the
+// interpolation rule of the passes (nearest entry plus slope, in T).  |k| only
+// depends on |ky| and |kz|, so the octant 0 <= ky <= N1/2, 0 <= kz <= N2/2
+// holds every value of the half spectrum.  The shape-specialised z passes read
+// it in place of the FP64 square root and division and the gathered pairs that
+// the rule takes at every point: alone that changed nothing (their time was
+// barriers), but a tile's values become rows that can be staged beside it.
+// 54 MB per FP32 context at 256^3, m = 3.
+template <typename T>
+__global__ void __launch_bounds__(256) k_octant(Geo g, const typename Vec2<T>::type *__restrict__ tab, int ntab, int nrad,
+                                                double dkr, T *__restrict__ out) {
+  const int H1 = g.N1 / 2 + 1, H2 = g.N2 / 2 + 1;
+  const int OR = oct_row(g);
+  const long long oct = (long long)H1 * H2 * OR;
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= oct) return;
+  const int kx = (int)(e % OR);
+  const int kz = (int)((e / OR) % H2), ky = (int)(e / ((long long)OR * H2));
+  const double k0 = kx * g.dk0, k1 = ky * g.dk1, k2 = kz * g.dk2;
+  const double kk = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(k0, k0), __dmul_rn(k1, k1)), __dmul_rn(k2, k2)));
+  const double ix = kk / dkr - 0.5;
+  int i = (int)(ix + 0.5);
+  i = min(max(i, 0), nrad - 1);
+  const T fr = T(ix - i);
+  for (int q = 0; q < ntab; ++q) {
+    const typename Vec2<T>::type t = tab[(long long)q * nrad + i];
+    out[q * oct + e] = kx < g.Nh ? t.x + t.y * fr : T(0);
+  }
+}
 
 // z pass: forward transform along z of all m sites, OZ contraction with the
 // radial chi-1 tables (+ long-range terms in MODE_F), inverse along z.

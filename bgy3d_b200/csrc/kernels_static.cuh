@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(Split<N>::R1 * B) k_y_s(Geo g, const __grid_co
   }
 }
 
-// Elements whose chi table entries a thread has in flight during the z
+// Row pairs whose chi - 1 values a thread has in flight during the z
 // contraction: 4 in the FP32 Jacobian pass, 2 where the residual's
 // long-range terms or FP64 values take the registers (the FP32 passes stay
 // within 128 registers, i.e. the 4 CTAs per SM that shared memory allows).
@@ -281,63 +281,93 @@ template <typename T, int MODE> __host__ __device__ constexpr int zpf_default() 
 }
 
 // One z tile in shared memory: forward transform along z of the m [N][B]
-// site columns, the OZ contraction with the radial chi-1 tables (+ the
-// long-range terms in MODE_F), inverse transform; ends after a barrier.
-// Run by the NTHR = R1 B threads tid of a group (act false: barriers only);
-// JOINT: the MS site tiles (all allocated) transform as one MS B-column
-// tile by R1 B MS threads.
+// site columns, the OZ contraction with chi - 1 (+ the long-range terms in
+// MODE_F), inverse transform; ends after a barrier.  Run by the NTHR = R1 B
+// threads tid of a group (act false: barriers only); JOINT: the MS site
+// tiles (all allocated) transform as one MS B-column tile by R1 B MS threads.
 //
-// The contraction is software-pipelined: the table entries of an element
-// depend only on where it sits on the k grid, so a thread keeps those of its
-// next ZPF elements (and, in MODE_F, their long-range values) in flight
+// chi - 1 comes from the octant table (k_octant): rows z and N - z of a
+// column share its values, so a thread contracts both on one set of loads
+// (row 0 is paired with row N / 2, which has values of its own).  The loads
+// depend only on where the row sits on the k grid, so a thread keeps those of
+// its next ZPF row pairs (and, in MODE_F, their long-range values) in flight
 // while it contracts the current one, and issues the first ZPF before the
-// forward transforms, under whose latency they arrive.  Same arithmetic in
-// the same order as contracting element by element.
+// forward transforms, under whose latency they arrive.  Same arithmetic as
+// the rule evaluated at every element.
 template <typename T, int MODE, int N, int B, int MS, bool JOINT = false, int ZPF = zpf_default<T, MODE>(),
           class S = Split<N>>
 __device__ __forceinline__ void z_tile_g(const Geo &g, typename Cx<T>::type *buf, const typename Cx<T>::type *tw,
                                          const ZParams<T> &zp, int kx0, int y, int tid, bool act) {
   using V = typename Cx<T>::type;
-  using P2 = typename Vec2<T>::type;
   constexpr int NTHR = S::R1 * B * (JOINT ? MS : 1);
   constexpr int NP = MS * (MS + 1) / 2;
-  constexpr int NIT = (N * B + NTHR - 1) / NTHR;
+  constexpr int H = N / 2;
+  static_assert(N % 2 == 0, "rows pair up as (z, N - z)");
+  constexpr int NIT = (H * B + NTHR - 1) / NTHR;
   constexpr int D = NIT < ZPF ? NIT : ZPF;
   const int m = g.m;
   const int np = m * (m + 1) / 2;
   const int bw = min(B, g.Nh - kx0);
   const bool full = MODE == MODE_F && zp.L != nullptr;
-  const int ky = kfreq(y, g.N1);
-  const double k1 = ky * g.dk1;
   const long long zstride = (long long)g.N1 * g.Nhp;
   const long long col = (long long)y * g.Nhp + kx0;
-  P2 tq[D][NP];   // chi - 1 (value, slope) of each pair
-  P2 sq[D][MS];   // beta/eps0 s_i (value, slope), MODE_F
-  V lq[D];        // long-range value, MODE_F
-  T fq[D];        // interpolation fraction
-  auto fetch = [&](int it, int slot) {
-    const int e = tid + it * NTHR;
-    if (!act || e >= N * B) return;
-    const int z = e / B, b = e % B;
-    const int kx = kx0 + b;
-    const int kz = kfreq(z, N);
-    const double k0 = kx * g.dk0, k2 = kz * g.dk2;
-    const double kk = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(k0, k0), __dmul_rn(k1, k1)), __dmul_rn(k2, k2)));
-    const double ix = kk / zp.dkr - 0.5;
-    int i = (int)(ix + 0.5);
-    i = min(max(i, 0), zp.nrad - 1);
-    fq[slot] = T(ix - i);
+  const int OR = oct_row(g);
+  const long long orow = (long long)(y <= g.N1 / 2 ? y : g.N1 - y) * (H + 1) * OR + kx0;  // octant row kz = 0
+  T tq[D][NP];     // chi - 1 of each pair
+  T sq[D][MS];     // beta/eps0 s_i, MODE_F
+  V lq[D][2];      // long-range values of rows z and N - z, MODE_F
+  auto load = [&](int r, int b, T *tv, T *sv) {
+    const long long o = orow + (long long)r * OR + b;
 #pragma unroll
     for (int q = 0; q < NP; ++q)
-      if (q < np) tq[slot][q] = __ldg(&zp.chi[(long long)q * zp.nrad + i]);
-    lq[slot].x = T(0); lq[slot].y = T(0);
-    if (full) {
-      if (zp.stab != nullptr) {
+      if (q < np) tv[q] = __ldg(&zp.kt[q * zp.oct + o]);
+    if (full && zp.ks != nullptr) {
 #pragma unroll
-        for (int ii = 0; ii < MS; ++ii)
-          if (ii < m) sq[slot][ii] = __ldg(&zp.stab[(long long)ii * zp.nrad + i]);
+      for (int ii = 0; ii < MS; ++ii)
+        if (ii < m) sv[ii] = __ldg(&zp.ks[ii * zp.oct + o]);
+    }
+  };
+  auto fetch = [&](int it, int slot) {
+    const int e = tid + it * NTHR;
+    const int r = e / B, b = e % B;
+    if (!act || e >= H * B || b >= bw) return;
+    load(r, b, tq[slot], sq[slot]);
+    if (full) {
+      lq[slot][0] = __ldg(&zp.L[r * zstride + col + b]);
+      lq[slot][1] = __ldg(&zp.L[(r == 0 ? H : N - r) * zstride + col + b]);
+    }
+  };
+  auto contract = [&](int e, const T *xv, const T *sv, V Lk) {
+    V c[MS];
+#pragma unroll
+    for (int j = 0; j < MS; ++j)
+      if (j < m) c[j] = buf[j * N * B + e];
+    if (full) {
+#pragma unroll
+      for (int j = 0; j < MS; ++j)
+        if (j < m) { c[j].x -= zp.a[j] * Lk.x; c[j].y -= zp.a[j] * Lk.y; }
+    }
+#pragma unroll
+    for (int ii = 0; ii < MS; ++ii) {
+      if (ii < m) {
+        V t;
+        t.x = T(0); t.y = T(0);
+#pragma unroll
+        for (int j = 0; j < MS; ++j) {
+          if (j < m) {
+            const T x = xv[ii >= j ? ii * (ii + 1) / 2 + j : j * (j + 1) / 2 + ii];
+            t.x += x * c[j].x;
+            t.y += x * c[j].y;
+          }
+        }
+        if (full) {
+          T bb = zp.bconst[ii];
+          if (zp.ks != nullptr) bb += sv[ii];
+          t.x -= bb * Lk.x;
+          t.y -= bb * Lk.y;
+        }
+        buf[ii * N * B + e] = t;
       }
-      if (b < bw) lq[slot] = __ldg(&zp.L[z * zstride + col + b]);
     }
   };
 #pragma unroll
@@ -349,46 +379,11 @@ __device__ __forceinline__ void z_tile_g(const Geo &g, typename Cx<T>::type *buf
   for (int it = 0; it < NIT; ++it) {
     const int slot = it % D;
     const int e = tid + it * NTHR;
-    if (act && e < N * B) {
-      const int b = e % B;
-      const bool valid = b < bw;
-      const T fr = fq[slot];
-      const V Lk = lq[slot];
-      V c[MS];
-#pragma unroll
-      for (int j = 0; j < MS; ++j)
-        if (j < m) c[j] = buf[j * N * B + e];
-      if (full) {
-#pragma unroll
-        for (int j = 0; j < MS; ++j)
-          if (j < m) { c[j].x -= zp.a[j] * Lk.x; c[j].y -= zp.a[j] * Lk.y; }
-      }
-      T xv[NP];
-#pragma unroll
-      for (int q = 0; q < NP; ++q)
-        if (q < np) xv[q] = tq[slot][q].x + tq[slot][q].y * fr;
-#pragma unroll
-      for (int ii = 0; ii < MS; ++ii) {
-        if (ii < m) {
-          V t;
-          t.x = T(0); t.y = T(0);
-#pragma unroll
-          for (int j = 0; j < MS; ++j) {
-            if (j < m) {
-              const T x = xv[ii >= j ? ii * (ii + 1) / 2 + j : j * (j + 1) / 2 + ii];
-              t.x += x * c[j].x;
-              t.y += x * c[j].y;
-            }
-          }
-          if (full) {
-            T bb = zp.bconst[ii];
-            if (zp.stab != nullptr) bb += sq[slot][ii].x + sq[slot][ii].y * fr;
-            t.x -= bb * Lk.x;
-            t.y -= bb * Lk.y;
-          }
-          if (valid) buf[ii * N * B + e] = t;
-        }
-      }
+    const int r = e / B, b = e % B;
+    if (act && e < H * B && b < bw) {
+      contract(e, tq[slot], sq[slot], lq[slot][0]);
+      if (r == 0) load(H, b, tq[slot], sq[slot]);
+      contract((r == 0 ? H : N - r) * B + b, tq[slot], sq[slot], lq[slot][1]);
     }
     if (it + D < NIT) fetch(it + D, slot);
   }
@@ -397,29 +392,239 @@ __device__ __forceinline__ void z_tile_g(const Geo &g, typename Cx<T>::type *buf
   else
     for (int s = 0; s < m; ++s) fft2g<N, B, NTHR, true, true, LayCol<N, B>, S>(buf + s * N * B, tw, tid, act);
 }
+// ---- the fused z tile
+//
+// Forward transform, contraction and inverse transform of the m site columns
+// with the middle of all three in registers.  With N = R1 R2, n = R2 n1 + n2
+// and k = k1 + R1 k2,
+//
+//   A  per (site, n2, column): R1-point DFT over n1, times W^(n2 k1), back in
+//      place (rows R2 k1 + n2);
+//   M  per (k1, column): the R2-point DFTs over n2 of all m sites give
+//      X[k1 + R1 k2] for every k2 in registers; contract each k with chi - 1;
+//      the inverse R2-point DFTs over k2, times W^(-n2 k1), back in place;
+//   E  per (site, n2, column): inverse R1-point DFT over k1, back in place.
+//
+// Every step reads and writes the thread's own rows, so a tile takes three
+// shared-memory round trips and three barriers, where two whole transforms
+// per site and a separate contraction took five round trips and 6 m + 1
+// barriers: with four 128-thread CTAs per SM the pass was bound by those
+// barriers and the latency behind them (2.4 of 6.5 TB/s), not by memory.
+// J / F passes before -> after, us: 256^3 FP32 169 / 234 -> 127 / 201, FP64
+// 341 / 474 -> 245 / 315; 96^3 FP32 21.9 / 26.0 -> 11.0 / 17.7, FP64 32.5 /
+// 42.0 -> 17.3 / 22.4; 512^3 FP32 1923 / 4195 -> 1426 / 2512.  What is left is
+// the FP64 units (FP64) and twelve resident warps per SM (FP32).
+template <typename T, int N> struct ZFused {
+  // R2 bounds the registers of M (m R2 complex values): 16 in FP32, 8 in FP64
+  static constexpr bool f64 = sizeof(T) == 8;
+  static constexpr int R2 = f64 ? (N % 8 == 0 ? 8 : 6)
+                                : N == 48 ? 6 : N == 64 ? 8 : N == 72 ? 6 : N == 96 ? 8 : N == 128 ? 8
+                                : N == 144 ? 9 : N == 192 ? 12 : 16;
+  static constexpr int R1 = N / R2;
+  static constexpr bool on = R1 * R2 == N && R1 <= 32;
+  // chi - 1 of the tile's rows staged in shared memory where that leaves room
+  // for as many CTAs as the registers do
+  static constexpr bool stage = N <= 256;
+};
+
+// Shared memory of a tile's staged values: chi - 1 [m(m+1)/2][N/2 + 1][B] and,
+// in MODE_F, beta/eps0 s_i [m][N/2 + 1][B] and the long-range field [N][B].
+template <typename T, int MODE, int N, int B> __host__ __device__ constexpr size_t zf_stage_bytes(int m) {
+  return !(ZFused<T, N>::on && ZFused<T, N>::stage)
+             ? 0
+             : sizeof(T) * ((size_t)(m * (m + 1) / 2 + (MODE == MODE_F ? m : 0)) * (N / 2 + 1) * B +
+                            (MODE == MODE_F ? (size_t)2 * N * B : 0));
+}
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Issues the copies of the tile's staged values, which land while the tile
+// is loaded and A runs: every thread waits for its own before the barrier
+// that follows A.  The long-range rows end at Nhp (even, so whole 16-byte
+// pieces in FP32 and FP64); what lies beyond is not read (M skips columns
+// past Nh).
+template <typename T, int MODE, int N, int B, int NTHR>
+__device__ __forceinline__ void zf_stage(const Geo &g, const ZParams<T> &zp, int kx0, int y, T *tab) {
+  if constexpr (ZFused<T, N>::on && ZFused<T, N>::stage) {
+    using V = typename Cx<T>::type;
+    constexpr int H2 = N / 2 + 1;
+    constexpr int E16 = 16 / (int)sizeof(T);
+    constexpr int PER = B / E16;  // 16-byte pieces per row
+    static_assert(PER >= 1, "a table row is at least one 16-byte piece");
+    const int OR = oct_row(g);
+    const int np = g.m * (g.m + 1) / 2;
+    const long long o = (long long)(y <= g.N1 / 2 ? y : g.N1 - y) * H2 * OR + kx0;
+    for (int q = 0; q < np + (MODE == MODE_F && zp.ks ? g.m : 0); ++q) {
+      const T *src = (q < np ? zp.kt + q * zp.oct : zp.ks + (q - np) * zp.oct) + o;
+      for (int e = threadIdx.x; e < H2 * PER; e += NTHR) {
+        const int r = e / PER, c = (e % PER) * E16;
+        cp_async16(tab + ((size_t)q * H2 + r) * B + c, src + (long long)r * OR + c);
+      }
+    }
+    if (MODE == MODE_F && zp.L) {
+      V *ls = reinterpret_cast<V *>(tab + (size_t)(np + g.m) * H2 * B);
+      for (int e = threadIdx.x; e < N * 2 * PER; e += NTHR) {
+        const int z = e / (2 * PER), c = (e % (2 * PER)) * E16 / 2;
+        if (kx0 + c < g.Nhp) cp_async16(ls + z * B + c, zp.L + ((long long)z * g.N1 + y) * g.Nhp + kx0 + c);
+      }
+    }
+  }
+}
+
+template <typename T, int MODE, int N, int B, int MS, int NTHR>
+__device__ __forceinline__ void z_tile_f(const Geo &g, typename Cx<T>::type *buf, const typename Cx<T>::type *tw,
+                                         const T *tab, const ZParams<T> &zp, int kx0, int y) {
+  using V = typename Cx<T>::type;
+  using Z = ZFused<T, N>;
+  constexpr int R1 = Z::R1, R2 = Z::R2;
+  constexpr int NP = MS * (MS + 1) / 2;
+  constexpr int H2 = N / 2 + 1;
+  const int tid = threadIdx.x;
+  const int m = g.m;
+  const int np = m * (m + 1) / 2;
+  const bool full = MODE == MODE_F && zp.L != nullptr;
+  // A
+#pragma unroll 1
+  for (int w = tid; w < m * R2 * B; w += NTHR) {
+    const int col = w % B, n2 = (w / B) % R2, s = w / (B * R2);
+    V *p = buf + s * N * B + n2 * B + col;
+    V u[R1];
+#pragma unroll
+    for (int n1 = 0; n1 < R1; ++n1) u[n1] = p[n1 * R2 * B];
+    RDft<R1, false, V>::run(u, tw, N / R1);
+#pragma unroll
+    for (int k1 = 0; k1 < R1; ++k1) p[k1 * R2 * B] = k1 == 0 ? u[0] : cmul(u[k1], tw[n2 * k1]);
+  }
+  if constexpr (Z::stage) cp_async_wait_all();
+  __syncthreads();
+  // M
+#pragma unroll 1
+  for (int w = tid; w < R1 * B; w += NTHR) {
+    const int col = w % B, k1 = w / B;
+    V u[MS][R2];
+#pragma unroll
+    for (int s = 0; s < MS; ++s) {
+      if (s < m) {
+        const V *p = buf + s * N * B + k1 * R2 * B + col;
+#pragma unroll
+        for (int n2 = 0; n2 < R2; ++n2) u[s][n2] = p[n2 * B];
+        RDft<R2, false, V>::run(u[s], tw, N / R2);
+      } else {
+#pragma unroll
+        for (int n2 = 0; n2 < R2; ++n2) u[s][n2].x = u[s][n2].y = T(0);
+      }
+    }
+    const bool valid = kx0 + col < g.Nh;
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) {
+      const int z = k1 + R1 * k2;
+      const int zz = z <= N / 2 ? z : N - z;
+      T x[NP];
+      const long long o = ((long long)(y <= g.N1 / 2 ? y : g.N1 - y) * H2 + zz) * oct_row(g) + kx0 + col;
+#pragma unroll
+      for (int q = 0; q < NP; ++q)
+        if (q < np) x[q] = Z::stage ? tab[((size_t)q * H2 + zz) * B + col] : __ldg(&zp.kt[q * zp.oct + o]);
+        else x[q] = T(0);
+      V Lk;
+      Lk.x = Lk.y = T(0);
+      if (full && valid)
+        Lk = Z::stage ? reinterpret_cast<const V *>(tab + (size_t)(np + m) * H2 * B)[z * B + col]
+                      : __ldg(&zp.L[((long long)z * g.N1 + y) * g.Nhp + kx0 + col]);
+      V c[MS];
+#pragma unroll
+      for (int j = 0; j < MS; ++j) {
+        c[j] = u[j][k2];
+        if (full && j < m) { c[j].x -= zp.a[j] * Lk.x; c[j].y -= zp.a[j] * Lk.y; }
+      }
+#pragma unroll
+      for (int i = 0; i < MS; ++i) {
+        V t;
+        t.x = T(0); t.y = T(0);
+#pragma unroll
+        for (int j = 0; j < MS; ++j) {
+          const T xv = x[i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i];
+          t.x += xv * c[j].x;
+          t.y += xv * c[j].y;
+        }
+        if (full && i < m) {
+          T bb = zp.bconst[i];
+          if (zp.ks != nullptr)
+            bb += Z::stage ? tab[((size_t)(np + i) * H2 + zz) * B + col] : __ldg(&zp.ks[i * zp.oct + o]);
+          t.x -= bb * Lk.x;
+          t.y -= bb * Lk.y;
+        }
+        u[i][k2] = t;
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < MS; ++s) {
+      if (s < m) {
+        V *p = buf + s * N * B + k1 * R2 * B + col;
+        RDft<R2, true, V>::run(u[s], tw, N / R2);
+#pragma unroll
+        for (int n2 = 0; n2 < R2; ++n2) p[n2 * B] = n2 == 0 ? u[s][0] : cmul(u[s][n2], cconj(tw[n2 * k1]));
+      }
+    }
+  }
+  __syncthreads();
+  // E
+#pragma unroll 1
+  for (int w = tid; w < m * R2 * B; w += NTHR) {
+    const int col = w % B, n2 = (w / B) % R2, s = w / (B * R2);
+    V *p = buf + s * N * B + n2 * B + col;
+    V u[R1];
+#pragma unroll
+    for (int k1 = 0; k1 < R1; ++k1) u[k1] = p[k1 * R2 * B];
+    RDft<R1, true, V>::run(u, tw, N / R1);
+#pragma unroll
+    for (int n1 = 0; n1 < R1; ++n1) p[n1 * R2 * B] = u[n1];
+  }
+  __syncthreads();
+}
+
+// Threads of a z-pass CTA.
+template <typename T, int N, int B> __host__ __device__ constexpr int z_threads() {
+  return ZFused<T, N>::on ? (ZFused<T, N>::R1 * B + 31) / 32 * 32 : Split<N>::R1 * B;
+}
 template <typename T, int MODE, int N, int B, int MS>
 __device__ __forceinline__ void z_tile(const Geo &g, typename Cx<T>::type *buf, const typename Cx<T>::type *tw,
-                                       const ZParams<T> &zp, int kx0, int y) {
-  z_tile_g<T, MODE, N, B, MS>(g, buf, tw, zp, kx0, y, (int)threadIdx.x, true);
+                                       const T *tab, const ZParams<T> &zp, int kx0, int y) {
+  if constexpr (ZFused<T, N>::on)
+    z_tile_f<T, MODE, N, B, MS, z_threads<T, N, B>()>(g, buf, tw, tab, zp, kx0, y);
+  else
+    z_tile_g<T, MODE, N, B, MS>(g, buf, tw, zp, kx0, y, (int)threadIdx.x, true);
+}
+// Rows of the pass in launch order: y and N1 - y, which share their chi - 1
+// rows, next to one another (0, 1, N1 - 1, 2, N1 - 2, ...).
+__device__ __forceinline__ int z_row(int i, int N1) { return i == 0 ? 0 : ((i & 1) ? (i + 1) / 2 : N1 - i / 2); }
+
+// CTAs per SM that the z pass's registers are bounded for (shared memory
+// allows as many): the fused tile holds m R2 complex values per thread.
+template <typename T, int MODE, int N> __host__ __device__ constexpr int z_min_ctas() {
+  if (!ZFused<T, N>::on) return sizeof(T) == 4 ? 4 : 1;
+  return sizeof(T) == 8 || N > 256 || MODE == MODE_F ? 2 : 3;
 }
 
 // z pass: the m [N][B] tiles of one (ky, kx-block) by TMA, forward transform,
 // OZ contraction (+ long-range terms in MODE_F), inverse transform, TMA out.
 // tm: W as {2 Nhp, N1, m N2} scalars, box {2B, 1, N2}.
 template <typename T, int MODE, int N, int B, int MS>
-__global__ void __launch_bounds__(Split<N>::R1 * B, sizeof(T) == 4 ? 4 : 1) k_z_s(Geo g,
-                                                                                  const __grid_constant__ CUtensorMap tm,
-                                                         const typename Cx<T>::type *__restrict__ twg,
-                                                         ZParams<T> zp, int *__restrict__ err) {
+__global__ void __launch_bounds__((z_threads<T, N, B>()), (z_min_ctas<T, MODE, N>()))
+    k_z_s(Geo g, const __grid_constant__ CUtensorMap tm, const typename Cx<T>::type *__restrict__ twg, ZParams<T> zp,
+          int *__restrict__ err) {
   using V = typename Cx<T>::type;
-  constexpr int NTHR = Split<N>::R1 * B;
+  constexpr int NTHR = z_threads<T, N, B>();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int m = g.m;
   V *buf = reinterpret_cast<V *>(smem_raw);
   V *tw = buf + m * N * B;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(tw + N);
+  T *tab = reinterpret_cast<T *>(tw + N);
+  uint64_t *bar = reinterpret_cast<uint64_t *>(reinterpret_cast<unsigned char *>(tab) + zf_stage_bytes<T, MODE, N, B>(m));
   const int tid = threadIdx.x;
-  const int kx0 = blockIdx.x * B, y = blockIdx.y;
+  const int kx0 = blockIdx.x * B, y = z_row(blockIdx.y, g.N1);
   if (tid == 0) mbar_init(bar, 1);
   __syncthreads();
   if (tid == 0) {
@@ -428,9 +633,13 @@ __global__ void __launch_bounds__(Split<N>::R1 * B, sizeof(T) == 4 ? 4 : 1) k_z_
 #pragma unroll
       for (int c = 0; c < N; c += kTmaRows) tma_load_3d(buf + s * N * B + c * B, &tm, bar, 2 * kx0, y, s * g.N2 + c);
   }
+  zf_stage<T, MODE, N, B, NTHR>(g, zp, kx0, y, tab);
   for (int q = tid; q < N; q += NTHR) tw[q] = twg[q];
-  if (!cta_wait_tile(bar, 0, kMbarPolls, err, 2)) return;
-  z_tile<T, MODE, N, B, MS>(g, buf, tw, zp, kx0, y);
+  if (!cta_wait_tile(bar, 0, kMbarPolls, err, 2)) {
+    cp_async_wait_all();
+    return;
+  }
+  z_tile<T, MODE, N, B, MS>(g, buf, tw, tab, zp, kx0, y);
   fence_proxy_async();
   __syncthreads();
   if (tid == 0) {
@@ -447,18 +656,19 @@ __global__ void __launch_bounds__(Split<N>::R1 * B, sizeof(T) == 4 ? 4 : 1) k_z_
 // store of a tile drains while the next is transformed.  Tiles t =
 // blockIdx.x, blockIdx.x + gridDim.x, ... (kx-block t % nkx, ky t / nkx).
 template <typename T, int MODE, int N, int B, int MS>
-__global__ void __launch_bounds__(Split<N>::R1 * B) k_z_sp(Geo g, const __grid_constant__ CUtensorMap tm,
-                                                          const typename Cx<T>::type *__restrict__ twg,
-                                                          ZParams<T> zp, int *__restrict__ err) {
+__global__ void __launch_bounds__(z_threads<T, N, B>())
+    k_z_sp(Geo g, const __grid_constant__ CUtensorMap tm, const typename Cx<T>::type *__restrict__ twg, ZParams<T> zp,
+           int *__restrict__ err) {
   using V = typename Cx<T>::type;
-  constexpr int NTHR = Split<N>::R1 * B;
+  constexpr int NTHR = z_threads<T, N, B>();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int m = g.m;
   V *bufs[2];
   bufs[0] = reinterpret_cast<V *>(smem_raw);
   bufs[1] = bufs[0] + m * N * B;
   V *tw = bufs[1] + m * N * B;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(tw + N);
+  T *tab = reinterpret_cast<T *>(tw + N);
+  uint64_t *bar = reinterpret_cast<uint64_t *>(reinterpret_cast<unsigned char *>(tab) + zf_stage_bytes<T, MODE, N, B>(m));
   const int tid = threadIdx.x;
   const int nkx = (g.Nh + B - 1) / B;
   const int ntile = nkx * g.N1;
@@ -490,8 +700,11 @@ __global__ void __launch_bounds__(Split<N>::R1 * B) k_z_sp(Geo g, const __grid_c
           tma_load_3d(bufs[cur ^ 1] + s * N * B + c * B, &tm, &bar[cur ^ 1], 2 * (tn % nkx) * B, tn / nkx,
                       s * g.N2 + c);
     }
+    const int kx0 = (t % nkx) * B, y = t / nkx;
+    zf_stage<T, MODE, N, B, NTHR>(g, zp, kx0, y, tab);
     const bool ok = mbar_wait(&bar[cur], (uint32_t)((it >> 1) & 1), kMbarPolls);
     if (__syncthreads_or(!ok)) {
+      cp_async_wait_all();
       // a CTA-uniform exit: both buffers' loads (this tile's and the
       // prefetch of the next) get one more bounded wait, and the stores
       // drain, before the CTA leaves
@@ -504,8 +717,7 @@ __global__ void __launch_bounds__(Split<N>::R1 * B) k_z_sp(Geo g, const __grid_c
       __syncthreads();
       return;
     }
-    const int kx0 = (t % nkx) * B, y = t / nkx;
-    z_tile<T, MODE, N, B, MS>(g, bufs[cur], tw, zp, kx0, y);
+    z_tile<T, MODE, N, B, MS>(g, bufs[cur], tw, tab, zp, kx0, y);
     fence_proxy_async();
     __syncthreads();
     if (tid == 0) {

@@ -225,6 +225,8 @@ struct rism3d_ctx {
   float2 *L32 = nullptr;
   double2 *chi64 = nullptr, *s64 = nullptr;
   float2 *chi32 = nullptr, *s32 = nullptr;
+  double *kt64 = nullptr, *ks64 = nullptr;  // the tables above on the octant of the k grid (made on first use)
+  float *kt32 = nullptr, *ks32 = nullptr;
   double2 *chi3_64 = nullptr;  // chi - 1 on the k grid (W layout, packed pairs), or null
   float2 *chi3_32 = nullptr;
   // pure-solvent context: solvent sites (0 for a solute context), the pair
@@ -299,7 +301,7 @@ struct rism3d_ctx {
     auto fr = [](void *p) { dfree(p); };
     for (int i = 0; i < 3; ++i) { fr(tw64[i]); fr(tw32[i]); }
     fr(post64); fr(post32); fr(v64); fr(uc64); fr(v32); fr(L64); fr(L32);
-    fr(chi64); fr(s64); fr(chi32); fr(s32); fr(chi3_64); fr(chi3_32); fr(ck); fr(W); fr(d_solute); fr(d_solvent); fr(d_charge);
+    fr(chi64); fr(s64); fr(chi32); fr(s32); fr(kt64); fr(ks64); fr(kt32); fr(ks32); fr(chi3_64); fr(chi3_32); fr(ck); fr(W); fr(d_solute); fr(d_solvent); fr(d_charge);
     fr(npart); fr(dpart); fr(dres); fr(F64); fr(X64t); fr(F64t); fr(X32); fr(F32); fr(X32t); fr(F32t);
     fr(d64); fr(d32); fr(dx64); fr(dx32); fr(d_err);
     for (auto p : basis64) fr(p);
@@ -347,32 +349,51 @@ struct TimeScope {
   }
 };
 
-template <typename T> ZParams<T> zparams(rism3d_ctx *c, bool full);
-template <> ZParams<double> zparams<double>(rism3d_ctx *c, bool full) {
-  ZParams<double> z{};
-  z.chi = c->chi64;
-  z.chi3 = c->chi3_64;
-  z.stab = (full && c->pd.renorm) ? c->s64 : nullptr;
-  z.L = full ? c->L64 : nullptr;
-  z.nrad = c->pd.nrad;
-  z.dkr = c->dkr;
-  for (int i = 0; i < c->m && !c->pure; ++i) {
-    z.a[i] = c->pd.renorm ? 0.0 : c->pd.beta * c->charge[i];
-    z.bconst[i] = c->pd.renorm ? 0.0 : c->pd.beta * c->charge[i];
+long long octant_size(const Geo &g) { return (long long)(g.N1 / 2 + 1) * (g.N2 / 2 + 1) * oct_row(g); }
+
+// Radial tables on the octant of the k grid: made once per context and
+// precision, on the stream of the pass that first needs them (before any
+// capture: coarse_graph and coarse_pk_ready ask for theirs up front).
+template <typename T>
+const T *octant_table(rism3d_ctx *c, const typename Vec2<T>::type *tab, int ntab, T **slot) {
+  if (!*slot && tab) {
+    const long long oct = octant_size(c->g);
+    T *p = dalloc<T>((size_t)ntab * oct);
+    k_octant<T><<<(unsigned)((oct + 255) / 256), 256, 0, c->stream>>>(c->g, tab, ntab, c->pd.nrad, c->dkr, p);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) dfree(p);
+    CK(e);
+    *slot = p;
   }
-  return z;
+  return *slot;
 }
-template <> ZParams<float> zparams<float>(rism3d_ctx *c, bool full) {
-  ZParams<float> z{};
-  z.chi = c->chi32;
-  z.chi3 = c->chi3_32;
-  z.stab = (full && c->pd.renorm) ? c->s32 : nullptr;
-  z.L = full ? c->L32 : nullptr;
+
+template <typename T> ZParams<T> zparams(rism3d_ctx *c, bool full) {
+  constexpr bool f64 = sizeof(T) == 8;
+  ZParams<T> z{};
+  const int np = c->m * (c->m + 1) / 2;
+  const bool oct = c->stat[f64 ? 0 : 1];  // the shape-specialised z passes read the octant tables
+  if constexpr (f64) {
+    z.chi = c->chi64;
+    z.chi3 = c->chi3_64;
+    z.stab = (full && c->pd.renorm) ? c->s64 : nullptr;
+    z.L = full ? c->L64 : nullptr;
+    if (oct) z.kt = octant_table<T>(c, c->chi64, np, &c->kt64);
+    if (oct && z.stab) z.ks = octant_table<T>(c, c->s64, c->m, &c->ks64);
+  } else {
+    z.chi = c->chi32;
+    z.chi3 = c->chi3_32;
+    z.stab = (full && c->pd.renorm) ? c->s32 : nullptr;
+    z.L = full ? c->L32 : nullptr;
+    if (oct) z.kt = octant_table<T>(c, c->chi32, np, &c->kt32);
+    if (oct && z.stab) z.ks = octant_table<T>(c, c->s32, c->m, &c->ks32);
+  }
+  z.oct = octant_size(c->g);
   z.nrad = c->pd.nrad;
   z.dkr = c->dkr;
   for (int i = 0; i < c->m && !c->pure; ++i) {
-    z.a[i] = c->pd.renorm ? 0.f : (float)(c->pd.beta * c->charge[i]);
-    z.bconst[i] = c->pd.renorm ? 0.f : (float)(c->pd.beta * c->charge[i]);
+    z.a[i] = c->pd.renorm ? T(0) : (T)(c->pd.beta * c->charge[i]);
+    z.bconst[i] = c->pd.renorm ? T(0) : (T)(c->pd.beta * c->charge[i]);
   }
   return z;
 }
@@ -406,11 +427,12 @@ template <typename T, int M> constexpr size_t xs_smem() {
 template <typename T, int N> constexpr size_t ys_smem() {
   return sizeof(typename Cx<T>::type) * (size_t)(N * static_B<T>() + N) + 16;
 }
-template <typename T, int N> size_t zs_smem(int m, int B = static_Bz<T>()) {
-  return sizeof(typename Cx<T>::type) * (size_t)(m * N * B + N) + 16;
+template <typename T, int MODE, int N, int B = static_Bz<T>()> size_t zs_smem(int m) {
+  return sizeof(typename Cx<T>::type) * (size_t)(m * N * B + N) + zf_stage_bytes<T, MODE, N, B>(m) + 16;
 }
-template <typename T, int N> size_t zsp_smem(int m) {  // two tile buffers, two mbarriers
-  return sizeof(typename Cx<T>::type) * (size_t)(2 * m * N * static_Bz<T>() + N) + 16;
+template <typename T, int MODE, int N> size_t zsp_smem(int m) {  // two tile buffers, two mbarriers
+  return sizeof(typename Cx<T>::type) * (size_t)(2 * m * N * static_Bz<T>() + N) +
+         zf_stage_bytes<T, MODE, N, static_Bz<T>()>(m) + 16;
 }
 // Lengths with shape-specialised passes: the coarse grids (48, 96) and the
 // even 2^a 3^b grids of the many-solute workloads whose two-step split fits
@@ -552,15 +574,15 @@ template <typename T, int MODE> void launch_z(rism3d_ctx *c) {
   case N:                                                                                                  \
     if (B == BW && c->zpers[sizeof(T) == 8 ? 0 : 1]) {                                                     \
       const unsigned nt = (unsigned)(((c->g.Nh + BW - 1) / BW) * c->g.N1);                                 \
-      const size_t sm = zsp_smem<T, N>(c->m);                                                               \
+      const size_t sm = zsp_smem<T, MODE, N>(c->m);                                                               \
       const void *fn = (const void *)k_z_sp<T, MODE, N, BW, 3>;                                             \
-      k_z_sp<T, MODE, N, BW, 3><<<persistent_grid(fn, sm, nt, Split<N>::R1 * BW), Split<N>::R1 * BW, sm,    \
+      k_z_sp<T, MODE, N, BW, 3><<<persistent_grid(fn, sm, nt, z_threads<T, N, BW>()), z_threads<T, N, BW>(), sm, \
                                   c->stream>>>(c->g, tm, tw, zp, c->d_err);                                \
     } else if (B == BW)                                                                                    \
-      k_z_s<T, MODE, N, BW, 3><<<grid, Split<N>::R1 * BW, zs_smem<T, N>(c->m, BW), c->stream>>>(c->g, tm, tw, \
+      k_z_s<T, MODE, N, BW, 3><<<grid, z_threads<T, N, BW>(), zs_smem<T, MODE, N, BW>(c->m), c->stream>>>(c->g, tm, tw, \
                                                                                                zp, c->d_err); \
     else                                                                                                   \
-      k_z_s<T, MODE, N, BN, 3><<<grid, Split<N>::R1 * BN, zs_smem<T, N>(c->m, BN), c->stream>>>(c->g, tm, tw, \
+      k_z_s<T, MODE, N, BN, 3><<<grid, z_threads<T, N, BN>(), zs_smem<T, MODE, N, BN>(c->m), c->stream>>>(c->g, tm, tw, \
                                                                                                zp, c->d_err); \
     break;
       Z_CASE(48) Z_CASE(64) Z_CASE(72) Z_CASE(96) Z_CASE(128) Z_CASE(144) Z_CASE(192) Z_CASE(256) Z_CASE(512)
@@ -1180,6 +1202,7 @@ bool coarse_graph(rism3d_ctx *c, int k) {
   }
   rism3d_ctx *cc = c->coarse;
   ensure_basis<float>(cc, k + 1);  // every buffer the graph touches exists before capture
+  zparams<float>(cc, false);
   slopebuf<float>(cc);
   if (!c->cg_H) c->cg_H = dalloc<double>((size_t)k * (k + 1));
   if (!c->cg_aux) c->cg_aux = dalloc<double>((size_t)k + 2);
@@ -1272,6 +1295,7 @@ bool coarse_pk_ready(rism3d_ctx *c, int k) {
     return false;
   }
   ensure_basis<float>(cc, k + 1);
+  zparams<float>(cc, false);
   slopebuf<float>(cc);
   c->pk_dot = dalloc<double>((size_t)grid * kVecMax);
   c->pk_nrm = dalloc<double>((size_t)2 * grid);
@@ -2551,9 +2575,8 @@ int create_impl(const rism3d_problem *pd, int m, const rism3d_site *solvent, int
     OPTIN_Z(float)
 #undef OPTIN_Z
     if (c->stat[0]) {
-      need = std::max({xs_smem<double, 256>(), ys_smem<double, 512>(), zsp_smem<double, 512>(m),
-                       zsp_smem<float, 512>(m), zs_smem<double, 512>(m),
-                       xs_smem<float, 256>(), ys_smem<float, 512>(), zs_smem<float, 512>(m)});
+      need = std::max({xs_smem<double, 256>(), ys_smem<double, 512>(), zsp_smem<double, MODE_F, 512>(m),
+                       zsp_smem<double, MODE_F, 256>(m), xs_smem<float, 256>(), ys_smem<float, 512>()});
 #define OPTIN_S(T)                                               \
   allow((const void *)k_xfwd_s<T, MODE_F, 24, kStaticRX>);       \
   allow((const void *)k_xfwd_s<T, MODE_J, 24, kStaticRX>);       \
