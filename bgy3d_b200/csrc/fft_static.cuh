@@ -96,7 +96,18 @@ template <int N> struct SplitSq {
 // radix would leave most of the CTA idle in one step (32 = 16 x 2 gives R2 x
 // rows items of 16-point DFTs); here both steps keep the CTA busy.
 template <int N> struct SplitRow {
-  static constexpr int R1 = N == 24 ? 6 : N == 32 ? 8 : N == 36 ? 6 : N == 48 ? 8 : N == 96 ? 12 : Split<N>::R1;
+  static constexpr int R1 = N == 16 ? 4 : N == 18 ? 6 : N == 24 ? 6 : N == 27 ? 9 : N == 32 ? 8 : N == 36 ? 6
+                            : N == 48 ? 8 : N == 54 ? 9 : N == 81 ? 9 : N == 96 ? 12 : N == 108 ? 12 : N == 144 ? 12
+                            : N == 162 ? 18 : N == 216 ? 18 : N == 243 ? 27 : Split<N>::R1;
+  static constexpr int R2 = N / R1;
+};
+
+// The split of the y columns (R1 B threads, one second-step DFT each): Split
+// where it has a balanced one, factors of 6, 9, 12, 18 and 27 elsewhere.
+template <int N> struct SplitY {
+  static constexpr int R1 = N == 32 ? 8 : N == 36 ? 6 : N == 54 ? 9 : N == 108 ? 12 : N == 162 ? 18 : N == 216 ? 18
+                            : N == 288 ? 18 : N == 324 ? 18 : N == 384 ? 24 : N == 432 ? 24 : N == 486 ? 27
+                            : Split<N>::R1;
   static constexpr int R2 = N / R1;
 };
 

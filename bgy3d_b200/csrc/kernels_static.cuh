@@ -11,6 +11,8 @@
 // B columns of a y/z tile are 128 bytes (16 float2 or 8 double2): one TMA box
 // row per transform index, so every HBM access is a whole 128-byte line.
 #pragma once
+#include <type_traits>
+
 #include "fft_static.cuh"
 #include "kernels.cuh"
 
@@ -18,9 +20,16 @@ namespace rism {
 
 constexpr uint32_t kMbarPolls = 1u << 26;  // bounded mbarrier wait (seconds)
 
-template <typename T> struct VecW;  // complex values per vector load in the x passes
-template <> struct VecW<float> { static constexpr int n = 2; using vec = float4; };
-template <> struct VecW<double> { static constexpr int n = 1; using vec = double2; };
+// Complex values per vector load in the x passes: 16 bytes, or one value
+// where an odd half row leaves every other row off a 16-byte boundary.
+template <typename T, int M> struct VecW { static constexpr int n = 1; using vec = typename Cx<T>::type; };
+template <int M> struct VecW<float, M> {
+  static constexpr int n = M % 2 == 0 ? 2 : 1;
+  using vec = std::conditional_t<M % 2 == 0, float4, float2>;
+};
+
+// Rows per CTA of the x passes.
+__host__ __device__ constexpr int x_rows(int) { return 16; }
 
 // x forward (see k_xfwd): MODE_F c = closure(p B, A); MODE_J c = B (p A).
 template <typename T, int MODE, int M, int RX>
@@ -30,8 +39,8 @@ __global__ void __launch_bounds__(256) k_xfwd_s(Geo g, const T *__restrict__ A, 
                                                const typename Cx<T>::type *__restrict__ twg) {
   using V = typename Cx<T>::type;
   using Lay = LayRow<M, SplitRow<M>::R2>;
-  constexpr int VW = VecW<T>::n;
-  using VEC = typename VecW<T>::vec;
+  constexpr int VW = VecW<T, M>::n;
+  using VEC = typename VecW<T, M>::vec;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   V *tw = reinterpret_cast<V *>(smem_raw);
   V *buf = tw + M;
@@ -112,8 +121,8 @@ __global__ void __launch_bounds__(256) k_xinv_s(Geo g, const typename Cx<T>::typ
                                                NormPartial *__restrict__ part) {
   using V = typename Cx<T>::type;
   using Lay = LayRow<M, SplitRow<M>::R2>;
-  constexpr int VW = VecW<T>::n;
-  using VEC = typename VecW<T>::vec;
+  constexpr int VW = VecW<T, M>::n;
+  using VEC = typename VecW<T, M>::vec;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   V *tw = reinterpret_cast<V *>(smem_raw);
   V *buf = tw + M;
@@ -234,18 +243,25 @@ __global__ void __launch_bounds__(256) k_xinv_s(Geo g, const typename Cx<T>::typ
   block_norms(amax, sum2, part + (blockIdx.y * gridDim.x + blockIdx.x));
 }
 
-// A TMA box spans at most 256 elements per dimension: tiles along a 512-point
-// axis move as two boxes of kTmaRows rows.
-constexpr int kTmaRows = 256;
+// A TMA box spans at most 256 elements per dimension: tiles along a longer
+// axis move as two boxes of half its rows, or three of a third where half is
+// odd: a box lands on a 128-byte boundary of shared memory, and a z row is 64
+// bytes.
+__host__ __device__ constexpr int tma_rows(int n) { return n <= 256 ? n : (n % 4 == 0 ? n / 2 : n / 3); }
+template <typename V, int N, int B> __host__ __device__ constexpr bool tma_tile_ok() {
+  return N % tma_rows(N) == 0 && tma_rows(N) <= 256 && (size_t)N * B * sizeof(V) % 128 == 0 &&
+         (size_t)tma_rows(N) * B * sizeof(V) % 128 == 0;
+}
 
 // y pass: one [N][B] tile (kx0 .. kx0+B-1 at fixed z, site) by TMA.
 // tm: W as {2 Nhp, N1, m N2} scalars, box {2B, N1, 1}.
 template <typename T, bool INV, int N, int B>
-__global__ void __launch_bounds__(Split<N>::R1 * B) k_y_s(Geo g, const __grid_constant__ CUtensorMap tm,
+__global__ void __launch_bounds__(SplitY<N>::R1 * B) k_y_s(Geo g, const __grid_constant__ CUtensorMap tm,
                                                          const typename Cx<T>::type *__restrict__ twg,
                                                          int *__restrict__ err) {
   using V = typename Cx<T>::type;
-  constexpr int NTHR = Split<N>::R1 * B;
+  constexpr int NTHR = SplitY<N>::R1 * B;
+  static_assert(tma_tile_ok<V, N, B>(), "every box starts on a 128-byte boundary");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   V *buf = reinterpret_cast<V *>(smem_raw);
   V *tw = buf + N * B;
@@ -257,16 +273,16 @@ __global__ void __launch_bounds__(Split<N>::R1 * B) k_y_s(Geo g, const __grid_co
   if (tid == 0) {
     mbar_expect_tx(bar, (uint32_t)(N * B * sizeof(V)));
 #pragma unroll
-    for (int c = 0; c < N; c += kTmaRows) tma_load_3d(buf + c * B, &tm, bar, 2 * kx0, c, site * g.N2 + z);
+    for (int c = 0; c < N; c += tma_rows(N)) tma_load_3d(buf + c * B, &tm, bar, 2 * kx0, c, site * g.N2 + z);
   }
   for (int q = tid; q < N; q += NTHR) tw[q] = twg[q];
   if (!cta_wait_tile(bar, 0, kMbarPolls, err, 1)) return;
-  fft2<N, B, NTHR, INV, true, LayCol<N, B>>(buf, tw);
+  fft2<N, B, NTHR, INV, true, LayCol<N, B>, SplitY<N>>(buf, tw);
   fence_proxy_async();
   __syncthreads();
   if (tid == 0) {
 #pragma unroll
-    for (int c = 0; c < N; c += kTmaRows) tma_store_3d(&tm, buf + c * B, 2 * kx0, c, site * g.N2 + z);
+    for (int c = 0; c < N; c += tma_rows(N)) tma_store_3d(&tm, buf + c * B, 2 * kx0, c, site * g.N2 + z);
     tma_commit();
     tma_wait_read0();
   }
@@ -415,16 +431,19 @@ __device__ __forceinline__ void z_tile_g(const Geo &g, typename Cx<T>::type *buf
 // 42.0 -> 17.3 / 22.4; 512^3 FP32 1923 / 4195 -> 1426 / 2512.  What is left is
 // the FP64 units (FP64) and twelve resident warps per SM (FP32).
 template <typename T, int N> struct ZFused {
-  // R2 bounds the registers of M (m R2 complex values): 16 in FP32, 8 in FP64
+  // R2 bounds the registers of M (m R2 complex values): at most 18 in FP32, 9
+  // in FP64; R1 those of A and E: at most 32.  FP64 columns of 324 points and
+  // more have no such pair and keep the separate transforms.
   static constexpr bool f64 = sizeof(T) == 8;
-  static constexpr int R2 = f64 ? (N % 8 == 0 ? 8 : 6)
-                                : N == 48 ? 6 : N == 64 ? 8 : N == 72 ? 6 : N == 96 ? 8 : N == 128 ? 8
-                                : N == 144 ? 9 : N == 192 ? 12 : 16;
+  static constexpr int R2 =
+      f64 ? (N == 32 ? 4 : N == 36 || N == 54 ? 6 : N % 9 == 0 && N > 100 ? 9 : N % 8 == 0 ? 8 : 6)
+          : N == 32 ? 4 : N == 36 || N == 48 || N == 54 || N == 72 ? 6 : N == 64 || N == 96 || N == 128 ? 8
+          : N == 108 || N == 144 || N == 162 ? 9 : N == 192 || N == 216 || N == 324 ? 12 : N == 486 ? 18 : 16;
   static constexpr int R1 = N / R2;
   static constexpr bool on = R1 * R2 == N && R1 <= 32;
-  // chi - 1 of the tile's rows staged in shared memory where that leaves room
-  // for as many CTAs as the registers do
-  static constexpr bool stage = N <= 256;
+  // chi - 1 (and in MODE_F the long-range values) of the tile staged in shared
+  // memory, where the tile leaves room
+  static constexpr bool stage = N <= 288;
 };
 
 // Shared memory of a tile's staged values: chi - 1 [m(m+1)/2][N/2 + 1][B] and,
@@ -587,7 +606,7 @@ __device__ __forceinline__ void z_tile_f(const Geo &g, typename Cx<T>::type *buf
 
 // Threads of a z-pass CTA.
 template <typename T, int N, int B> __host__ __device__ constexpr int z_threads() {
-  return ZFused<T, N>::on ? (ZFused<T, N>::R1 * B + 31) / 32 * 32 : Split<N>::R1 * B;
+  return ZFused<T, N>::on ? (ZFused<T, N>::R1 * B + 31) / 32 * 32 : SplitY<N>::R1 * B;
 }
 template <typename T, int MODE, int N, int B, int MS>
 __device__ __forceinline__ void z_tile(const Geo &g, typename Cx<T>::type *buf, const typename Cx<T>::type *tw,
@@ -595,28 +614,35 @@ __device__ __forceinline__ void z_tile(const Geo &g, typename Cx<T>::type *buf, 
   if constexpr (ZFused<T, N>::on)
     z_tile_f<T, MODE, N, B, MS, z_threads<T, N, B>()>(g, buf, tw, tab, zp, kx0, y);
   else
-    z_tile_g<T, MODE, N, B, MS>(g, buf, tw, zp, kx0, y, (int)threadIdx.x, true);
+    z_tile_g<T, MODE, N, B, MS, false, zpf_default<T, MODE>(), SplitY<N>>(g, buf, tw, zp, kx0, y, (int)threadIdx.x, true);
 }
 // Rows of the pass in launch order: y and N1 - y, which share their chi - 1
 // rows, next to one another (0, 1, N1 - 1, 2, N1 - 2, ...).
 __device__ __forceinline__ int z_row(int i, int N1) { return i == 0 ? 0 : ((i & 1) ? (i + 1) / 2 : N1 - i / 2); }
 
-// CTAs per SM that the z pass's registers are bounded for (shared memory
-// allows as many): the fused tile holds m R2 complex values per thread.
-template <typename T, int MODE, int N> __host__ __device__ constexpr int z_min_ctas() {
+// CTAs per SM that the z pass's registers are bounded for: as many as its
+// shared memory admits at m = 3 (3 at 256 points in FP32), while each thread
+// keeps the m R2 complex values of M and about 72 registers beside them.
+template <typename T, int MODE, int N, int B> __host__ __device__ constexpr int z_min_ctas() {
   if (!ZFused<T, N>::on) return sizeof(T) == 4 ? 4 : 1;
-  return sizeof(T) == 8 || N > 256 || MODE == MODE_F ? 2 : 3;
+  constexpr int w = sizeof(T) / 4;
+  const int smem = (int)(sizeof(T) * 2 * (3 * N * B + N) + zf_stage_bytes<T, MODE, N, B>(3)) + 16 + 1024;
+  const int by_smem = 228 * 1024 / smem;
+  const int by_regs = 65536 / (z_threads<T, N, B>() * (3 * ZFused<T, N>::R2 * 2 * w + 72));
+  const int c = by_smem < by_regs ? by_smem : by_regs;
+  return c < 1 ? 1 : c;
 }
 
 // z pass: the m [N][B] tiles of one (ky, kx-block) by TMA, forward transform,
 // OZ contraction (+ long-range terms in MODE_F), inverse transform, TMA out.
 // tm: W as {2 Nhp, N1, m N2} scalars, box {2B, 1, N2}.
 template <typename T, int MODE, int N, int B, int MS>
-__global__ void __launch_bounds__((z_threads<T, N, B>()), (z_min_ctas<T, MODE, N>()))
+__global__ void __launch_bounds__((z_threads<T, N, B>()), (z_min_ctas<T, MODE, N, B>()))
     k_z_s(Geo g, const __grid_constant__ CUtensorMap tm, const typename Cx<T>::type *__restrict__ twg, ZParams<T> zp,
           int *__restrict__ err) {
   using V = typename Cx<T>::type;
   constexpr int NTHR = z_threads<T, N, B>();
+  static_assert(tma_tile_ok<V, N, B>(), "every box starts on a 128-byte boundary");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int m = g.m;
   V *buf = reinterpret_cast<V *>(smem_raw);
@@ -631,7 +657,7 @@ __global__ void __launch_bounds__((z_threads<T, N, B>()), (z_min_ctas<T, MODE, N
     mbar_expect_tx(bar, (uint32_t)(m * N * B * sizeof(V)));
     for (int s = 0; s < m; ++s)
 #pragma unroll
-      for (int c = 0; c < N; c += kTmaRows) tma_load_3d(buf + s * N * B + c * B, &tm, bar, 2 * kx0, y, s * g.N2 + c);
+      for (int c = 0; c < N; c += tma_rows(N)) tma_load_3d(buf + s * N * B + c * B, &tm, bar, 2 * kx0, y, s * g.N2 + c);
   }
   zf_stage<T, MODE, N, B, NTHR>(g, zp, kx0, y, tab);
   for (int q = tid; q < N; q += NTHR) tw[q] = twg[q];
@@ -645,7 +671,7 @@ __global__ void __launch_bounds__((z_threads<T, N, B>()), (z_min_ctas<T, MODE, N
   if (tid == 0) {
     for (int s = 0; s < m; ++s)
 #pragma unroll
-      for (int c = 0; c < N; c += kTmaRows) tma_store_3d(&tm, buf + s * N * B + c * B, 2 * kx0, y, s * g.N2 + c);
+      for (int c = 0; c < N; c += tma_rows(N)) tma_store_3d(&tm, buf + s * N * B + c * B, 2 * kx0, y, s * g.N2 + c);
     tma_commit();
     tma_wait_read0();
   }
@@ -661,6 +687,7 @@ __global__ void __launch_bounds__(z_threads<T, N, B>())
            int *__restrict__ err) {
   using V = typename Cx<T>::type;
   constexpr int NTHR = z_threads<T, N, B>();
+  static_assert(tma_tile_ok<V, N, B>(), "every box starts on a 128-byte boundary");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int m = g.m;
   V *bufs[2];
@@ -683,7 +710,7 @@ __global__ void __launch_bounds__(z_threads<T, N, B>())
     mbar_expect_tx(&bar[0], bytes);
     for (int s = 0; s < m; ++s)
 #pragma unroll
-      for (int c = 0; c < N; c += kTmaRows)
+      for (int c = 0; c < N; c += tma_rows(N))
         tma_load_3d(bufs[0] + s * N * B + c * B, &tm, &bar[0], 2 * (t % nkx) * B, t / nkx, s * g.N2 + c);
   }
   for (int q = tid; q < N; q += NTHR) tw[q] = twg[q];
@@ -696,7 +723,7 @@ __global__ void __launch_bounds__(z_threads<T, N, B>())
       mbar_expect_tx(&bar[cur ^ 1], bytes);
       for (int s = 0; s < m; ++s)
 #pragma unroll
-        for (int c = 0; c < N; c += kTmaRows)
+        for (int c = 0; c < N; c += tma_rows(N))
           tma_load_3d(bufs[cur ^ 1] + s * N * B + c * B, &tm, &bar[cur ^ 1], 2 * (tn % nkx) * B, tn / nkx,
                       s * g.N2 + c);
     }
@@ -723,7 +750,7 @@ __global__ void __launch_bounds__(z_threads<T, N, B>())
     if (tid == 0) {
       for (int s = 0; s < m; ++s)
 #pragma unroll
-        for (int c = 0; c < N; c += kTmaRows)
+        for (int c = 0; c < N; c += tma_rows(N))
           tma_store_3d(&tm, bufs[cur] + s * N * B + c * B, 2 * kx0, y, s * g.N2 + c);
       tma_commit();
     }

@@ -29,6 +29,7 @@
 #include "coarse_pk.cuh"
 #include "kernels.cuh"
 #include "kernels_static.cuh"
+#include "passes.cuh"
 #include "grad.cuh"
 #include "krylov.cuh"
 #include "info.cuh"
@@ -415,35 +416,6 @@ template <typename T> size_t zsmem(rism3d_ctx *c) {
   return sizeof(typename Cx<T>::type) * (size_t)(c->g.N2 + c->g.N2 * c->m * c->tl<T>().BZ);
 }
 
-// ---- shape-specialised passes
-constexpr int kStaticRX = 16;
-// y tile width: 128-byte rows (16 float2 or 8 double2); z tile width: 64-byte
-// rows, so the m-site z tile is half as large and four CTAs share an SM
-template <typename T> constexpr int static_B() { return sizeof(T) == 4 ? 16 : 8; }
-template <typename T> constexpr int static_Bz() { return sizeof(T) == 4 ? 8 : 4; }
-template <typename T, int M> constexpr size_t xs_smem() {
-  return sizeof(typename Cx<T>::type) * (size_t)(M + kStaticRX * LayRow<M, SplitRow<M>::R2>::RS);
-}
-template <typename T, int N> constexpr size_t ys_smem() {
-  return sizeof(typename Cx<T>::type) * (size_t)(N * static_B<T>() + N) + 16;
-}
-template <typename T, int MODE, int N, int B = static_Bz<T>()> size_t zs_smem(int m) {
-  return sizeof(typename Cx<T>::type) * (size_t)(m * N * B + N) + zf_stage_bytes<T, MODE, N, B>(m) + 16;
-}
-template <typename T, int MODE, int N> size_t zsp_smem(int m) {  // two tile buffers, two mbarriers
-  return sizeof(typename Cx<T>::type) * (size_t)(2 * m * N * static_Bz<T>() + N) +
-         zf_stage_bytes<T, MODE, N, static_Bz<T>()>(m) + 16;
-}
-// Lengths with shape-specialised passes: the coarse grids (48, 96) and the
-// even 2^a 3^b grids of the many-solute workloads whose two-step split fits
-// the register transforms (108 and 162 do not: no split of 54 / odd 81).
-bool static_len_x(int M) {
-  return M == 24 || M == 32 || M == 36 || M == 48 || M == 64 || M == 72 || M == 96 || M == 128 || M == 256;
-}
-bool static_len_yz(int N) {
-  return N == 48 || N == 64 || N == 72 || N == 96 || N == 128 || N == 144 || N == 192 || N == 256 || N == 512;
-}
-
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {  // thread-safe one-time lookup
     void *p = nullptr;
@@ -467,9 +439,7 @@ void make_tmap(rism3d_ctx *c, CUtensorMap *tm, bool fp64, int B, int by, int bz)
   const size_t es = fp64 ? 8 : 4;
   cuuint64_t dims[3] = {(cuuint64_t)(2 * G.Nhp), (cuuint64_t)G.N1, (cuuint64_t)G.N2 * G.m};
   cuuint64_t strides[2] = {(cuuint64_t)(2 * G.Nhp) * es, (cuuint64_t)(2 * G.Nhp) * G.N1 * es};
-  // a box spans at most 256 elements per dimension (the kernels move
-  // 512-point tiles as two boxes)
-  cuuint32_t box[3] = {(cuuint32_t)(2 * B), (cuuint32_t)std::min(by, 256), (cuuint32_t)std::min(bz, 256)};
+  cuuint32_t box[3] = {(cuuint32_t)(2 * B), (cuuint32_t)tma_rows(by), (cuuint32_t)tma_rows(bz)};
   cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = encode_fn()(tm, fp64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                                  c->W, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -485,16 +455,14 @@ template <typename T, bool INV> void launch_y(rism3d_ctx *c) {
   TimeScope ts(c, TK_Y, sizeof(T) == 8 ? 0 : 1);
   auto *W = c->work<T>();
   if (c->stat[sizeof(T) == 8 ? 0 : 1]) {
-    constexpr int B = static_B<T>();
-    dim3 grid((c->g.Nh + B - 1) / B, c->g.N2, c->m);
     const CUtensorMap &tm = c->tmy[sizeof(T) == 8 ? 0 : 1];
     const auto *tw = static_cast<const typename Cx<T>::type *>(c->plan<T>(1).tw);
     switch (c->g.N1) {
-#define Y_CASE(N)                                                                                   \
-  case N:                                                                                           \
-    k_y_s<T, INV, N, B><<<grid, Split<N>::R1 * B, ys_smem<T, N>(), c->stream>>>(c->g, tm, tw, c->d_err); \
+#define Y_CASE(N)                                                       \
+  case N:                                                               \
+    YPass<T, N>::run(INV, c->g, tm, tw, c->d_err, c->stream);           \
     break;
-      Y_CASE(48) Y_CASE(64) Y_CASE(72) Y_CASE(96) Y_CASE(128) Y_CASE(144) Y_CASE(192) Y_CASE(256) Y_CASE(512)
+      RISM_YZ_LENS(Y_CASE)
 #undef Y_CASE
     }
     CKL();
@@ -564,28 +532,14 @@ template <typename T, int MODE> void launch_z(rism3d_ctx *c) {
   auto *W = c->work<T>();
   const ZParams<T> zp = zparams<T>(c, MODE == MODE_F);
   if (c->stat[sizeof(T) == 8 ? 0 : 1]) {
-    constexpr int BW = static_Bz<T>(), BN = static_Bz<T>() / 2;  // wide / narrow tiles
-    const int B = c->zb[sizeof(T) == 8 ? 0 : 1];
-    dim3 grid((c->g.Nh + B - 1) / B, c->g.N1);
-    const CUtensorMap &tm = c->tmz[sizeof(T) == 8 ? 0 : 1];
+    const int pr = sizeof(T) == 8 ? 0 : 1;
     const auto *tw = static_cast<const typename Cx<T>::type *>(c->plan<T>(2).tw);
     switch (c->g.N2) {
-#define Z_CASE(N)                                                                                          \
-  case N:                                                                                                  \
-    if (B == BW && c->zpers[sizeof(T) == 8 ? 0 : 1]) {                                                     \
-      const unsigned nt = (unsigned)(((c->g.Nh + BW - 1) / BW) * c->g.N1);                                 \
-      const size_t sm = zsp_smem<T, MODE, N>(c->m);                                                               \
-      const void *fn = (const void *)k_z_sp<T, MODE, N, BW, 3>;                                             \
-      k_z_sp<T, MODE, N, BW, 3><<<persistent_grid(fn, sm, nt, z_threads<T, N, BW>()), z_threads<T, N, BW>(), sm, \
-                                  c->stream>>>(c->g, tm, tw, zp, c->d_err);                                \
-    } else if (B == BW)                                                                                    \
-      k_z_s<T, MODE, N, BW, 3><<<grid, z_threads<T, N, BW>(), zs_smem<T, MODE, N, BW>(c->m), c->stream>>>(c->g, tm, tw, \
-                                                                                               zp, c->d_err); \
-    else                                                                                                   \
-      k_z_s<T, MODE, N, BN, 3><<<grid, z_threads<T, N, BN>(), zs_smem<T, MODE, N, BN>(c->m), c->stream>>>(c->g, tm, tw, \
-                                                                                               zp, c->d_err); \
+#define Z_CASE(N)                                                                                           \
+  case N:                                                                                                   \
+    ZPass<T, N>::run(MODE, c->zb[pr], c->zpers[pr], c->g, c->tmz[pr], tw, zp, c->d_err, c->stream);         \
     break;
-      Z_CASE(48) Z_CASE(64) Z_CASE(72) Z_CASE(96) Z_CASE(128) Z_CASE(144) Z_CASE(192) Z_CASE(256) Z_CASE(512)
+      RISM_YZ_LENS(Z_CASE)
 #undef Z_CASE
     }
     CKL();
@@ -625,20 +579,18 @@ int pipeline(rism3d_ctx *c, const T *A, const T *Bv, T p, T sub, T *out) {
   const int rows = c->g.N1 * c->g.N2;
   auto *W = c->work<T>();
   const bool st = c->stat[sizeof(T) == 8 ? 0 : 1];
-  const int RX = st ? kStaticRX : c->tl<T>().RX;
+  const int RX = st ? x_rows(c->g.M) : c->tl<T>().RX;
   dim3 gx((rows + RX - 1) / RX, c->m);
   const auto *twx = static_cast<const typename Cx<T>::type *>(c->plan<T>(0).tw);
   {
     TimeScope ts(c, TK_XFWD, sizeof(T) == 8 ? 0 : 1);
     if (st) {
       switch (c->g.M) {
-#define XF_CASE(M)                                                                                     \
-  case M:                                                                                              \
-    k_xfwd_s<T, MODE, M, kStaticRX><<<gx, 256, xs_smem<T, M>(), c->stream>>>(c->g, A, Bv, p, c->pd.closure, \
-                                                                             W, postw<T>(c), twx);      \
+#define XF_CASE(M)                                                                                         \
+  case M:                                                                                                  \
+    XPass<T, M>::fwd(MODE, c->g, A, Bv, p, c->pd.closure, W, postw<T>(c), twx, c->stream);                 \
     break;
-        XF_CASE(24) XF_CASE(32) XF_CASE(36) XF_CASE(48) XF_CASE(64) XF_CASE(72) XF_CASE(96) XF_CASE(128)
-        XF_CASE(256)
+        RISM_X_LENS(XF_CASE)
 #undef XF_CASE
       }
     } else {
@@ -655,13 +607,11 @@ int pipeline(rism3d_ctx *c, const T *A, const T *Bv, T p, T sub, T *out) {
     const T scale = (T)(1.0 / (double)c->g.Nr);
     if (st) {
       switch (c->g.M) {
-#define XI_CASE(M)                                                                                            \
-  case M:                                                                                                     \
-    k_xinv_s<T, M, kStaticRX><<<gx, 256, xs_smem<T, M>(), c->stream>>>(c->g, W, A, out, scale, sub, postw<T>(c), \
-                                                                       twx, c->npart);                        \
+#define XI_CASE(M)                                                                                         \
+  case M:                                                                                                  \
+    XPass<T, M>::inv(c->g, W, A, out, scale, sub, postw<T>(c), twx, c->npart, c->stream);                  \
     break;
-        XI_CASE(24) XI_CASE(32) XI_CASE(36) XI_CASE(48) XI_CASE(64) XI_CASE(72) XI_CASE(96) XI_CASE(128)
-        XI_CASE(256)
+        RISM_X_LENS(XI_CASE)
 #undef XI_CASE
       }
     } else {
@@ -2216,14 +2166,14 @@ template <typename T> void tune_precision(rism3d_ctx *c, const T *A, const T *Bv
     // in flight per SM)
     const int wide = c->zb[pr];
     float n_ms = 1e30f;
-    if (pr == 1) {  // FP32 only: 64-byte rows (FP64 would drop to 32-thread CTAs)
+    if (pr == 1 && z_has_variants(G.N2)) {  // FP32 only: 64-byte rows (FP64 would drop to 32-thread CTAs)
       c->zb[pr] = wide / 2;
       make_tmap(c, &c->tmz[pr], pr == 0, c->zb[pr], 1, G.N2);
       n_ms = time_ms(c, run, reps);
     }
     if (n_ms < 0.95f * s_ms) {
       s_ms = n_ms;
-    } else {
+    } else if (z_has_variants(G.N2)) {
       c->zb[pr] = wide;
       make_tmap(c, &c->tmz[pr], pr == 0, wide, 1, G.N2);
       // persistent double-buffered CTAs for the wide tiles
@@ -2243,7 +2193,7 @@ void force_z_persistent(rism3d_ctx *c) {
   if (!env || (env[0] != '0' && env[0] != '1')) return;
   const int wide[2] = {static_Bz<double>(), static_Bz<float>()};
   for (int pr = 0; pr < 2; ++pr) {
-    if (!c->stat[pr]) continue;
+    if (!c->stat[pr] || !z_has_variants(c->g.N2)) continue;
     if (c->zb[pr] != wide[pr]) {
       c->zb[pr] = wide[pr];
       make_tmap(c, &c->tmz[pr], pr == 0, wide[pr], 1, c->g.N2);
@@ -2575,111 +2525,31 @@ int create_impl(const rism3d_problem *pd, int m, const rism3d_site *solvent, int
     OPTIN_Z(float)
 #undef OPTIN_Z
     if (c->stat[0]) {
-      need = std::max({xs_smem<double, 256>(), ys_smem<double, 512>(), zsp_smem<double, MODE_F, 512>(m),
-                       zsp_smem<double, MODE_F, 256>(m), xs_smem<float, 256>(), ys_smem<float, 512>()});
-#define OPTIN_S(T)                                               \
-  allow((const void *)k_xfwd_s<T, MODE_F, 24, kStaticRX>);       \
-  allow((const void *)k_xfwd_s<T, MODE_J, 24, kStaticRX>);       \
-  allow((const void *)k_xinv_s<T, 24, kStaticRX>);               \
-  allow((const void *)k_xfwd_s<T, MODE_F, 32, kStaticRX>);       \
-  allow((const void *)k_xfwd_s<T, MODE_J, 32, kStaticRX>);       \
-  allow((const void *)k_xinv_s<T, 32, kStaticRX>);               \
-  allow((const void *)k_xfwd_s<T, MODE_F, 36, kStaticRX>);       \
-  allow((const void *)k_xfwd_s<T, MODE_J, 36, kStaticRX>);       \
-  allow((const void *)k_xinv_s<T, 36, kStaticRX>);               \
-  allow((const void *)k_xfwd_s<T, MODE_F, 48, kStaticRX>);       \
-  allow((const void *)k_xfwd_s<T, MODE_J, 48, kStaticRX>);       \
-  allow((const void *)k_xinv_s<T, 48, kStaticRX>);               \
-  allow((const void *)k_xfwd_s<T, MODE_F, 64, kStaticRX>);       \
-  allow((const void *)k_xfwd_s<T, MODE_J, 64, kStaticRX>);       \
-  allow((const void *)k_xinv_s<T, 64, kStaticRX>);               \
-  allow((const void *)k_xfwd_s<T, MODE_F, 72, kStaticRX>);       \
-  allow((const void *)k_xfwd_s<T, MODE_J, 72, kStaticRX>);       \
-  allow((const void *)k_xinv_s<T, 72, kStaticRX>);               \
-  allow((const void *)k_xfwd_s<T, MODE_F, 96, kStaticRX>);       \
-  allow((const void *)k_xfwd_s<T, MODE_J, 96, kStaticRX>);       \
-  allow((const void *)k_xinv_s<T, 96, kStaticRX>);               \
-  allow((const void *)k_xfwd_s<T, MODE_F, 128, kStaticRX>);      \
-  allow((const void *)k_xfwd_s<T, MODE_J, 128, kStaticRX>);      \
-  allow((const void *)k_xinv_s<T, 128, kStaticRX>);              \
-  allow((const void *)k_xfwd_s<T, MODE_F, 256, kStaticRX>);      \
-  allow((const void *)k_xfwd_s<T, MODE_J, 256, kStaticRX>);      \
-  allow((const void *)k_xinv_s<T, 256, kStaticRX>);              \
-  allow((const void *)k_y_s<T, false, 512, static_B<T>()>);      \
-  allow((const void *)k_y_s<T, true, 512, static_B<T>()>);       \
-  allow((const void *)k_z_s<T, MODE_F, 512, static_Bz<T>(), 3>); \
-  allow((const void *)k_z_s<T, MODE_J, 512, static_Bz<T>(), 3>); \
-  allow((const void *)k_z_s<T, MODE_F, 512, static_Bz<T>() / 2, 3>); \
-  allow((const void *)k_z_s<T, MODE_J, 512, static_Bz<T>() / 2, 3>); \
-  allow((const void *)k_z_sp<T, MODE_F, 512, static_Bz<T>(), 3>);   \
-  allow((const void *)k_z_sp<T, MODE_J, 512, static_Bz<T>(), 3>);   \
-  allow((const void *)k_y_s<T, false, 48, static_B<T>()>);       \
-  allow((const void *)k_y_s<T, true, 48, static_B<T>()>);        \
-  allow((const void *)k_z_s<T, MODE_F, 48, static_Bz<T>(), 3>);  \
-  allow((const void *)k_z_s<T, MODE_J, 48, static_Bz<T>(), 3>);  \
-  allow((const void *)k_y_s<T, false, 64, static_B<T>()>);       \
-  allow((const void *)k_y_s<T, true, 64, static_B<T>()>);        \
-  allow((const void *)k_z_s<T, MODE_F, 64, static_Bz<T>(), 3>);  \
-  allow((const void *)k_z_s<T, MODE_J, 64, static_Bz<T>(), 3>);  \
-  allow((const void *)k_y_s<T, false, 72, static_B<T>()>);       \
-  allow((const void *)k_y_s<T, true, 72, static_B<T>()>);        \
-  allow((const void *)k_z_s<T, MODE_F, 72, static_Bz<T>(), 3>);  \
-  allow((const void *)k_z_s<T, MODE_J, 72, static_Bz<T>(), 3>);  \
-  allow((const void *)k_y_s<T, false, 96, static_B<T>()>);       \
-  allow((const void *)k_y_s<T, true, 96, static_B<T>()>);        \
-  allow((const void *)k_z_s<T, MODE_F, 96, static_Bz<T>(), 3>);  \
-  allow((const void *)k_z_s<T, MODE_J, 96, static_Bz<T>(), 3>);  \
-  allow((const void *)k_y_s<T, false, 128, static_B<T>()>);      \
-  allow((const void *)k_y_s<T, true, 128, static_B<T>()>);       \
-  allow((const void *)k_z_s<T, MODE_F, 128, static_Bz<T>(), 3>); \
-  allow((const void *)k_z_s<T, MODE_J, 128, static_Bz<T>(), 3>); \
-  allow((const void *)k_y_s<T, false, 144, static_B<T>()>);      \
-  allow((const void *)k_y_s<T, true, 144, static_B<T>()>);       \
-  allow((const void *)k_z_s<T, MODE_F, 144, static_Bz<T>(), 3>); \
-  allow((const void *)k_z_s<T, MODE_J, 144, static_Bz<T>(), 3>); \
-  allow((const void *)k_y_s<T, false, 192, static_B<T>()>);      \
-  allow((const void *)k_y_s<T, true, 192, static_B<T>()>);       \
-  allow((const void *)k_z_s<T, MODE_F, 192, static_Bz<T>(), 3>); \
-  allow((const void *)k_z_s<T, MODE_J, 192, static_Bz<T>(), 3>); \
-  allow((const void *)k_y_s<T, false, 256, static_B<T>()>);      \
-  allow((const void *)k_y_s<T, true, 256, static_B<T>()>);       \
-  allow((const void *)k_z_s<T, MODE_F, 256, static_Bz<T>(), 3>); \
-  allow((const void *)k_z_s<T, MODE_J, 256, static_Bz<T>(), 3>); \
-  allow((const void *)k_z_s<T, MODE_F, 48, static_Bz<T>() / 2, 3>);  \
-  allow((const void *)k_z_s<T, MODE_J, 48, static_Bz<T>() / 2, 3>);  \
-  allow((const void *)k_z_s<T, MODE_F, 64, static_Bz<T>() / 2, 3>);  \
-  allow((const void *)k_z_s<T, MODE_J, 64, static_Bz<T>() / 2, 3>);  \
-  allow((const void *)k_z_s<T, MODE_F, 72, static_Bz<T>() / 2, 3>);  \
-  allow((const void *)k_z_s<T, MODE_J, 72, static_Bz<T>() / 2, 3>);  \
-  allow((const void *)k_z_s<T, MODE_F, 96, static_Bz<T>() / 2, 3>);  \
-  allow((const void *)k_z_s<T, MODE_J, 96, static_Bz<T>() / 2, 3>);  \
-  allow((const void *)k_z_s<T, MODE_F, 128, static_Bz<T>() / 2, 3>); \
-  allow((const void *)k_z_s<T, MODE_J, 128, static_Bz<T>() / 2, 3>); \
-  allow((const void *)k_z_s<T, MODE_F, 144, static_Bz<T>() / 2, 3>); \
-  allow((const void *)k_z_s<T, MODE_J, 144, static_Bz<T>() / 2, 3>); \
-  allow((const void *)k_z_s<T, MODE_F, 192, static_Bz<T>() / 2, 3>); \
-  allow((const void *)k_z_s<T, MODE_J, 192, static_Bz<T>() / 2, 3>); \
-  allow((const void *)k_z_s<T, MODE_F, 256, static_Bz<T>() / 2, 3>); \
-  allow((const void *)k_z_s<T, MODE_J, 256, static_Bz<T>() / 2, 3>); \
-  allow((const void *)k_z_sp<T, MODE_F, 48, static_Bz<T>(), 3>);    \
-  allow((const void *)k_z_sp<T, MODE_J, 48, static_Bz<T>(), 3>);    \
-  allow((const void *)k_z_sp<T, MODE_F, 64, static_Bz<T>(), 3>);    \
-  allow((const void *)k_z_sp<T, MODE_J, 64, static_Bz<T>(), 3>);    \
-  allow((const void *)k_z_sp<T, MODE_F, 72, static_Bz<T>(), 3>);    \
-  allow((const void *)k_z_sp<T, MODE_J, 72, static_Bz<T>(), 3>);    \
-  allow((const void *)k_z_sp<T, MODE_F, 96, static_Bz<T>(), 3>);    \
-  allow((const void *)k_z_sp<T, MODE_J, 96, static_Bz<T>(), 3>);    \
-  allow((const void *)k_z_sp<T, MODE_F, 128, static_Bz<T>(), 3>);   \
-  allow((const void *)k_z_sp<T, MODE_J, 128, static_Bz<T>(), 3>);   \
-  allow((const void *)k_z_sp<T, MODE_F, 144, static_Bz<T>(), 3>);   \
-  allow((const void *)k_z_sp<T, MODE_J, 144, static_Bz<T>(), 3>);   \
-  allow((const void *)k_z_sp<T, MODE_F, 192, static_Bz<T>(), 3>);   \
-  allow((const void *)k_z_sp<T, MODE_J, 192, static_Bz<T>(), 3>);   \
-  allow((const void *)k_z_sp<T, MODE_F, 256, static_Bz<T>(), 3>);   \
-  allow((const void *)k_z_sp<T, MODE_J, 256, static_Bz<T>(), 3>);
-      OPTIN_S(double)
-      OPTIN_S(float)
-#undef OPTIN_S
+      std::vector<PassKernel> ks;
+      switch (G.M) {
+#define ALLOW_X(M)                      \
+  case M:                               \
+    XPass<double, M>::kernels(ks);      \
+    XPass<float, M>::kernels(ks);       \
+    break;
+        RISM_X_LENS(ALLOW_X)
+#undef ALLOW_X
+      }
+#define ALLOW_Y(N)                      \
+  case N:                               \
+    YPass<double, N>::kernels(ks);      \
+    YPass<float, N>::kernels(ks);       \
+    break;
+      switch (G.N1) { RISM_YZ_LENS(ALLOW_Y) }
+#undef ALLOW_Y
+#define ALLOW_Z(N)                      \
+  case N:                               \
+    ZPass<double, N>::kernels(m, ks);   \
+    ZPass<float, N>::kernels(m, ks);    \
+    break;
+      switch (G.N2) { RISM_YZ_LENS(ALLOW_Z) }
+#undef ALLOW_Z
+      for (const PassKernel &k : ks) allow_smem(k.fn, k.smem);
     }
     autotune(c);
     // two-grid preconditioner: a copy of the problem on a coarse grid.  The

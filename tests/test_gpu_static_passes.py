@@ -14,7 +14,9 @@ pytestmark = pytest.mark.gpu
 from bgy3d_b200 import RismContext  # noqa: E402
 
 GRIDS = [(48, 64, 72), (72, 48, 64), (64, 72, 48), (96, 128, 144), (144, 96, 128), (128, 144, 96), (192, 256, 48),
-         (48, 192, 256)]
+         (48, 192, 256), (32, 36, 54), (54, 32, 36), (36, 54, 32), (54, 108, 162), (108, 162, 216), (162, 216, 108),
+         (216, 288, 32), (288, 324, 36), (324, 32, 288), (384, 36, 324), (36, 384, 432), (432, 32, 486), (486, 432, 32),
+         (32, 486, 384)]
 
 
 def make(meta, arr, m, s, generic, monkeypatch):
