@@ -152,8 +152,9 @@ __device__ __forceinline__ void pk_block_sum(double s, double *part) {
 
 // The split of the x-phase transforms (measured: the larger first radix of
 // Split beats SplitRow at 48-row items of 32-point rows, and ties with it at
-// the plane form's 64-row items).
-template <int M> using PkSplit = Split<M>;
+// the plane form's 64-row items; 16, 18 and 27 points, where Split has no
+// balanced pair, take SplitRow's).
+template <int M> using PkSplit = std::conditional_t<M == 16 || M == 18 || M == 27, SplitRow<M>, Split<M>>;
 
 // Rows of the x phases per work item: about one item per CTA of a 2 x 148
 // grid for m = 3, a multiple of 8, at most 4 float4 of a vector per thread.
@@ -167,9 +168,17 @@ template <int M> __host__ __device__ constexpr int pk_rx() {
 // of each).
 template <int CNT> __host__ __device__ constexpr int pk_group() { return CNT <= 2 ? 4 : 2; }
 
-// The column tile of the plane phases: [N][M + 2] complex (y, kx), the row
-// stride of W (Nhp = M + 2 for the even M here), after the row tile.
-template <int M> __host__ __device__ constexpr int pk_ncp() { return M + 2; }
+// The column tile of the plane phases: [N][Nhp] complex (y, kx), the row
+// stride of W (Nhp = M + 1 rounded up to even), after the row tile.
+template <int M> __host__ __device__ constexpr int pk_ncp() { return (M + 2) & ~1; }
+
+// The rows of an item as float4: RX rows of M / 2 each, or, in the plane form,
+// the whole contiguous plane (M^2 float4, N = 2 M rows), whose rows may end
+// inside a float4 where M is odd.
+template <int M, int RX, bool PLANE> __host__ __device__ constexpr int pk_vec() { return PLANE ? M * M : RX * (M / 2); }
+// Complex value c (in memory order) of an item: its row and index in the row.
+template <int M> __device__ __forceinline__ int pk_row(int c) { return c / M; }
+template <int M> __device__ __forceinline__ int pk_col(int c) { return c % M; }
 
 // XF: V_j -= sum_{i<nu} cf_i V_i (nu = 0: no update) with |V_j|^2 into nrm2;
 // then, if fft, c'_H V_j and the r2c along x into W.  PLANE (RX = N, the
@@ -182,8 +191,8 @@ __device__ __forceinline__ void pk_xf(const PkArgs &a, float *const *V, int j, i
   using Lay = LayRow<M, PkSplit<M>::R2>;
   constexpr int NCP = pk_ncp<M>();
   float2 *T = buf + RX * Lay::RS;  // PLANE: the column tile
-  constexpr int PER_ROW = M / 2;  // float4 per row (two complex values)
-  constexpr int CNT = (RX * PER_ROW + kPkThreads - 1) / kPkThreads;
+  constexpr int NV = pk_vec<M, RX, PLANE>();  // float4 (two complex values) per item
+  constexpr int CNT = (NV + kPkThreads - 1) / kPkThreads;
   constexpr int H = M / 2 + 1;
   const int tid = threadIdx.x;
   const int rows_total = a.g.m * a.g.N1 * a.g.N2;
@@ -191,14 +200,14 @@ __device__ __forceinline__ void pk_xf(const PkArgs &a, float *const *V, int j, i
   float *w = V[j];
   for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
     const int row0 = item * RX;
+    const long long base = (long long)row0 * (2 * M);  // first value of the item
+    const int nvec = PLANE ? NV : min(NV, (rows_total - row0) * (M / 2));
     float4 x[CNT];
 #pragma unroll
     for (int it = 0; it < CNT; ++it) {
       const int e = tid + it * kPkThreads;
-      const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
       x[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (e < RX * PER_ROW && row0 + row < rows_total)
-        x[it] = *reinterpret_cast<const float4 *>(w + (long long)(row0 + row) * a.g.N0 + 2 * jj);
+      if (e < nvec) x[it] = *reinterpret_cast<const float4 *>(w + base + 4 * e);
     }
     if (nu > 0) {
       // the basis vectors in groups, all loads of a group in flight
@@ -210,9 +219,8 @@ __device__ __forceinline__ void pk_xf(const PkArgs &a, float *const *V, int j, i
 #pragma unroll
           for (int it = 0; it < CNT; ++it) {
             const int e = tid + it * kPkThreads;
-            const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
-            if (i0 + u < nu && e < RX * PER_ROW && row0 + row < rows_total)
-              b[u][it] = *reinterpret_cast<const float4 *>(V[i0 + u] + (long long)(row0 + row) * a.g.N0 + 2 * jj);
+            if (i0 + u < nu && e < nvec)
+              b[u][it] = *reinterpret_cast<const float4 *>(V[i0 + u] + base + 4 * e);
             else
               b[u][it] = make_float4(0.f, 0.f, 0.f, 0.f);
           }
@@ -231,9 +239,8 @@ __device__ __forceinline__ void pk_xf(const PkArgs &a, float *const *V, int j, i
 #pragma unroll
       for (int it = 0; it < CNT; ++it) {
         const int e = tid + it * kPkThreads;
-        const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
-        if (e < RX * PER_ROW && row0 + row < rows_total) {
-          *reinterpret_cast<float4 *>(w + (long long)(row0 + row) * a.g.N0 + 2 * jj) = x[it];
+        if (e < nvec) {
+          *reinterpret_cast<float4 *>(w + base + 4 * e) = x[it];
           nrm2 += (double)(x[it].x * x[it].x + x[it].y * x[it].y + x[it].z * x[it].z + x[it].w * x[it].w);
         }
       }
@@ -242,16 +249,15 @@ __device__ __forceinline__ void pk_xf(const PkArgs &a, float *const *V, int j, i
 #pragma unroll
     for (int it = 0; it < CNT; ++it) {
       const int e = tid + it * kPkThreads;
-      if (e >= RX * PER_ROW) break;
-      const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
+      if (e >= NV) break;
       float2 z0 = make_float2(0.f, 0.f), z1 = make_float2(0.f, 0.f);
-      if (row0 + row < rows_total) {
-        const float4 dd = *reinterpret_cast<const float4 *>(a.d + (long long)(row0 + row) * a.g.N0 + 2 * jj);
+      if (e < nvec) {
+        const float4 dd = *reinterpret_cast<const float4 *>(a.d + base + 4 * e);
         z0 = make_float2(dd.x * x[it].x, dd.y * x[it].y);
         z1 = make_float2(dd.z * x[it].z, dd.w * x[it].w);
       }
-      buf[Lay::at(jj, row)] = z0;
-      buf[Lay::at(jj + 1, row)] = z1;
+      buf[Lay::at(pk_col<M>(2 * e), pk_row<M>(2 * e))] = z0;
+      buf[Lay::at(pk_col<M>(2 * e + 1), pk_row<M>(2 * e + 1))] = z1;
     }
     __syncthreads();
     fft2<M, RX, kPkThreads, false, false, Lay, PkSplit<M>>(buf, tw);
@@ -293,8 +299,8 @@ __device__ __forceinline__ void pk_xi(const PkArgs &a, float *const *V, int j, f
   using Lay = LayRow<M, PkSplit<M>::R2>;
   constexpr int NCP = pk_ncp<M>();
   float2 *T = buf + RX * Lay::RS;  // PLANE: the column tile
-  constexpr int PER_ROW = M / 2;
-  constexpr int CNT = (RX * PER_ROW + kPkThreads - 1) / kPkThreads;
+  constexpr int NV = pk_vec<M, RX, PLANE>();
+  constexpr int CNT = (NV + kPkThreads - 1) / kPkThreads;
   constexpr int GV = pk_group<CNT>();
   constexpr int H = M / 2 + 1;
   const int tid = threadIdx.x;
@@ -306,13 +312,13 @@ __device__ __forceinline__ void pk_xi(const PkArgs &a, float *const *V, int j, f
   const int nv = j + 1;
   for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
     const int row0 = item * RX;
+    const long long base = (long long)row0 * (2 * M);  // first value of the item
+    const int nvec = PLANE ? NV : min(NV, (rows_total - row0) * (M / 2));
     float4 rin[CNT];
 #pragma unroll
     for (int it = 0; it < CNT; ++it) {
       const int e = tid + it * kPkThreads;
-      const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
-      if (e < RX * PER_ROW && row0 + row < rows_total)
-        rin[it] = *reinterpret_cast<const float4 *>(vin + (long long)(row0 + row) * a.g.N0 + 2 * jj);
+      if (e < nvec) rin[it] = *reinterpret_cast<const float4 *>(vin + base + 4 * e);
     }
     if constexpr (PLANE) {
       const float4 *src = reinterpret_cast<const float4 *>(a.W + (long long)item * N * NCP);
@@ -346,13 +352,13 @@ __device__ __forceinline__ void pk_xi(const PkArgs &a, float *const *V, int j, f
 #pragma unroll
     for (int it = 0; it < CNT; ++it) {
       const int e = tid + it * kPkThreads;
-      const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
       o[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (e < RX * PER_ROW && row0 + row < rows_total) {
-        const float2 z0 = buf[Lay::at(jj, row)], z1 = buf[Lay::at(jj + 1, row)];
+      if (e < nvec) {
+        const float2 z0 = buf[Lay::at(pk_col<M>(2 * e), pk_row<M>(2 * e))];
+        const float2 z1 = buf[Lay::at(pk_col<M>(2 * e + 1), pk_row<M>(2 * e + 1))];
         o[it] = make_float4(z0.x * sc - sub * rin[it].x, z0.y * sc - sub * rin[it].y, z1.x * sc - sub * rin[it].z,
                             z1.y * sc - sub * rin[it].w);
-        *reinterpret_cast<float4 *>(vout + (long long)(row0 + row) * a.g.N0 + 2 * jj) = o[it];
+        *reinterpret_cast<float4 *>(vout + base + 4 * e) = o[it];
       }
     }
     // dots against the basis, GV vectors' loads in flight at a time; each
@@ -364,9 +370,8 @@ __device__ __forceinline__ void pk_xi(const PkArgs &a, float *const *V, int j, f
 #pragma unroll
         for (int it = 0; it < CNT; ++it) {
           const int e = tid + it * kPkThreads;
-          const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
-          if (i0 + u < nv && e < RX * PER_ROW && row0 + row < rows_total)
-            b[u][it] = *reinterpret_cast<const float4 *>(V[i0 + u] + (long long)(row0 + row) * a.g.N0 + 2 * jj);
+          if (i0 + u < nv && e < nvec)
+            b[u][it] = *reinterpret_cast<const float4 *>(V[i0 + u] + base + 4 * e);
           else
             b[u][it] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
@@ -515,7 +520,7 @@ template <int M, int N, bool PLANE = false> __host__ __device__ constexpr size_t
   constexpr size_t ys = PLANE ? 0 : (size_t)(kPkThreads / (Split<N>::R1 * 16)) * N * 16;
   constexpr size_t zs = (size_t)(kPkThreads / (PkZSplit<N>::R1 * kPkBz * 3)) * 3 * N * kPkBz;
   constexpr size_t tile = xs > ys ? (xs > zs ? xs : zs) : (ys > zs ? ys : zs);
-  return sizeof(float2) * (M + 2 * N + tile);
+  return sizeof(float2) * (M + M % 2 + 2 * N + tile);
 }
 
 // Grid barriers of one GMRES step: XF Y Z YI XI, or XY Z YXI with PLANE.
@@ -531,7 +536,7 @@ __global__ void __launch_bounds__(kPkThreads, 2) k_coarse_gmres(PkArgs a) {
   float2 *twx = reinterpret_cast<float2 *>(smem_raw);
   float2 *twy = twx + M;
   float2 *twz = twy + N;
-  float2 *tile = twz + N;
+  float2 *tile = twz + N + M % 2;  // on a 16-byte boundary
   __shared__ double sH[kPkMaxSteps * (kPkMaxSteps + 1)];
   __shared__ double sS[kPkMaxSteps + 1];  // s_j = |V_j|
   __shared__ double sD[kVecMax];          // summed dot partials

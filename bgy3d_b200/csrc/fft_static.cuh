@@ -87,7 +87,8 @@ template <int N> struct Split {
 // (16 x 4 over 16 columns: 64 DFTs for 256 threads) and holds twice the
 // values per thread.
 template <int N> struct SplitSq {
-  static constexpr int R1 = N == 48 ? 8 : N == 64 ? 8 : N == 72 ? 8 : N == 96 ? 12 : N == 128 ? 16 : Split<N>::R1;
+  static constexpr int R1 = N == 32 ? 8 : N == 36 ? 6 : N == 48 ? 8 : N == 54 ? 9 : N == 64 ? 8 : N == 72 ? 8 : N == 96 ? 12
+                            : N == 128 ? 16 : Split<N>::R1;
   static constexpr int R2 = N / R1;
 };
 

@@ -340,7 +340,7 @@ int rism3d_coarse_grid(rism3d_ctx *ctx, int *n);
 
 /* How the last coarse solve of the preconditioner ran (diagnostics; no
    counterpart in the reference): 2 = one persistent cooperative kernel
-   (cubic coarse grids of 48, 64, 72, 96 or 128 points, m <= 3, coarse_steps
+   (cubic coarse grids of 32, 36, 48, 54, 64, 72, 96 or 128 points, m <= 3, coarse_steps
    <= 16, one solve per process at a time), 1 = a replayed CUDA graph of the
    step-by-step kernels, 0 = host-driven GMRES, -1 = none yet.
    RISM3D_COARSE_PERSIST=0 / RISM3D_COARSE_GRAPH=0 (environment, read when
