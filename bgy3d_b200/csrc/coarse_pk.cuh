@@ -1,5 +1,6 @@
 // coarse_pk.cuh -- the coarse solve of the two-grid preconditioner as ONE
-// persistent cooperative kernel (sm_100a).
+// persistent cooperative kernel (sm_100a): the five-phase form, used for 128^3
+// coarse grids, and what it shares with the plane form of coarse_planes.cuh.
 //
 // J_H^-1 r is k steps of GMRES from zero on the coarse problem (a 64^3 grid
 // at the 256^3 workload: every vector, the basis and the work buffer stay in
@@ -112,7 +113,9 @@ __device__ __forceinline__ bool grid_sync(unsigned *bar, unsigned gen, int *err,
 }
 
 // out[v] = sum_{b < nb} part[b * stride + v], v < nv (nv <= 32), by the whole
-// CTA in a fixed order (identical in every CTA); out in shared memory.
+// CTA in a fixed order (identical in every CTA); out in shared memory.  A
+// thread has eight of its partials in flight at once: they come from L2, and
+// a chain of dependent rounds was most of the phase's start.
 __device__ __forceinline__ void pk_sum_partials(const double *part, int stride, int nb, int nv, double *out) {
   __shared__ double red[kPkThreads];
   int lanes = 1;
@@ -121,8 +124,13 @@ __device__ __forceinline__ void pk_sum_partials(const double *part, int stride, 
   const int v = threadIdx.x % lanes, q = threadIdx.x / lanes;
   double s = 0.0;
   if (v < nv) {
-#pragma unroll 4
-    for (int b = q; b < nb; b += groups) s += part[(long long)b * stride + v];
+    for (int b0 = q; b0 < nb; b0 += 8 * groups) {
+      double p[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) p[u] = b0 + u * groups < nb ? part[(long long)(b0 + u * groups) * stride + v] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += p[u];
+    }
   }
   red[threadIdx.x] = s;
   __syncthreads();
@@ -137,24 +145,23 @@ __device__ __forceinline__ void pk_sum_partials(const double *part, int stride, 
 }
 
 // Block sum of a per-thread double into part[blockIdx.x] (thread 0 writes).
-__device__ __forceinline__ void pk_block_sum(double s, double *part) {
-  __shared__ double sm[kPkThreads / 32];
+template <int THR = kPkThreads> __device__ __forceinline__ void pk_block_sum(double s, double *part) {
+  __shared__ double sm[THR / 32];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) sm[wid] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
-    for (int w = 0; w < kPkThreads / 32; ++w) t += sm[w];
+    for (int w = 0; w < THR / 32; ++w) t += sm[w];
     part[blockIdx.x] = t;
   }
 }
 
 // The split of the x-phase transforms (measured: the larger first radix of
 // Split beats SplitRow at 48-row items of 32-point rows, and ties with it at
-// the plane form's 64-row items; 16, 18 and 27 points, where Split has no
-// balanced pair, take SplitRow's).
-template <int M> using PkSplit = std::conditional_t<M == 16 || M == 18 || M == 27, SplitRow<M>, Split<M>>;
+// the plane form's 64-row items).
+template <int M> using PkSplit = Split<M>;
 
 // Rows of the x phases per work item: about one item per CTA of a 2 x 148
 // grid for m = 3, a multiple of 8, at most 4 float4 of a vector per thread.
@@ -168,31 +175,14 @@ template <int M> __host__ __device__ constexpr int pk_rx() {
 // of each).
 template <int CNT> __host__ __device__ constexpr int pk_group() { return CNT <= 2 ? 4 : 2; }
 
-// The column tile of the plane phases: [N][Nhp] complex (y, kx), the row
-// stride of W (Nhp = M + 1 rounded up to even), after the row tile.
-template <int M> __host__ __device__ constexpr int pk_ncp() { return (M + 2) & ~1; }
-
-// The rows of an item as float4: RX rows of M / 2 each, or, in the plane form,
-// the whole contiguous plane (M^2 float4, N = 2 M rows), whose rows may end
-// inside a float4 where M is odd.
-template <int M, int RX, bool PLANE> __host__ __device__ constexpr int pk_vec() { return PLANE ? M * M : RX * (M / 2); }
-// Complex value c (in memory order) of an item: its row and index in the row.
-template <int M> __device__ __forceinline__ int pk_row(int c) { return c / M; }
-template <int M> __device__ __forceinline__ int pk_col(int c) { return c % M; }
-
 // XF: V_j -= sum_{i<nu} cf_i V_i (nu = 0: no update) with |V_j|^2 into nrm2;
-// then, if fft, c'_H V_j and the r2c along x into W.  PLANE (RX = N, the
-// rows of one (site, z) plane per item): the spectrum goes into the column
-// tile, is transformed along y as well, and the plane is stored to W whole.
-template <int M, int RX = pk_rx<M>(), bool PLANE = false, int N = RX>
+// then, if fft, c'_H V_j and the r2c along x into W.
+template <int M, int RX = pk_rx<M>()>
 __device__ __forceinline__ void pk_xf(const PkArgs &a, float *const *V, int j, int nu, const float *cf, bool fft,
-                                      float2 *buf, const float2 *tw, const float2 *twy, double &nrm2) {
-  static_assert(!PLANE || RX == N, "a plane item holds the N rows of one (site, z) plane");
+                                      float2 *buf, const float2 *tw, double &nrm2) {
   using Lay = LayRow<M, PkSplit<M>::R2>;
-  constexpr int NCP = pk_ncp<M>();
-  float2 *T = buf + RX * Lay::RS;  // PLANE: the column tile
-  constexpr int NV = pk_vec<M, RX, PLANE>();  // float4 (two complex values) per item
-  constexpr int CNT = (NV + kPkThreads - 1) / kPkThreads;
+  constexpr int PER_ROW = M / 2;  // float4 per row (two complex values)
+  constexpr int CNT = (RX * PER_ROW + kPkThreads - 1) / kPkThreads;
   constexpr int H = M / 2 + 1;
   const int tid = threadIdx.x;
   const int rows_total = a.g.m * a.g.N1 * a.g.N2;
@@ -200,14 +190,14 @@ __device__ __forceinline__ void pk_xf(const PkArgs &a, float *const *V, int j, i
   float *w = V[j];
   for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
     const int row0 = item * RX;
-    const long long base = (long long)row0 * (2 * M);  // first value of the item
-    const int nvec = PLANE ? NV : min(NV, (rows_total - row0) * (M / 2));
     float4 x[CNT];
 #pragma unroll
     for (int it = 0; it < CNT; ++it) {
       const int e = tid + it * kPkThreads;
+      const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
       x[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (e < nvec) x[it] = *reinterpret_cast<const float4 *>(w + base + 4 * e);
+      if (e < RX * PER_ROW && row0 + row < rows_total)
+        x[it] = *reinterpret_cast<const float4 *>(w + (long long)(row0 + row) * a.g.N0 + 2 * jj);
     }
     if (nu > 0) {
       // the basis vectors in groups, all loads of a group in flight
@@ -219,8 +209,9 @@ __device__ __forceinline__ void pk_xf(const PkArgs &a, float *const *V, int j, i
 #pragma unroll
           for (int it = 0; it < CNT; ++it) {
             const int e = tid + it * kPkThreads;
-            if (i0 + u < nu && e < nvec)
-              b[u][it] = *reinterpret_cast<const float4 *>(V[i0 + u] + base + 4 * e);
+            const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
+            if (i0 + u < nu && e < RX * PER_ROW && row0 + row < rows_total)
+              b[u][it] = *reinterpret_cast<const float4 *>(V[i0 + u] + (long long)(row0 + row) * a.g.N0 + 2 * jj);
             else
               b[u][it] = make_float4(0.f, 0.f, 0.f, 0.f);
           }
@@ -239,8 +230,9 @@ __device__ __forceinline__ void pk_xf(const PkArgs &a, float *const *V, int j, i
 #pragma unroll
       for (int it = 0; it < CNT; ++it) {
         const int e = tid + it * kPkThreads;
-        if (e < nvec) {
-          *reinterpret_cast<float4 *>(w + base + 4 * e) = x[it];
+        const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
+        if (e < RX * PER_ROW && row0 + row < rows_total) {
+          *reinterpret_cast<float4 *>(w + (long long)(row0 + row) * a.g.N0 + 2 * jj) = x[it];
           nrm2 += (double)(x[it].x * x[it].x + x[it].y * x[it].y + x[it].z * x[it].z + x[it].w * x[it].w);
         }
       }
@@ -249,15 +241,16 @@ __device__ __forceinline__ void pk_xf(const PkArgs &a, float *const *V, int j, i
 #pragma unroll
     for (int it = 0; it < CNT; ++it) {
       const int e = tid + it * kPkThreads;
-      if (e >= NV) break;
+      if (e >= RX * PER_ROW) break;
+      const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
       float2 z0 = make_float2(0.f, 0.f), z1 = make_float2(0.f, 0.f);
-      if (e < nvec) {
-        const float4 dd = *reinterpret_cast<const float4 *>(a.d + base + 4 * e);
+      if (row0 + row < rows_total) {
+        const float4 dd = *reinterpret_cast<const float4 *>(a.d + (long long)(row0 + row) * a.g.N0 + 2 * jj);
         z0 = make_float2(dd.x * x[it].x, dd.y * x[it].y);
         z1 = make_float2(dd.z * x[it].z, dd.w * x[it].w);
       }
-      buf[Lay::at(pk_col<M>(2 * e), pk_row<M>(2 * e))] = z0;
-      buf[Lay::at(pk_col<M>(2 * e + 1), pk_row<M>(2 * e + 1))] = z1;
+      buf[Lay::at(jj, row)] = z0;
+      buf[Lay::at(jj + 1, row)] = z1;
     }
     __syncthreads();
     fft2<M, RX, kPkThreads, false, false, Lay, PkSplit<M>>(buf, tw);
@@ -273,34 +266,23 @@ __device__ __forceinline__ void pk_xf(const PkArgs &a, float *const *V, int j, i
       O.x = (zk.y + zm.y) * 0.5f;
       O.y = -(zk.x - zm.x) * 0.5f;
       const float2 wO = cmul(a.post[kk], O);
-      float2 *row_out = PLANE ? T + row * NCP : a.W + (long long)grow * a.g.Nhp;
+      float2 *row_out = a.W + (long long)grow * a.g.Nhp;
       row_out[kk] = cadd(E, wO);
       if (M - kk != kk) row_out[M - kk] = cconj(csub(E, wO));
     }
     __syncthreads();  // buf is refilled by the next item
-    if constexpr (PLANE) {
-      fft2g<N, M + 1, kPkThreads, false, true, LayCol<N, NCP>, SplitSq<N>>(T, twy, tid, true);
-      float4 *dst = reinterpret_cast<float4 *>(a.W + (long long)item * N * NCP);
-      const float4 *src = reinterpret_cast<const float4 *>(T);
-      for (int e = tid; e < N * NCP / 2; e += kPkThreads) dst[e] = src[e];
-      __syncthreads();  // T is refilled by the next item
-    }
   }
 }
 
 // XI: V_{j+1} = sc X - sub V_j (X the c2r of W along x), with the dots
 // <V_i, V_{j+1}>, i <= j, summed per warp into sdot[i][warp] (shared, zeroed
-// by the caller).  PLANE: the item's plane of W is loaded whole into the
-// column tile and transformed back along y first.
-template <int M, int RX = pk_rx<M>(), bool PLANE = false, int N = RX>
+// by the caller).
+template <int M, int RX = pk_rx<M>()>
 __device__ __forceinline__ void pk_xi(const PkArgs &a, float *const *V, int j, float sc, float sub, float2 *buf,
-                                      const float2 *tw, const float2 *twy, double (*sdot)[kPkThreads / 32]) {
-  static_assert(!PLANE || RX == N, "a plane item holds the N rows of one (site, z) plane");
+                                      const float2 *tw, double (*sdot)[kPkThreads / 32]) {
   using Lay = LayRow<M, PkSplit<M>::R2>;
-  constexpr int NCP = pk_ncp<M>();
-  float2 *T = buf + RX * Lay::RS;  // PLANE: the column tile
-  constexpr int NV = pk_vec<M, RX, PLANE>();
-  constexpr int CNT = (NV + kPkThreads - 1) / kPkThreads;
+  constexpr int PER_ROW = M / 2;
+  constexpr int CNT = (RX * PER_ROW + kPkThreads - 1) / kPkThreads;
   constexpr int GV = pk_group<CNT>();
   constexpr int H = M / 2 + 1;
   const int tid = threadIdx.x;
@@ -312,27 +294,20 @@ __device__ __forceinline__ void pk_xi(const PkArgs &a, float *const *V, int j, f
   const int nv = j + 1;
   for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
     const int row0 = item * RX;
-    const long long base = (long long)row0 * (2 * M);  // first value of the item
-    const int nvec = PLANE ? NV : min(NV, (rows_total - row0) * (M / 2));
     float4 rin[CNT];
 #pragma unroll
     for (int it = 0; it < CNT; ++it) {
       const int e = tid + it * kPkThreads;
-      if (e < nvec) rin[it] = *reinterpret_cast<const float4 *>(vin + base + 4 * e);
-    }
-    if constexpr (PLANE) {
-      const float4 *src = reinterpret_cast<const float4 *>(a.W + (long long)item * N * NCP);
-      float4 *dst = reinterpret_cast<float4 *>(T);
-      for (int e = tid; e < N * NCP / 2; e += kPkThreads) dst[e] = src[e];
-      __syncthreads();
-      fft2g<N, M + 1, kPkThreads, true, true, LayCol<N, NCP>, SplitSq<N>>(T, twy, tid, true);
+      const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
+      if (e < RX * PER_ROW && row0 + row < rows_total)
+        rin[it] = *reinterpret_cast<const float4 *>(vin + (long long)(row0 + row) * a.g.N0 + 2 * jj);
     }
     for (int e = tid; e < RX * H; e += kPkThreads) {
       const int row = e / H, kk = e % H;
       const int grow = row0 + row;
       float2 zk = make_float2(0.f, 0.f), zm = make_float2(0.f, 0.f);
       if (grow < rows_total) {
-        const float2 *row_in = PLANE ? T + row * NCP : a.W + (long long)grow * a.g.Nhp;
+        const float2 *row_in = a.W + (long long)grow * a.g.Nhp;
         float2 xk = row_in[kk];
         float2 xm = row_in[M - kk];
         if (kk == 0) { xk.y = 0.f; xm.y = 0.f; }  // c2r reads only Re X_0, Re X_{N0/2}
@@ -352,13 +327,13 @@ __device__ __forceinline__ void pk_xi(const PkArgs &a, float *const *V, int j, f
 #pragma unroll
     for (int it = 0; it < CNT; ++it) {
       const int e = tid + it * kPkThreads;
+      const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
       o[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (e < nvec) {
-        const float2 z0 = buf[Lay::at(pk_col<M>(2 * e), pk_row<M>(2 * e))];
-        const float2 z1 = buf[Lay::at(pk_col<M>(2 * e + 1), pk_row<M>(2 * e + 1))];
+      if (e < RX * PER_ROW && row0 + row < rows_total) {
+        const float2 z0 = buf[Lay::at(jj, row)], z1 = buf[Lay::at(jj + 1, row)];
         o[it] = make_float4(z0.x * sc - sub * rin[it].x, z0.y * sc - sub * rin[it].y, z1.x * sc - sub * rin[it].z,
                             z1.y * sc - sub * rin[it].w);
-        *reinterpret_cast<float4 *>(vout + base + 4 * e) = o[it];
+        *reinterpret_cast<float4 *>(vout + (long long)(row0 + row) * a.g.N0 + 2 * jj) = o[it];
       }
     }
     // dots against the basis, GV vectors' loads in flight at a time; each
@@ -370,8 +345,9 @@ __device__ __forceinline__ void pk_xi(const PkArgs &a, float *const *V, int j, f
 #pragma unroll
         for (int it = 0; it < CNT; ++it) {
           const int e = tid + it * kPkThreads;
-          if (i0 + u < nv && e < nvec)
-            b[u][it] = *reinterpret_cast<const float4 *>(V[i0 + u] + base + 4 * e);
+          const int row = e / PER_ROW, jj = (e % PER_ROW) * 2;
+          if (i0 + u < nv && e < RX * PER_ROW && row0 + row < rows_total)
+            b[u][it] = *reinterpret_cast<const float4 *>(V[i0 + u] + (long long)(row0 + row) * a.g.N0 + 2 * jj);
           else
             b[u][it] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
@@ -483,60 +459,72 @@ __device__ __forceinline__ void pk_z(const PkArgs &a, float2 *smem, const float2
 // Least squares of a k-step Arnoldi run, in place on the CTA's shared copy
 // of H (column j at H[j * (k + 1) + i], i <= j + 1) by Givens rotations:
 // y minimises |beta e1 - H y|; then y[0] += beta, so that sum y_j V_j = x +
-// r0.  One thread; g, cs, sn are shared scratch of k + 1 entries.
-__device__ __forceinline__ void pk_lsq(int k, double *H, double beta, double *y, double *gv, double *cs,
-                                       double *sn) {
-  const int ld = k + 1;
-  for (int i = 0; i <= k; ++i) gv[i] = 0.0;
-  gv[0] = beta;
-  for (int j = 0; j < k; ++j) {
-    double *col = H + j * ld;
-    for (int i = 0; i < j; ++i) {
-      const double p = col[i], q = col[i + 1];
-      col[i] = cs[i] * p + sn[i] * q;
-      col[i + 1] = -sn[i] * p + cs[i] * q;
-    }
-    const double p = col[j], q = col[j + 1];
+// r0.  By one warp, lane j the column j: rotation i comes from column i and is
+// applied to all later columns at once, and the back substitution takes each
+// y_i off every row above it at once (one thread took 10 us for 16 steps).
+__device__ __forceinline__ void pk_lsq(int k, double *H, double beta, double *y) {
+  const int ld = k + 1, lane = threadIdx.x & 31;
+  double g = lane == 0 ? beta : 0.0;  // entry `lane` of the rotated right-hand side
+  for (int i = 0; i < k; ++i) {
+    const double p = H[i * ld + i], q = H[i * ld + i + 1];  // the same words in every lane
     const double r = hypot(p, q);
-    cs[j] = r == 0.0 ? 1.0 : p / r;
-    sn[j] = r == 0.0 ? 0.0 : q / r;
-    col[j] = r;
-    gv[j + 1] = -sn[j] * gv[j];
-    gv[j] = cs[j] * gv[j];
+    const double cs = r == 0.0 ? 1.0 : p / r, sn = r == 0.0 ? 0.0 : q / r;
+    __syncwarp();
+    if (lane >= i && lane < k) {
+      double *col = H + lane * ld;
+      const double u = col[i], v = col[i + 1];
+      col[i] = lane == i ? r : cs * u + sn * v;
+      col[i + 1] = lane == i ? 0.0 : -sn * u + cs * v;
+    }
+    const double gi = __shfl_sync(0xffffffffu, g, i);
+    if (lane == i) g = cs * gi;
+    if (lane == i + 1) g = -sn * gi;
+    __syncwarp();
   }
+  double yi = 0.0;
   for (int i = k - 1; i >= 0; --i) {
-    double s = gv[i];
-    for (int l = i + 1; l < k; ++l) s -= H[l * ld + i] * y[l];
-    y[i] = H[i * ld + i] != 0.0 ? s / H[i * ld + i] : 0.0;
+    const double d = H[i * ld + i];
+    const double t = d != 0.0 ? __shfl_sync(0xffffffffu, g, i) / d : 0.0;
+    if (lane == i) yi = t;
+    if (lane < i) g -= H[i * ld + lane] * t;
   }
-  if (k > 0) y[0] += beta;
+  if (lane < k) y[lane] = yi + (lane == 0 ? beta : 0.0);
+  __syncwarp();
+}
+
+// The end of a solve, by warp 0 of every CTA: CTA 0 writes H, s_0 and y out;
+// sY holds y_j / s_j.  The caller synchronises.
+__device__ __forceinline__ void pk_finish(const PkArgs &a, double *sH, const double *sS, double *sY) {
+  if (threadIdx.x >= 32) return;
+  const int k = a.k, lane = threadIdx.x;
+  if (blockIdx.x == 0)
+    for (int q = lane; q < k * (k + 1); q += 32) a.H[q] = sH[q];
+  __syncwarp();
+  pk_lsq(k, sH, sS[0], sY);
+  if (blockIdx.x == 0) {
+    if (lane == 0) a.aux[0] = sS[0];
+    if (lane < k) a.aux[1 + lane] = sY[lane];
+  }
+  if (lane < k) sY[lane] = sS[lane] > 0.0 ? sY[lane] / sS[lane] : 0.0;
 }
 
 // Shared memory of the phases (dynamic part): the three twiddle tables and
-// the largest work tile (PLANE: a plane's row tile and its column tile).
-template <int M, int N, bool PLANE = false> __host__ __device__ constexpr size_t pk_smem() {
-  constexpr size_t xs = PLANE ? (size_t)N * (LayRow<M, PkSplit<M>::R2>::RS + pk_ncp<M>())
-                              : (size_t)pk_rx<M>() * LayRow<M, PkSplit<M>::R2>::RS;
-  constexpr size_t ys = PLANE ? 0 : (size_t)(kPkThreads / (Split<N>::R1 * 16)) * N * 16;
+// the largest work tile.
+template <int M, int N> __host__ __device__ constexpr size_t pk_smem() {
+  constexpr size_t xs = (size_t)pk_rx<M>() * LayRow<M, PkSplit<M>::R2>::RS;
+  constexpr size_t ys = (size_t)(kPkThreads / (Split<N>::R1 * 16)) * N * 16;
   constexpr size_t zs = (size_t)(kPkThreads / (PkZSplit<N>::R1 * kPkBz * 3)) * 3 * N * kPkBz;
   constexpr size_t tile = xs > ys ? (xs > zs ? xs : zs) : (ys > zs ? ys : zs);
-  return sizeof(float2) * (M + M % 2 + 2 * N + tile);
+  return sizeof(float2) * (M + 2 * N + tile);
 }
 
-// Grid barriers of one GMRES step: XF Y Z YI XI, or XY Z YXI with PLANE.
-template <bool PLANE> __host__ __device__ constexpr int pk_phases() { return PLANE ? 3 : 5; }
-
-// PLANE: every CTA owns whole (site, z) planes in the x phases, so that the
-// y transforms ride in them (XY: update, c'_H, r2c along x, forward y; YXI:
-// inverse y, c2r along x, dots) and a step has three grid barriers, not five.
-template <int M, int N, bool PLANE = false>
+template <int M, int N>
 __global__ void __launch_bounds__(kPkThreads, 2) k_coarse_gmres(PkArgs a) {
-  constexpr int RXP = PLANE ? N : pk_rx<M>();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float2 *twx = reinterpret_cast<float2 *>(smem_raw);
   float2 *twy = twx + M;
   float2 *twz = twy + N;
-  float2 *tile = twz + N + M % 2;  // on a 16-byte boundary
+  float2 *tile = twz + N;
   __shared__ double sH[kPkMaxSteps * (kPkMaxSteps + 1)];
   __shared__ double sS[kPkMaxSteps + 1];  // s_j = |V_j|
   __shared__ double sD[kVecMax];          // summed dot partials
@@ -584,7 +572,7 @@ __global__ void __launch_bounds__(kPkThreads, 2) k_coarse_gmres(PkArgs a) {
       }
       __syncthreads();
     }
-    pk_xf<M, RXP, PLANE, N>(a, sV, j, j, sC, j < k, tile, twx, twy, nrm2);
+    pk_xf<M>(a, sV, j, j, sC, j < k, tile, twx, nrm2);
     if (j > 0) pk_block_sum(nrm2, a.pnrm + (j & 1) * gridDim.x);
     if (!grid_sync(a.bar, ++gen, a.err, a.trace, a.trace_cta)) return;
     if (j > 0) {
@@ -596,23 +584,19 @@ __global__ void __launch_bounds__(kPkThreads, 2) k_coarse_gmres(PkArgs a) {
       __syncthreads();
     }
     if (j == k) break;
-    if constexpr (!PLANE) {
-      pk_y<N, false>(a, tile, twy);
-      if (!grid_sync(a.bar, ++gen, a.err, a.trace, a.trace_cta)) return;
-    }
+    pk_y<N, false>(a, tile, twy);
+    if (!grid_sync(a.bar, ++gen, a.err, a.trace, a.trace_cta)) return;
     pk_z<N>(a, tile, twz);
     if (!grid_sync(a.bar, ++gen, a.err, a.trace, a.trace_cta)) return;
-    if constexpr (!PLANE) {
-      pk_y<N, true>(a, tile, twy);
-      if (!grid_sync(a.bar, ++gen, a.err, a.trace, a.trace_cta)) return;
-    }
+    pk_y<N, true>(a, tile, twy);
+    if (!grid_sync(a.bar, ++gen, a.err, a.trace, a.trace_cta)) return;
     // V_{j+1} = J (V_j / s_j) = (X / N - V_j) / s_j
     const double sj = sS[j];
     const float inv = sj > 0.0 ? (float)(1.0 / sj) : 0.f;
     __shared__ double sdot[kPkMaxSteps][kPkThreads / 32];
     for (int q = tid; q < kPkMaxSteps * (kPkThreads / 32); q += kPkThreads) (&sdot[0][0])[q] = 0.0;
     __syncthreads();
-    pk_xi<M, RXP, PLANE, N>(a, sV, j, scale * inv, inv, tile, twx, twy, sdot);
+    pk_xi<M>(a, sV, j, scale * inv, inv, tile, twx, sdot);
     if (tid <= j) {
       double t = 0.0;
       for (int w = 0; w < kPkThreads / 32; ++w) t += sdot[tid][w];
@@ -622,17 +606,7 @@ __global__ void __launch_bounds__(kPkThreads, 2) k_coarse_gmres(PkArgs a) {
   }
 
   // least squares (every CTA, bitwise alike), then out = sum_j y_j V_j / s_j
-  if (tid == 0) {
-    __shared__ double sG[kPkMaxSteps + 1], sCs[kPkMaxSteps], sSn[kPkMaxSteps];
-    if (blockIdx.x == 0)
-      for (int q = 0; q < k * (k + 1); ++q) a.H[q] = sH[q];
-    pk_lsq(k, sH, sS[0], sY, sG, sCs, sSn);
-    if (blockIdx.x == 0) {
-      a.aux[0] = sS[0];
-      for (int i = 0; i < k; ++i) a.aux[1 + i] = sY[i];
-    }
-    for (int i = 0; i < k; ++i) sY[i] = sS[i] > 0.0 ? sY[i] / sS[i] : 0.0;
-  }
+  pk_finish(a, sH, sS, sY);
   __syncthreads();
   const long long nw = a.g.Nr * a.g.m / 4;
   for (long long i = (long long)blockIdx.x * kPkThreads + tid; i < nw; i += (long long)gridDim.x * kPkThreads) {

@@ -197,6 +197,35 @@ __device__ __forceinline__ void fft2(V *buf, const V *tw) {
   fft2g<N, NCOL, NTHR, INV, COLFAST, Lay, S>(buf, tw, (int)threadIdx.x, true);
 }
 
+// The two halves of a transform without the reordering between them: with
+// N = R1 R2, X[k1 + R1 k2] stands at index R2 k1 + k2 (perm_pos), where the
+// second step of the forward transform and the first of the inverse one work
+// in place, so neither holds its outputs across a barrier.
+template <class S> __host__ __device__ constexpr int perm_pos(int k) { return S::R2 * (k % S::R1) + k / S::R1; }
+template <class S> __host__ __device__ constexpr int perm_freq(int p) { return p / S::R2 + S::R1 * (p % S::R2); }
+
+// One R1-point DFT of the first forward step (last inverse step) and one
+// R2-point DFT of the second (first), in registers: column element `n2` and
+// block `k1` of a length-N transform, twiddles included.
+template <class S, typename V> __device__ __forceinline__ void fwd_step1(V *u, int n2, const V *tw) {
+  constexpr int R1 = S::R1, N = S::R1 * S::R2;
+  RDft<R1, false, V>::run(u, tw, N / R1);
+#pragma unroll
+  for (int k1 = 1; k1 < R1; ++k1) u[k1] = cmul(u[k1], tw[n2 * k1]);
+}
+template <class S, typename V> __device__ __forceinline__ void fwd_step2(V *u, const V *tw) {
+  RDft<S::R2, false, V>::run(u, tw, S::R1);
+}
+template <class S, typename V> __device__ __forceinline__ void inv_step1(V *u, int k1, const V *tw) {
+  constexpr int R2 = S::R2;
+  RDft<R2, true, V>::run(u, tw, S::R1);
+#pragma unroll
+  for (int n2 = 1; n2 < R2; ++n2) u[n2] = cmul(u[n2], cconj(tw[n2 * k1]));
+}
+template <class S, typename V> __device__ __forceinline__ void inv_step2(V *u, const V *tw) {
+  RDft<S::R1, true, V>::run(u, tw, S::R2);
+}
+
 // ------------------------------------------------------------- TMA + mbarrier
 // d_err code of a timed-out wait in the tensor-core grid transfers
 // (the passes record their pass number, the coarse solve kPkErr).

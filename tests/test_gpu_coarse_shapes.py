@@ -1,5 +1,6 @@
-"""The persistent coarse GMRES at the coarse grids of small boxes and odd half
-rows (32^3, 36^3, 54^3) and beside them (48^3): equal to the graph-replayed
+"""The persistent coarse GMRES at every coarse grid of its plane form (32^3 to
+96^3: whole basis, part of it and none of it resident in shared memory; odd
+half rows at 54^3): equal to the graph-replayed
 step-by-step kernels, and bitwise repeatable.
 
 Both run 16 FP32 GMRES steps on the same operator with different roundings;
@@ -15,7 +16,8 @@ from bgy3d_b200 import RismContext  # noqa: E402
 
 
 @pytest.mark.parametrize("sites", [1, 3])
-@pytest.mark.parametrize("n, L, nc", [(64, 12.0, 32), (72, 13.0, 36), (96, 18.0, 48), (108, 20.0, 54)])
+@pytest.mark.parametrize("n, L, nc", [(64, 12.0, 32), (72, 13.0, 36), (96, 18.0, 48), (108, 20.0, 54), (128, 24.0, 64), (144, 27.0, 72),
+                                      (192, 36.0, 96)])
 def test_persistent_shapes_match_graph(fixture_loader, n, L, nc, sites, monkeypatch):
     meta, arr = fixture_loader("synth6_kh_n32")
     s = dict(meta["settings"])
