@@ -13,10 +13,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "librism3d.so")
-SOURCES = ["rism3d.cu", "twogrid_fx2.cu", "twogrid_yz.cu", "twogrid_tc.cu", "coarse_pk.cu", "rism1d.cpp", "noalloc.cu",
+SOURCES = ["rism3d.cu", "twogrid_fx2a.cu", "twogrid_fx2b.cu", "twogrid_fx2c.cu", "twogrid_yz.cu", "twogrid_tc.cu", "coarse_pk.cu", "rism1d.cpp", "noalloc.cu",
            "passes_x1.cu", "passes_x2.cu", "passes_y.cu", "passes_z1.cu", "passes_z2.cu", "passes_z3.cu"]
 HEADERS = ["fft_core.cuh", "kernels.cuh", "fft_static.cuh", "kernels_static.cuh", "krylov.cuh", "twogrid.cuh",
-           "twogrid_fft.cuh", "grad.cuh", "solvent.cuh", "info.cuh", "coarse_pk.cuh", "coarse_planes.cuh", "passes.cuh", "passes_impl.cuh"]
+           "twogrid_fft.cuh", "twogrid_fx2.cuh", "twogrid_fx2_impl.cuh", "grad.cuh", "solvent.cuh", "info.cuh", "coarse_pk.cuh", "coarse_planes.cuh", "passes.cuh", "passes_impl.cuh"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 

@@ -82,13 +82,22 @@ template <int N> struct Split {
   static constexpr int R2 = N / R1;
 };
 
+// The split of the y columns (R1 B threads, one second-step DFT each): Split
+// where it has a balanced one, factors of 6, 9, 12, 18 and 27 elsewhere.
+template <int N> struct SplitY {
+  static constexpr int R1 = N == 32 ? 8 : N == 36 ? 6 : N == 54 ? 9 : N == 108 ? 12 : N == 162 ? 18 : N == 216 ? 18
+                            : N == 288 ? 18 : N == 324 ? 18 : N == 384 ? 24 : N == 432 ? 24 : N == 486 ? 27
+                            : Split<N>::R1;
+  static constexpr int R2 = N / R1;
+};
+
 // A split with R1 near sqrt(N) (64 = 8 x 8, 96 = 12 x 8): where a tile has
 // few columns, Split's larger first radix leaves most threads of a step idle
 // (16 x 4 over 16 columns: 64 DFTs for 256 threads) and holds twice the
 // values per thread.
 template <int N> struct SplitSq {
   static constexpr int R1 = N == 32 ? 8 : N == 36 ? 6 : N == 48 ? 8 : N == 54 ? 9 : N == 64 ? 8 : N == 72 ? 8 : N == 96 ? 12
-                            : N == 128 ? 16 : Split<N>::R1;
+                            : N == 128 ? 16 : SplitY<N>::R1;
   static constexpr int R2 = N / R1;
 };
 
@@ -100,15 +109,6 @@ template <int N> struct SplitRow {
   static constexpr int R1 = N == 16 ? 4 : N == 18 ? 6 : N == 24 ? 6 : N == 27 ? 9 : N == 32 ? 8 : N == 36 ? 6
                             : N == 48 ? 8 : N == 54 ? 9 : N == 81 ? 9 : N == 96 ? 12 : N == 108 ? 12 : N == 144 ? 12
                             : N == 162 ? 18 : N == 216 ? 18 : N == 243 ? 27 : Split<N>::R1;
-  static constexpr int R2 = N / R1;
-};
-
-// The split of the y columns (R1 B threads, one second-step DFT each): Split
-// where it has a balanced one, factors of 6, 9, 12, 18 and 27 elsewhere.
-template <int N> struct SplitY {
-  static constexpr int R1 = N == 32 ? 8 : N == 36 ? 6 : N == 54 ? 9 : N == 108 ? 12 : N == 162 ? 18 : N == 216 ? 18
-                            : N == 288 ? 18 : N == 324 ? 18 : N == 384 ? 24 : N == 432 ? 24 : N == 486 ? 27
-                            : Split<N>::R1;
   static constexpr int R2 = N / R1;
 };
 

@@ -37,11 +37,11 @@
 #include "solvent.cuh"
 #include "twogrid.cuh"
 #include "twogrid_fft.cuh"
+#include "twogrid_fx2.cuh"
 
 using namespace rism;
 
-namespace rism {  // twogrid_fx2.cu: x transfers with both sides by FFT
-bool fx2_has_pair(int M, int MC);
+namespace rism {
 // twogrid_yz.cu: y / z transfers by FFT
 bool yz_fft_transfer(int outer, int n_in, int n_out, int inner, const float *in, const float2 *twi,
                      const float2 *two, float *out, cudaStream_t st);
@@ -49,12 +49,6 @@ bool yz_fft_transfer(int outer, int n_in, int n_out, int inner, const float *in,
 int coarse_pk_grid(int M, int N, int per_sm);
 int coarse_pk_phases(int M, int N);
 cudaError_t coarse_pk_launch(const PkArgs &a, int M, int N, int grid, cudaStream_t st);
-template <typename T>
-bool fx2_restrict(int M, int MC, long long rows, const T *in, float s, const float2 *post, const float2 *tw,
-                  const float2 *postc, const float2 *twc, float *out, cudaStream_t st);
-template <typename T>
-bool fx2_prolong(int M, int MC, long long rows, const float *y, const float2 *post, const float2 *tw,
-                 const float2 *postc, const float2 *twc, const T *r, double s, T *out, cudaStream_t st);
 // twogrid_tc.cu: the x transfers of FP32 data on the tensor cores
 bool tc_x_has(int n0, int nc);
 bool tc_restrict_x(long long rows, int n0, int nc, const float *in, float s, const float *R, float *out, int *err,
@@ -980,14 +974,36 @@ bool fx_usable(const rism3d_ctx *c) {
 bool fx2_usable(const rism3d_ctx *c) {
   const char *dense = std::getenv("RISM3D_DENSE_TRANSFERS");
   if (dense && dense[0] == '2') return false;
-  return c->coarse && c->coarse->g.M == c->Nc[0] / 2 && rism::fx2_has_pair(c->g.M, c->Nc[0] / 2);
+  return c->coarse && c->coarse->g.M == c->Nc[0] / 2;
+}
+template <typename T>
+bool fx2_restrict(int M, int MC, long long rows, const T *in, float s, const float2 *post, const float2 *tw,
+                  const float2 *postc, const float2 *twc, float *out, cudaStream_t st) {
+  switch (M) {
+#define FX2_M(L) \
+  case L: return Fx2<L>::template restrict_x<T>(MC, rows, in, s, post, tw, postc, twc, out, st);
+    RISM_FX2_LENS(FX2_M)
+#undef FX2_M
+    default: return false;
+  }
+}
+template <typename T>
+bool fx2_prolong(int M, int MC, long long rows, const float *y, const float2 *post, const float2 *tw,
+                 const float2 *postc, const float2 *twc, const T *r, double s, T *out, cudaStream_t st) {
+  switch (M) {
+#define FX2_M(L) \
+  case L: return Fx2<L>::template prolong_x<T>(MC, rows, y, post, tw, postc, twc, r, s, out, st);
+    RISM_FX2_LENS(FX2_M)
+#undef FX2_M
+    default: return false;
+  }
 }
 template <typename T> bool fx_restrict(rism3d_ctx *c, long long rows, const T *in, double s) {
   if (!fx_usable(c)) return false;
   const int K = c->Nc[0] / 2;
   const auto *post = postw<float>(c);
   const auto *tw = static_cast<const float2 *>(c->plan<float>(0).tw);
-  if (fx2_usable(c) && rism::fx2_restrict<T>(c->g.M, c->Nc[0] / 2, rows, in, (float)s, post, tw, c->coarse->post32,
+  if (fx2_usable(c) && fx2_restrict<T>(c->g.M, c->Nc[0] / 2, rows, in, (float)s, post, tw, c->coarse->post32,
                                               c->coarse->tw32[0], c->tA, c->stream)) {
     CKL();
     return true;
@@ -1015,7 +1031,7 @@ template <typename T> bool fx_prolong(rism3d_ctx *c, long long rows, const T *r,
   const int K = c->Nc[0] / 2;
   const auto *post = postw<float>(c);
   const auto *tw = static_cast<const float2 *>(c->plan<float>(0).tw);
-  if (fx2_usable(c) && rism::fx2_prolong<T>(c->g.M, c->Nc[0] / 2, rows, c->tA, post, tw, c->coarse->post32,
+  if (fx2_usable(c) && fx2_prolong<T>(c->g.M, c->Nc[0] / 2, rows, c->tA, post, tw, c->coarse->post32,
                                              c->coarse->tw32[0], r, s, out, c->stream)) {
     CKL();
     return true;

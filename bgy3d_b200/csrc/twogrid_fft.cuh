@@ -341,8 +341,11 @@ __global__ void __launch_bounds__(256, M == 128 ? 3 : 1) k_restrict_fx2(long lon
   using Q = typename Quad<TI>::type;
   static_assert(MC < M && fx_buf<MC, RX>() <= fx_buf<M, RX>(), "coarse row tile must fit the fine one");
   constexpr int N0 = 2 * M, Nc = 2 * MC, K = MC, K1 = MC + 1;
-  constexpr int PER = M / 2, CNT = (RX * PER + 255) / 256;
-  constexpr int PC = MC / 2;  // output float4 per row
+  // a batch of rows is one run of memory: RX M / 2 pairs of complex values,
+  // whose rows may end inside a pair (odd M), and RX MC / 2 output float4
+  static_assert(RX % 2 == 0, "a batch holds whole pairs");
+  constexpr int NQ = RX * M / 2, CNT = (NQ + 255) / 256;
+  constexpr int NC = RX * MC / 2;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   V *tw = reinterpret_cast<V *>(smem_raw);
   V *buf = tw + M;
@@ -358,8 +361,7 @@ __global__ void __launch_bounds__(256, M == 128 ? 3 : 1) k_restrict_fx2(long lon
     const long long r0 = (BAT) * RX;                                                                \
     _Pragma("unroll") for (int it = 0; it < CNT; ++it) {                                            \
       const int e = tid + it * 256;                                                                 \
-      const int row = e / PER, jj = (e % PER) * 2;                                                  \
-      if (e < RX * PER && r0 + row < rows) ra[it] = *reinterpret_cast<const Q *>(in + (r0 + row) * N0 + 2 * jj); \
+      if (e < NQ && e < (rows - r0) * M / 2) ra[it] = *reinterpret_cast<const Q *>(in + r0 * N0 + 4 * e); \
     }                                                                                               \
   }
   if (bat < nbat) FX2_LOAD_ROWS(bat)
@@ -370,15 +372,14 @@ __global__ void __launch_bounds__(256, M == 128 ? 3 : 1) k_restrict_fx2(long lon
 #pragma unroll
     for (int it = 0; it < CNT; ++it) {
       const int e = tid + it * 256;
-      if (e >= RX * PER) break;
-      const int row = e / PER, jj = (e % PER) * 2;
+      if (e >= NQ) break;
       V a = make_float2(0.f, 0.f), b = a;
-      if (row0 + row < rows) {
+      if (e < (rows - row0) * M / 2) {
         Quad<TI>::split(ra[it], a, b);
         a.x *= s; a.y *= s; b.x *= s; b.y *= s;
       }
-      buf[Lay::at(jj, row)] = a;
-      buf[Lay::at(jj + 1, row)] = b;
+      buf[Lay::at((2 * e) % M, (2 * e) / M)] = a;
+      buf[Lay::at((2 * e + 1) % M, (2 * e + 1) / M)] = b;
     }
     if (bat + gridDim.x < nbat) FX2_LOAD_ROWS(bat + gridDim.x)
     __syncthreads();
@@ -398,11 +399,10 @@ __global__ void __launch_bounds__(256, M == 128 ? 3 : 1) k_restrict_fx2(long lon
     fx_pack_c2r<MC, RX, LayC>(X, K, K1, postc, buf);
     __syncthreads();
     fft2<MC, RX, 256, true, false, LayC, SplitRow<MC>>(buf, twc);
-    for (int e = tid; e < RX * PC; e += 256) {
-      const int row = e / PC, jj = (e - row * PC) * 2;
-      if (row0 + row >= rows) continue;
-      const V za = buf[LayC::at(jj, row)], zb = buf[LayC::at(jj + 1, row)];
-      *reinterpret_cast<float4 *>(out + (row0 + row) * Nc + 2 * jj) =
+    for (int e = tid; e < NC; e += 256) {
+      if (e >= (rows - row0) * MC / 2) break;
+      const V za = buf[LayC::at((2 * e) % MC, (2 * e) / MC)], zb = buf[LayC::at((2 * e + 1) % MC, (2 * e + 1) / MC)];
+      *reinterpret_cast<float4 *>(out + row0 * Nc + 4 * e) =
           make_float4(za.x * inv_n0, za.y * inv_n0, zb.x * inv_n0, zb.y * inv_n0);
     }
     __syncthreads();
@@ -425,7 +425,8 @@ __global__ void __launch_bounds__(256, M == 128 ? (RX >= 32 ? 2 : 3) : 1) k_prol
   using QR = typename Quad<TR>::type;
   static_assert(MC < M && fx_buf<MC, RX>() <= fx_buf<M, RX>(), "coarse row tile must fit the fine one");
   constexpr int N0 = 2 * M, Nc = 2 * MC, K = MC, K1 = MC + 1;
-  constexpr int PER = M / 2, CNT = (RX * PER + 255) / 256;
+  static_assert(RX % 2 == 0, "a batch holds whole pairs");
+  constexpr int NQ = RX * M / 2, CNT = (NQ + 255) / 256;  // pairs of complex values of a batch, as above
   constexpr int YC = (RX * MC + 255) / 256;  // coarse pairs per thread
   extern __shared__ __align__(128) unsigned char smem_raw[];
   V *tw = reinterpret_cast<V *>(smem_raw);
@@ -443,8 +444,7 @@ __global__ void __launch_bounds__(256, M == 128 ? (RX >= 32 ? 2 : 3) : 1) k_prol
     const long long r0 = (BAT) * RX;                                                                \
     _Pragma("unroll") for (int it = 0; it < CNT; ++it) {                                            \
       const int e = tid + it * 256;                                                                 \
-      const int row = e / PER, jj = (e % PER) * 2;                                                  \
-      if (e < RX * PER && r0 + row < rows) RR[it] = *reinterpret_cast<const QR *>(r + (r0 + row) * N0 + 2 * jj); \
+      if (e < NQ && e < (rows - r0) * M / 2) RR[it] = *reinterpret_cast<const QR *>(r + r0 * N0 + 4 * e); \
     }                                                                                               \
     _Pragma("unroll") for (int q = 0; q < YC; ++q) {                                                \
       const int e = tid + q * 256;                                                                  \
@@ -493,14 +493,12 @@ __global__ void __launch_bounds__(256, M == 128 ? (RX >= 32 ? 2 : 3) : 1) k_prol
 #pragma unroll
     for (int it = 0; it < CNT; ++it) {
       const int e = tid + it * 256;
-      if (e >= RX * PER) break;
-      const int row = e / PER, jj = (e % PER) * 2;
-      if (row0 + row >= rows) continue;
+      if (e >= NQ || e >= (rows - row0) * M / 2) break;
       V ra, rb;
       Quad<TR>::split(rr[it], ra, rb);
-      const V za = buf[Lay::at(jj, row)], zb = buf[Lay::at(jj + 1, row)];
-      TO *o = out + (row0 + row) * N0 + 2 * jj;  // 4 consecutive outputs, 4-element aligned
-      const TR *rx = r + (row0 + row) * N0 + 2 * jj;
+      const V za = buf[Lay::at((2 * e) % M, (2 * e) / M)], zb = buf[Lay::at((2 * e + 1) % M, (2 * e + 1) / M)];
+      TO *o = out + row0 * N0 + 4 * e;  // 4 consecutive outputs, 4-element aligned
+      const TR *rx = r + row0 * N0 + 4 * e;
       if constexpr (sizeof(TR) == 8) {
         // the subtracted term in the output precision (r kept exact for FP64)
         const double2 r01 = *reinterpret_cast<const double2 *>(rx), r23 = *reinterpret_cast<const double2 *>(rx + 2);
