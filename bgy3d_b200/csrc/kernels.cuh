@@ -30,8 +30,10 @@ constexpr double kEps0Inv = 331.84164;  // EPSILON0INV, bgy3d.h:145
 constexpr double kG = 1.2;              // G_COULOMB_INVERSE_RANGE, bgy3d-solvents.h:9
 
 // MODE_FWD: plain forward 3D transform of A (x and z passes; the z pass
-// stops after its forward transform), used by the gradient.
-enum { MODE_F = 0, MODE_J = 1, MODE_FWD = 2 };
+// stops after its forward transform), used by the gradient.  MODE_S: the x
+// forward pass of a single Jacobian product, which takes the closure slope
+// from t and v itself instead of from a slope field made beforehand.
+enum { MODE_F = 0, MODE_J = 1, MODE_FWD = 2, MODE_S = 3 };
 enum { CL_HNC = 0, CL_KH = 1, CL_PY = 2, CL_PSE0 = 3 };
 
 struct Geo {

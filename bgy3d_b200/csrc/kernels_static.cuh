@@ -28,17 +28,35 @@ template <int M> struct VecW<float, M> {
   using vec = std::conditional_t<M % 2 == 0, float4, float2>;
 };
 
-// Rows per CTA of the x passes.
-__host__ __device__ constexpr int x_rows(int) { return 16; }
+// The x passes take RX rows with 128 threads (256 in the FP32 forward pass, whose
+// exponentials want the warps): about 8 KB of a field per CTA, so that a thread
+// has all its loads in flight and several small CTAs share an SM.  Sixteen rows
+// of 512 points in FP64 took 256 registers of loads, and long FP32 rows fell
+// back to a loop of two loads in flight.  Inverse pass, us, with 256 threads and
+// whole transforms through shared memory -> here: 128^3 FP32 21.7 -> 20.7, FP64
+// 46 -> 34; 256^3 133 -> 110, 288 -> 241; 512^3 1413 -> 888, 3985 -> 2352.
+constexpr int kXThreads = 128;
+template <typename T> __host__ __device__ constexpr int xfwd_threads() { return sizeof(T) == 4 ? 256 : 128; }
+__host__ __device__ constexpr int x_rows(bool f64, int M) {
+  return f64 ? (M <= 64 ? 16 : M <= 162 ? 8 : 4) : (M <= 128 ? 16 : 8);
+}
+template <typename T, int M> __host__ __device__ constexpr int x_rx() { return x_rows(sizeof(T) == 8, M); }
 
-// x forward (see k_xfwd): MODE_F c = closure(p B, A); MODE_J c = B (p A).
+// x forward (see k_xfwd): MODE_F c = closure(p B, A); MODE_J c = B (p A);
+// MODE_S c = closure'(p B, Tv) A.  In FP64 the spectrum stays in the order of
+// the two transform steps (perm_pos) and the untangling indexes it there (J at
+// 256^3 207 -> 197 us); in FP32 the natural order is the faster one (125 -> 116).
 template <typename T, int MODE, int M, int RX>
-__global__ void __launch_bounds__(256) k_xfwd_s(Geo g, const T *__restrict__ A, const T *__restrict__ Bv, T p,
-                                               int closure, typename Cx<T>::type *__restrict__ W,
-                                               const typename Cx<T>::type *__restrict__ post,
-                                               const typename Cx<T>::type *__restrict__ twg) {
+__global__ void __launch_bounds__(xfwd_threads<T>()) k_xfwd_s(Geo g, const T *__restrict__ A, const T *__restrict__ Bv,
+                                                     const T *__restrict__ Tv, T p, int closure,
+                                                     typename Cx<T>::type *__restrict__ W,
+                                                     const typename Cx<T>::type *__restrict__ post,
+                                                     const typename Cx<T>::type *__restrict__ twg) {
   using V = typename Cx<T>::type;
-  using Lay = LayRow<M, SplitRow<M>::R2>;
+  using S = SplitRow<M>;
+  using Lay = LayRow<M, S::R2>;
+  constexpr int THR = xfwd_threads<T>();
+  constexpr bool PERM = sizeof(T) == 8;
   constexpr int VW = VecW<T, M>::n;
   using VEC = typename VecW<T, M>::vec;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -48,25 +66,26 @@ __global__ void __launch_bounds__(256) k_xfwd_s(Geo g, const T *__restrict__ A, 
   const int rows_total = g.N1 * g.N2;
   const int row0 = blockIdx.x * RX;
   const int site = blockIdx.y;
-  for (int q = tid; q < M; q += 256) tw[q] = twg[q];
+  for (int q = tid; q < M; q += THR) tw[q] = twg[q];
   const long long sbase = (long long)site * g.Nr;
   constexpr int PER_ROW = M / VW;
-  constexpr int CNT = (RX * PER_ROW + 255) / 256;
+  constexpr int CNT = (RX * PER_ROW + THR - 1) / THR;
   // all loads of the thread in flight before any use
-  VEC ra[CNT], rb[CNT];
+  VEC ra[CNT], rb[CNT], rt[MODE == MODE_S ? CNT : 1];
 #pragma unroll
   for (int it = 0; it < CNT; ++it) {
-    const int e = tid + it * 256;
+    const int e = tid + it * THR;
     const int row = e / PER_ROW, jj = (e % PER_ROW) * VW;
     if (e < RX * PER_ROW && row0 + row < rows_total) {
       const long long off = sbase + (long long)(row0 + row) * g.N0 + 2 * jj;
       ra[it] = *reinterpret_cast<const VEC *>(A + off);
       rb[it] = *reinterpret_cast<const VEC *>(Bv + off);
+      if (MODE == MODE_S) rt[it] = *reinterpret_cast<const VEC *>(Tv + off);
     }
   }
 #pragma unroll
   for (int it = 0; it < CNT; ++it) {
-    const int e = tid + it * 256;
+    const int e = tid + it * THR;
     if (e >= RX * PER_ROW) break;
     const int row = e / PER_ROW, jj = (e % PER_ROW) * VW;
     const int grow = row0 + row;
@@ -76,11 +95,15 @@ __global__ void __launch_bounds__(256) k_xfwd_s(Geo g, const T *__restrict__ A, 
     if (grow < rows_total) {
       const T *ar = reinterpret_cast<const T *>(&ra[it]);
       const T *br = reinterpret_cast<const T *>(&rb[it]);
+      const T *tr = reinterpret_cast<const T *>(&rt[MODE == MODE_S ? it : 0]);
 #pragma unroll
       for (int v = 0; v < VW; ++v) {
         if (MODE == MODE_F) {
           z[v].x = closure_c<T>(closure, p * br[2 * v], ar[2 * v]);
           z[v].y = closure_c<T>(closure, p * br[2 * v + 1], ar[2 * v + 1]);
+        } else if (MODE == MODE_S) {
+          z[v].x = closure_d<T>(closure, p * br[2 * v], tr[2 * v]) * ar[2 * v];
+          z[v].y = closure_d<T>(closure, p * br[2 * v + 1], tr[2 * v + 1]) * ar[2 * v + 1];
         } else {
           z[v].x = br[2 * v] * (ar[2 * v] * p);
           z[v].y = br[2 * v + 1] * (ar[2 * v + 1] * p);
@@ -91,15 +114,41 @@ __global__ void __launch_bounds__(256) k_xfwd_s(Geo g, const T *__restrict__ A, 
     for (int v = 0; v < VW; ++v) buf[Lay::at(jj + v, row)] = z[v];
   }
   __syncthreads();
-  fft2<M, RX, 256, false, false, Lay, SplitRow<M>>(buf, tw);
+  if constexpr (PERM) {
+#pragma unroll
+    for (int q = tid; q < RX * S::R2; q += THR) {
+      const int row = q / S::R2, n2 = q % S::R2;
+      V u[S::R1];
+#pragma unroll
+      for (int n1 = 0; n1 < S::R1; ++n1) u[n1] = buf[Lay::at(S::R2 * n1 + n2, row)];
+      fwd_step1<S>(u, n2, tw);
+#pragma unroll
+      for (int k1 = 0; k1 < S::R1; ++k1) buf[Lay::at(S::R2 * k1 + n2, row)] = u[k1];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = tid; q < RX * S::R1; q += THR) {
+      const int row = q / S::R1, k1 = q % S::R1;
+      V u[S::R2];
+#pragma unroll
+      for (int n2 = 0; n2 < S::R2; ++n2) u[n2] = buf[Lay::at(S::R2 * k1 + n2, row)];
+      fwd_step2<S>(u, tw);
+#pragma unroll
+      for (int k2 = 0; k2 < S::R2; ++k2) buf[Lay::at(S::R2 * k1 + k2, row)] = u[k2];
+    }
+    __syncthreads();
+  } else {
+    fft2<M, RX, THR, false, false, Lay, S>(buf, tw);
+  }
   constexpr int H = M / 2 + 1;
   const long long wbase = (long long)site * g.Nc;
-  for (int e = tid; e < RX * H; e += 256) {
+  for (int e = tid; e < RX * H; e += THR) {
     const int row = e / H, k = e % H;
     const int grow = row0 + row;
     if (grow >= rows_total) continue;
-    const V zk = buf[Lay::at(k, row)];
-    const V zm = buf[Lay::at(k == 0 ? 0 : M - k, row)];
+    const int km = k == 0 ? 0 : M - k;
+    const V zk = buf[Lay::at(PERM ? perm_pos<S>(k) : k, row)];
+    const V zm = buf[Lay::at(PERM ? perm_pos<S>(km) : km, row)];
     V E, O;
     E.x = (zk.x + zm.x) * T(0.5);
     E.y = (zk.y - zm.y) * T(0.5);
@@ -112,17 +161,24 @@ __global__ void __launch_bounds__(256) k_xfwd_s(Geo g, const T *__restrict__ A, 
   }
 }
 
-// x inverse (see k_xinv): out = scale x - sub In, residual norms.
+// x inverse (see k_xinv): out = scale x - sub In, and, where part is given,
+// the residual norms.  The packed input is written in the order that the first
+// inverse step works on.  The last step's outputs leave from its registers
+// where its lanes cover whole 32-byte sectors (R2 complex values in a row),
+// else through shared memory as 16-byte vectors.
 template <typename T, int M, int RX>
-__global__ void __launch_bounds__(256) k_xinv_s(Geo g, const typename Cx<T>::type *__restrict__ W,
-                                               const T *__restrict__ In, T *__restrict__ Out, T scale, T sub,
-                                               const typename Cx<T>::type *__restrict__ post,
-                                               const typename Cx<T>::type *__restrict__ twg,
-                                               NormPartial *__restrict__ part) {
+__global__ void __launch_bounds__(kXThreads) k_xinv_s(Geo g, const typename Cx<T>::type *__restrict__ W,
+                                                     const T *__restrict__ In, T *__restrict__ Out, T scale, T sub,
+                                                     const typename Cx<T>::type *__restrict__ post,
+                                                     const typename Cx<T>::type *__restrict__ twg,
+                                                     NormPartial *__restrict__ part) {
   using V = typename Cx<T>::type;
-  using Lay = LayRow<M, SplitRow<M>::R2>;
-  constexpr int VW = VecW<T, M>::n;
-  using VEC = typename VecW<T, M>::vec;
+  using S = SplitRow<M>;
+  using Lay = LayRow<M, S::R2>;
+  constexpr int THR = kXThreads;
+  constexpr bool direct = S::R2 * sizeof(V) % 32 == 0;
+  constexpr int VW = direct ? 1 : VecW<T, M>::n;
+  using VEC = std::conditional_t<direct, V, typename VecW<T, M>::vec>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   V *tw = reinterpret_cast<V *>(smem_raw);
   V *buf = tw + M;
@@ -130,117 +186,127 @@ __global__ void __launch_bounds__(256) k_xinv_s(Geo g, const typename Cx<T>::typ
   const int rows_total = g.N1 * g.N2;
   const int row0 = blockIdx.x * RX;
   const int site = blockIdx.y;
-  for (int q = tid; q < M; q += 256) tw[q] = twg[q];
+  for (int q = tid; q < M; q += THR) tw[q] = twg[q];
   constexpr int H = M / 2 + 1;
   const long long wbase = (long long)site * g.Nc;
   const long long sbase = (long long)site * g.Nr;
   constexpr int PER_ROW = M / VW;
-  constexpr int CNT = (RX * PER_ROW + 255) / 256;
-  // the subtracted input is fetched first; its latency hides behind the
-  // transform
+  constexpr int ITEMS = (RX * S::R2 + THR - 1) / THR;  // last-step DFTs per thread
+  constexpr int CNT = direct ? ITEMS * S::R1 : (RX * PER_ROW + THR - 1) / THR;
+  // element `it` of this thread: (row, complex index), or row < 0
+  auto where = [&](int it, int &row, int &jj) {
+    if (direct) {
+      const int q = tid + (it / S::R1) * THR;
+      row = q < RX * S::R2 ? q / S::R2 : -1;
+      jj = S::R2 * (it % S::R1) + q % S::R2;
+    } else {
+      const int e = tid + it * THR;
+      row = e < RX * PER_ROW ? e / PER_ROW : -1;
+      jj = (e % PER_ROW) * VW;
+    }
+    if (row0 + row >= rows_total) row = -1;
+  };
+  constexpr int CW = (RX * H + THR - 1) / THR;
+  // every (X_k, X_{M-k}) pair of this thread and the subtracted input are
+  // loaded before the first is used
+  V xkv[CW], xmv[CW];
+#pragma unroll
+  for (int it = 0; it < CW; ++it) {
+    const int e = tid + it * THR;
+    const int row = e / H, k = e % H;
+    xkv[it].x = xkv[it].y = xmv[it].x = xmv[it].y = T(0);
+    if (e < RX * H && row0 + row < rows_total) {
+      const V *row_in = W + wbase + (long long)(row0 + row) * g.Nhp;
+      xkv[it] = row_in[k];
+      xmv[it] = row_in[M - k];
+    }
+  }
   VEC rin[CNT];
 #pragma unroll
   for (int it = 0; it < CNT; ++it) {
-    const int e = tid + it * 256;
-    const int row = e / PER_ROW, jj = (e % PER_ROW) * VW;
-    if (e < RX * PER_ROW && row0 + row < rows_total)
-      rin[it] = *reinterpret_cast<const VEC *>(In + sbase + (long long)(row0 + row) * g.N0 + 2 * jj);
+    int row, jj;
+    where(it, row, jj);
+    if (row >= 0) rin[it] = *reinterpret_cast<const VEC *>(In + sbase + (long long)(row0 + row) * g.N0 + 2 * jj);
   }
-  // packed c2r input of element e = (row, k <= M/2) from X_k and X_{M-k}
-  auto pack = [&](int e, V xk, V xm) {
-    const int row = e / H, k = e % H;
-    V zk, zm;
-    zk.x = zk.y = zm.x = zm.y = T(0);
-    if (row0 + row < rows_total) {
-      if (k == 0) { xk.y = T(0); xm.y = T(0); }  // c2r reads only Re X_0, Re X_{N0/2}
-      V Aa, D;
-      Aa.x = xk.x + xm.x; Aa.y = xk.y - xm.y;
-      D.x = xk.x - xm.x;  D.y = xk.y + xm.y;
-      const V Pp = cmul(D, cconj(post[k]));
-      zk.x = Aa.x - Pp.y; zk.y = Aa.y + Pp.x;
-      zm.x = Aa.x + Pp.y; zm.y = -(Aa.y - Pp.x);
-    }
-    buf[Lay::at(k, row)] = zk;
-    if (k != 0 && M - k != k) buf[Lay::at(M - k, row)] = zm;
-  };
-  auto ld = [&](int e, V &xk, V &xm) {
-    const int row = e / H, k = e % H;
-    if (row0 + row < rows_total) {
-      const V *row_in = W + wbase + (long long)(row0 + row) * g.Nhp;
-      xk = row_in[k];
-      xm = row_in[M - k];
-    } else {
-      xk.x = xk.y = xm.x = xm.y = T(0);
-    }
-  };
-  constexpr int CW = (RX * H + 255) / 256;
-  if constexpr (CW <= 6) {
-    // every (X_k, X_{M-k}) pair of this thread is loaded before the first is
-    // used: one memory latency per CTA instead of one per pair of iterations
-    // (longer rows keep the loop below: the registers would cost occupancy)
-    V xkv[CW], xmv[CW];
 #pragma unroll
-    for (int it = 0; it < CW; ++it) {
-      const int e = tid + it * 256;
-      if (e < RX * H) ld(e, xkv[it], xmv[it]);
-    }
-#pragma unroll
-    for (int it = 0; it < CW; ++it) {
-      const int e = tid + it * 256;
-      if (e < RX * H) pack(e, xkv[it], xmv[it]);
-    }
-  } else {
-#pragma unroll 2
-    for (int e = tid; e < RX * H; e += 256) {
-      const int row = e / H, k = e % H;
-      const int grow = row0 + row;
-      V zk, zm;
-      zk.x = zk.y = zm.x = zm.y = T(0);
-      if (grow < rows_total) {
-        const V *row_in = W + wbase + (long long)grow * g.Nhp;
-        V xk = row_in[k];
-        V xm = row_in[M - k];
-        if (k == 0) { xk.y = T(0); xm.y = T(0); }
-        V Aa, D;
-        Aa.x = xk.x + xm.x; Aa.y = xk.y - xm.y;
-        D.x = xk.x - xm.x;  D.y = xk.y + xm.y;
-        const V Pp = cmul(D, cconj(post[k]));
-        zk.x = Aa.x - Pp.y; zk.y = Aa.y + Pp.x;
-        zm.x = Aa.x + Pp.y; zm.y = -(Aa.y - Pp.x);
-      }
-      buf[Lay::at(k, row)] = zk;
-      if (k != 0 && M - k != k) buf[Lay::at(M - k, row)] = zm;
-    }
+  for (int it = 0; it < CW; ++it) {
+    const int e = tid + it * THR;
+    const int row = e / H, k = e % H;
+    if (e >= RX * H) break;
+    V xk = xkv[it], xm = xmv[it];
+    if (k == 0) { xk.y = T(0); xm.y = T(0); }  // c2r reads only Re X_0, Re X_{N0/2}
+    V Aa, D, zk, zm;
+    Aa.x = xk.x + xm.x; Aa.y = xk.y - xm.y;
+    D.x = xk.x - xm.x;  D.y = xk.y + xm.y;
+    const V Pp = cmul(D, cconj(post[k]));
+    zk.x = Aa.x - Pp.y; zk.y = Aa.y + Pp.x;
+    zm.x = Aa.x + Pp.y; zm.y = -(Aa.y - Pp.x);
+    buf[Lay::at(perm_pos<S>(k), row)] = zk;
+    if (k != 0 && M - k != k) buf[Lay::at(perm_pos<S>(M - k), row)] = zm;
   }
   __syncthreads();
-  fft2<M, RX, 256, true, false, Lay, SplitRow<M>>(buf, tw);
-  double amax = 0.0, sum2 = 0.0;
 #pragma unroll
-  for (int it = 0; it < CNT; ++it) {
-    const int e = tid + it * 256;
-    if (e >= RX * PER_ROW) break;
-    const int row = e / PER_ROW, jj = (e % PER_ROW) * VW;
-    const int grow = row0 + row;
-    if (grow >= rows_total) continue;
-    const long long off = sbase + (long long)grow * g.N0 + 2 * jj;
+  for (int q = tid; q < RX * S::R1; q += THR) {
+    const int row = q / S::R1, k1 = q % S::R1;
+    V u[S::R2];
+#pragma unroll
+    for (int k2 = 0; k2 < S::R2; ++k2) u[k2] = buf[Lay::at(S::R2 * k1 + k2, row)];
+    inv_step1<S>(u, k1, tw);
+#pragma unroll
+    for (int n2 = 0; n2 < S::R2; ++n2) buf[Lay::at(S::R2 * k1 + n2, row)] = u[n2];
+  }
+  __syncthreads();
+  double amax = 0.0, sum2 = 0.0;
+  auto put = [&](int it, int row, int jj, const V *z) {
+    if (row < 0) return;
     const T *ir = reinterpret_cast<const T *>(&rin[it]);
     VEC o;
     T *orr = reinterpret_cast<T *>(&o);
 #pragma unroll
     for (int v = 0; v < VW; ++v) {
-      const V z = buf[Lay::at(jj + v, row)];
-      orr[2 * v] = z.x * scale - sub * ir[2 * v];
-      orr[2 * v + 1] = z.y * scale - sub * ir[2 * v + 1];
+      orr[2 * v] = z[v].x * scale - sub * ir[2 * v];
+      orr[2 * v + 1] = z[v].y * scale - sub * ir[2 * v + 1];
     }
-    *reinterpret_cast<VEC *>(Out + off) = o;
+    *reinterpret_cast<VEC *>(Out + sbase + (long long)(row0 + row) * g.N0 + 2 * jj) = o;
+    if (part) {
 #pragma unroll
-    for (int v = 0; v < 2 * VW; ++v) {
-      const double ov = (double)orr[v];
-      amax = fmax(amax, fabs(ov));
-      sum2 += ov * ov;
+      for (int v = 0; v < 2 * VW; ++v) {
+        const double ov = (double)orr[v];
+        amax = fmax(amax, fabs(ov));
+        sum2 += ov * ov;
+      }
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const int q = tid + i * THR;
+    if (q >= RX * S::R2) break;
+    const int row = q / S::R2, n2 = q % S::R2;
+    V u[S::R1];
+#pragma unroll
+    for (int k1 = 0; k1 < S::R1; ++k1) u[k1] = buf[Lay::at(S::R2 * k1 + n2, row)];
+    inv_step2<S>(u, tw);
+#pragma unroll
+    for (int n1 = 0; n1 < S::R1; ++n1) {
+      if constexpr (direct)
+        put(i * S::R1 + n1, row0 + row < rows_total ? row : -1, S::R2 * n1 + n2, &u[n1]);
+      else
+        buf[Lay::at(S::R2 * n1 + n2, row)] = u[n1];
     }
   }
-  block_norms(amax, sum2, part + (blockIdx.y * gridDim.x + blockIdx.x));
+  if constexpr (!direct) {
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < CNT; ++it) {
+      int row, jj;
+      where(it, row, jj);
+      V z[VW];
+#pragma unroll
+      for (int v = 0; v < VW; ++v) z[v] = row >= 0 ? buf[Lay::at(jj + v, row)] : V{};
+      put(it, row, jj, z);
+    }
+  }
+  if (part) block_norms(amax, sum2, part + (blockIdx.y * gridDim.x + blockIdx.x));
 }
 
 // A TMA box spans at most 256 elements per dimension: tiles along a longer

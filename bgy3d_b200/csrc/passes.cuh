@@ -59,8 +59,9 @@ struct PassKernel {
 
 template <typename T, int M> struct XPass {
   using V = typename Cx<T>::type;
-  static void fwd(int mode, const Geo &g, const T *A, const T *B, T p, int closure, V *W, const V *post, const V *tw,
-                  cudaStream_t st);
+  // mode MODE_F, MODE_J or MODE_S (t: the state of MODE_S)
+  static void fwd(int mode, const Geo &g, const T *A, const T *B, const T *t, T p, int closure, V *W, const V *post,
+                  const V *tw, cudaStream_t st);
   static void inv(const Geo &g, const V *W, const T *In, T *Out, T scale, T sub, const V *post, const V *tw,
                   NormPartial *part, cudaStream_t st);
   static void kernels(std::vector<PassKernel> &k);

@@ -8,7 +8,7 @@
 namespace rism {
 
 template <typename T, int M> constexpr size_t xs_smem() {
-  return sizeof(typename Cx<T>::type) * (size_t)(M + x_rows(M) * LayRow<M, SplitRow<M>::R2>::RS);
+  return sizeof(typename Cx<T>::type) * (size_t)(M + x_rx<T, M>() * LayRow<M, SplitRow<M>::R2>::RS);
 }
 template <typename T, int N> constexpr size_t ys_smem() {
   return sizeof(typename Cx<T>::type) * (size_t)(N * static_B<T>() + N) + 16;
@@ -22,26 +22,30 @@ template <typename T, int MODE, int N> size_t zsp_smem(int m) {  // two tile buf
 }
 
 template <typename T, int M>
-void XPass<T, M>::fwd(int mode, const Geo &g, const T *A, const T *B, T p, int closure, V *W, const V *post,
-                      const V *tw, cudaStream_t st) {
-  constexpr int RX = x_rows(M);
+void XPass<T, M>::fwd(int mode, const Geo &g, const T *A, const T *B, const T *t, T p, int closure, V *W,
+                      const V *post, const V *tw, cudaStream_t st) {
+  constexpr int RX = x_rx<T, M>();
+  constexpr size_t sm = xs_smem<T, M>();
   const dim3 grid((unsigned)((g.N1 * g.N2 + RX - 1) / RX), g.m);
   if (mode == MODE_F)
-    k_xfwd_s<T, MODE_F, M, RX><<<grid, 256, xs_smem<T, M>(), st>>>(g, A, B, p, closure, W, post, tw);
+    k_xfwd_s<T, MODE_F, M, RX><<<grid, xfwd_threads<T>(), sm, st>>>(g, A, B, nullptr, p, closure, W, post, tw);
+  else if (mode == MODE_S)
+    k_xfwd_s<T, MODE_S, M, RX><<<grid, xfwd_threads<T>(), sm, st>>>(g, A, B, t, p, closure, W, post, tw);
   else
-    k_xfwd_s<T, MODE_J, M, RX><<<grid, 256, xs_smem<T, M>(), st>>>(g, A, B, p, closure, W, post, tw);
+    k_xfwd_s<T, MODE_J, M, RX><<<grid, xfwd_threads<T>(), sm, st>>>(g, A, B, nullptr, p, closure, W, post, tw);
 }
 template <typename T, int M>
 void XPass<T, M>::inv(const Geo &g, const V *W, const T *In, T *Out, T scale, T sub, const V *post, const V *tw,
                       NormPartial *part, cudaStream_t st) {
-  constexpr int RX = x_rows(M);
+  constexpr int RX = x_rx<T, M>();
   const dim3 grid((unsigned)((g.N1 * g.N2 + RX - 1) / RX), g.m);
-  k_xinv_s<T, M, RX><<<grid, 256, xs_smem<T, M>(), st>>>(g, W, In, Out, scale, sub, post, tw, part);
+  k_xinv_s<T, M, RX><<<grid, kXThreads, xs_smem<T, M>(), st>>>(g, W, In, Out, scale, sub, post, tw, part);
 }
 template <typename T, int M> void XPass<T, M>::kernels(std::vector<PassKernel> &k) {
-  constexpr int RX = x_rows(M);
+  constexpr int RX = x_rx<T, M>();
   k.push_back({(const void *)k_xfwd_s<T, MODE_F, M, RX>, xs_smem<T, M>()});
   k.push_back({(const void *)k_xfwd_s<T, MODE_J, M, RX>, xs_smem<T, M>()});
+  k.push_back({(const void *)k_xfwd_s<T, MODE_S, M, RX>, xs_smem<T, M>()});
   k.push_back({(const void *)k_xinv_s<T, M, RX>, xs_smem<T, M>()});
 }
 

@@ -567,13 +567,15 @@ void reduce_norms(rism3d_ctx *c, int nblk, double *resid) {
 
 // The five passes of one residual (MODE_F: A = t, Bv = v, p = beta) or
 // Jacobian product (MODE_J: A = dt, Bv = d = c'(t), p = scale of dt);
-// out = (FFT^-1 ...) / N - sub * A.  Returns the number of norm partials.
+// out = (FFT^-1 ...) / N - sub * A.  Returns the number of norm partials (made
+// where `norms`).  MODE_S (shape-specialised passes only): a Jacobian product
+// with the slope at `t` (A = dt, Bv = v, p = beta).
 template <typename T, int MODE>
-int pipeline(rism3d_ctx *c, const T *A, const T *Bv, T p, T sub, T *out) {
+int pipeline(rism3d_ctx *c, const T *A, const T *Bv, T p, T sub, T *out, bool norms = true, const T *t = nullptr) {
   const int rows = c->g.N1 * c->g.N2;
   auto *W = c->work<T>();
   const bool st = c->stat[sizeof(T) == 8 ? 0 : 1];
-  const int RX = st ? x_rows(c->g.M) : c->tl<T>().RX;
+  const int RX = st ? x_rows(sizeof(T) == 8, c->g.M) : c->tl<T>().RX;
   dim3 gx((rows + RX - 1) / RX, c->m);
   const auto *twx = static_cast<const typename Cx<T>::type *>(c->plan<T>(0).tw);
   {
@@ -582,19 +584,19 @@ int pipeline(rism3d_ctx *c, const T *A, const T *Bv, T p, T sub, T *out) {
       switch (c->g.M) {
 #define XF_CASE(M)                                                                                         \
   case M:                                                                                                  \
-    XPass<T, M>::fwd(MODE, c->g, A, Bv, p, c->pd.closure, W, postw<T>(c), twx, c->stream);                 \
+    XPass<T, M>::fwd(MODE, c->g, A, Bv, t, p, c->pd.closure, W, postw<T>(c), twx, c->stream);              \
     break;
         RISM_X_LENS(XF_CASE)
 #undef XF_CASE
       }
-    } else {
+    } else if constexpr (MODE != MODE_S) {
       k_xfwd<T, MODE><<<gx, 256, xsmem<T>(c), c->stream>>>(c->g, c->plan<T>(0), RX, A, Bv, p, c->pd.closure, W,
                                                           postw<T>(c));
     }
     CKL();
   }
   launch_y<T, false>(c);
-  launch_z<T, MODE>(c);
+  launch_z<T, MODE == MODE_S ? MODE_J : MODE>(c);
   launch_y<T, true>(c);
   {
     TimeScope ts(c, TK_XINV, sizeof(T) == 8 ? 0 : 1);
@@ -603,7 +605,7 @@ int pipeline(rism3d_ctx *c, const T *A, const T *Bv, T p, T sub, T *out) {
       switch (c->g.M) {
 #define XI_CASE(M)                                                                                         \
   case M:                                                                                                  \
-    XPass<T, M>::inv(c->g, W, A, out, scale, sub, postw<T>(c), twx, c->npart, c->stream);                  \
+    XPass<T, M>::inv(c->g, W, A, out, scale, sub, postw<T>(c), twx, norms ? c->npart : nullptr, c->stream); \
     break;
         RISM_X_LENS(XI_CASE)
 #undef XI_CASE
@@ -619,16 +621,15 @@ int pipeline(rism3d_ctx *c, const T *A, const T *Bv, T p, T sub, T *out) {
 
 // F(x) -> out (iterate_t1).  resid: ||out||_inf, ||out||_2 (host), or null.
 template <typename T> void eval_F(rism3d_ctx *c, const T *x, T *out, double *resid) {
-  const int nb = pipeline<T, MODE_F>(c, x, vfield<T>(c), (T)c->pd.beta, (T)1, out);
+  const int nb = pipeline<T, MODE_F>(c, x, vfield<T>(c), (T)c->pd.beta, (T)1, out, resid != nullptr);
   if (sizeof(T) == 8) c->f_evals++; else c->f32_evals++;
   if (resid) reduce_norms(c, nb, resid);
 }
 
 // out = J(x0) (s * vin) with d = c'(x0) precomputed (jacobian_t1).
-template <typename T> void eval_J(rism3d_ctx *c, const T *d, const T *vin, double s, T *out, double *resid) {
-  const int nb = pipeline<T, MODE_J>(c, vin, d, (T)s, (T)s, out);
+template <typename T> void eval_J(rism3d_ctx *c, const T *d, const T *vin, double s, T *out) {
+  pipeline<T, MODE_J>(c, vin, d, (T)s, (T)s, out, false);
   if (sizeof(T) == 8) c->jv_evals++; else c->jv32_evals++;
-  if (resid) reduce_norms(c, nb, resid);
 }
 
 int vec_grid(long long n) {
@@ -768,7 +769,7 @@ int gmres(rism3d_ctx *c, const T *d, const T *b, T *x, double rtol, int maxit, i
     // nothing), else B0 = b - J x
     T *r0 = const_cast<T *>(b);
     if (have_x) {
-      eval_J<T>(c, d, x, 1.0, B[0], nullptr);  // B0 = J x
+      eval_J<T>(c, d, x, 1.0, B[0]);  // B0 = J x
       xpay<T, T, T>(c, b, -1.0, B[0], B[0]);   // B0 = b - J x
       r0 = B[0];
       its++;
@@ -782,7 +783,7 @@ int gmres(rism3d_ctx *c, const T *d, const T *b, T *x, double rtol, int maxit, i
     int j = 0;
     bool done = false;
     for (; j < restart && its < maxit; ++j) {
-      eval_J<T>(c, d, V[j].p, V[j].s, B[j + 1], nullptr);
+      eval_J<T>(c, d, V[j].p, V[j].s, B[j + 1]);
       its++;
       double hn;
       if ((int)V.size() <= kVecMax) {
@@ -893,6 +894,27 @@ template <typename TS, typename TJ> void closure_slope(rism3d_ctx *c, const TS *
   k_slope_any<TS><<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, x, c->v64, c->pd.beta, c->pd.closure,
                                                                        d32, d64);
   CKL();
+}
+
+// One Jacobian product at x from scratch (the jacobian_t1 entry points).  The
+// shape-specialised x pass takes the slope from x and v as it goes, where a
+// slope field beforehand cost a write and a read of it (246 us of a 1256 us
+// FP64 product at 256^3).
+template <typename T> int jacobian_product(rism3d_ctx *c, const T *x, const T *dx, T *out) {
+  const int pr = sizeof(T) == 8 ? 0 : 1;
+  if (c->stat[pr] && !c->pure) {
+    pipeline<T, MODE_S>(c, dx, vfield<T>(c), (T)c->pd.beta, (T)1, out, false, x);
+    if (pr == 0) c->jv_evals++; else c->jv32_evals++;
+  } else {
+    T *d = slopebuf<T>(c);
+    if constexpr (sizeof(T) == 8) {
+      if (c->pure) eval_F<double>(c, x, out, nullptr);  // C(k) at x for the OZ differential
+    }
+    closure_slope<T, T>(c, x, d);
+    eval_J<T>(c, d, dx, 1.0, out);
+  }
+  CK(cudaStreamSynchronize(c->stream));
+  return RISM3D_OK;
 }
 
 // ------------------------------------------------ two-grid preconditioner
@@ -1138,7 +1160,7 @@ void coarse_solve_dev(rism3d_ctx *c, int k) {
   k_scale_norm<float><<<gv, 256, 0, st>>>(cc->nvec, B[0], nrm, beta);
   CKL();
   for (int j = 0; j < k; ++j) {
-    pipeline<float, MODE_J>(cc, B[j], d, 1.f, 1.f, B[j + 1]);
+    pipeline<float, MODE_J>(cc, B[j], d, 1.f, 1.f, B[j + 1], false);
     VecSet<float> vs{};
     for (int i = 0; i < kVecMax; ++i) vs.p[i] = B[i <= j ? i : 0];
     double *h = H + (size_t)j * (k + 1);
@@ -1449,7 +1471,7 @@ int fgmres(rism3d_ctx *c, const T *d, const T *b, T *x, double rtol, int maxit, 
     // nothing), else B0 = b - J x
     T *r0 = const_cast<T *>(b);
     if (have_x) {
-      eval_J<T>(c, d, x, 1.0, B[0], nullptr);  // B0 = J x
+      eval_J<T>(c, d, x, 1.0, B[0]);  // B0 = J x
       its++;
       xpay<T, T, T>(c, b, -1.0, B[0], B[0]);   // B0 = b - J x
       r0 = B[0];
@@ -1466,7 +1488,7 @@ int fgmres(rism3d_ctx *c, const T *d, const T *b, T *x, double rtol, int maxit, 
       ensure_basis<T>(c, j + 2);
       while ((int)Z.size() <= j) Z.push_back(dalloc<T>(c->nvec));
       tg_apply<T>(c, V[j].p, V[j].s, Z[j]);
-      eval_J<T>(c, d, Z[j], 1.0, B[j + 1], nullptr);
+      eval_J<T>(c, d, Z[j], 1.0, B[j + 1]);
       its++;
       double hn;
       if ((int)V.size() <= kVecMax) {
@@ -1800,7 +1822,7 @@ void fwd3d(rism3d_ctx *c, const double *A) {
 // out = K v = (chi - 1) * v (the OZ convolution alone): the J.v passes with
 // unit slope and nothing subtracted.
 void kconv(rism3d_ctx *c, const double *ones, const double *v, double *out) {
-  pipeline<double, MODE_J>(c, v, ones, 1.0, 0.0, out);
+  pipeline<double, MODE_J>(c, v, ones, 1.0, 0.0, out, false);
 }
 
 double *ones_field(rism3d_ctx *c) {
@@ -1968,7 +1990,7 @@ int response_impl(rism3d_ctx *c, const double *T, rism3d_grad *gr) {
       CKL();
       // B = beta (chi - 1) * ((c' + 1) dv): the Jacobian passes with slope
       // c' + 1 and nothing subtracted (jacobian_t1 with its flag set)
-      pipeline<double, MODE_J>(c, dv, d1, pd.beta, 0.0, B);
+      pipeline<double, MODE_J>(c, dv, d1, pd.beta, 0.0, B, false);
       const double bnorm = maxpy<double>(c, B, 1.0, {}, {}, true);
       axpby<double, double>(c, 1.0, B, 0.0, Bc);  // the solvers may overwrite B
       if (c->coarse) fgmres<double>(c, d, B, dT, 1e-11, 4000, restart);
@@ -1977,7 +1999,7 @@ int response_impl(rism3d_ctx *c, const double *T, rism3d_grad *gr) {
                                        part + (size_t)(3 * u + dim) * rb);
       CKL();
       // true residual of the solve: B - J dT (into dv, no longer needed)
-      eval_J<double>(c, d, dT, 1.0, dv, nullptr);
+      eval_J<double>(c, d, dT, 1.0, dv);
       xpay<double, double, double>(c, Bc, -1.0, dv, dv);
       const double rn = maxpy<double>(c, dv, 1.0, {}, {}, true);
       if (bnorm > 0) worst = std::max(worst, rn / bnorm);
@@ -2145,7 +2167,7 @@ template <typename T> void tune_precision(rism3d_ctx *c, const T *A, const T *Bv
   const int reps = G.Nr >= (1LL << 22) ? 2 : 5;
   const bool had_stat = c->stat[pr];
   c->stat[pr] = false;
-  auto run = [&] { pipeline<T, MODE_J>(c, A, Bv, (T)1, (T)1, out); };
+  auto run = [&] { pipeline<T, MODE_J>(c, A, Bv, (T)1, (T)1, out, false); };
   const int cand[4] = {4, 8, 16, 32};
   // one axis at a time, the others held
   int *fields[3] = {&t.RX, &t.BY, &t.BZ};
@@ -3390,12 +3412,7 @@ int rism3d_jacobian_t1(rism3d_ctx *ctx, const double *T, const double *dT, doubl
   if (!ctx || !T || !dT || !JdT) return RISM3D_ERR_ARG;
   if (ctx->pd.closure == RISM3D_PY) return RISM3D_ERR_UNSUPPORTED;
   return guard([&] {
-    double *d = slopebuf<double>(ctx);
-    if (ctx->pure) eval_F<double>(ctx, T, JdT, nullptr);  // C(k) at T for the OZ differential
-    closure_slope<double, double>(ctx, T, d);
-    eval_J<double>(ctx, d, dT, 1.0, JdT, nullptr);
-    CK(cudaStreamSynchronize(ctx->stream));
-    return RISM3D_OK;
+    return jacobian_product<double>(ctx, T, dT, JdT);
   });
 }
 
@@ -3415,11 +3432,7 @@ int rism3d_jacobian_t1_f32(rism3d_ctx *ctx, const float *T, const float *dT, flo
   if (!ctx || !T || !dT || !JdT) return RISM3D_ERR_ARG;
   if (ctx->pd.closure == RISM3D_PY) return RISM3D_ERR_UNSUPPORTED;
   return guard([&] {
-    float *d = slopebuf<float>(ctx);
-    closure_slope<float, float>(ctx, T, d);
-    eval_J<float>(ctx, d, dT, 1.0, JdT, nullptr);
-    CK(cudaStreamSynchronize(ctx->stream));
-    return RISM3D_OK;
+    return jacobian_product<float>(ctx, T, dT, JdT);
   });
 }
 
