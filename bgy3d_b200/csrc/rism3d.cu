@@ -2814,6 +2814,8 @@ template <int MS> void chi_out_launch(rism3d_ctx *c, double2 *out) {
 
 // Newton-GMRES on the pair fields from T (device, in/out), then the
 // observables, chi - 1 on the k grid and g (host outputs, each optional).
+void d2h_large(void *dst, const void *src, size_t bytes, cudaStream_t st);
+
 int solvent_solve_impl(rism3d_ctx *c, double *T, double *chi_out, double *g_out, rism3d_solvent_result *res) {
   const rism3d_problem &pd = c->pd;
   *res = rism3d_solvent_result{};
@@ -2845,11 +2847,10 @@ int solvent_solve_impl(rism3d_ctx *c, double *T, double *chi_out, double *g_out,
       case 3: chi_out_launch<3>(c, dchi); break;
       default: chi_out_launch<4>(c, dchi); break;
     }
-    CK(cudaMemcpyAsync(chi_out, dchi, sizeof(double2) * (size_t)c->m * nk, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    d2h_large(chi_out, dchi, sizeof(double2) * (size_t)c->m * nk, c->stream);
     dfree(dchi);
   }
-  if (g_out) CK(cudaMemcpyAsync(g_out, g, sizeof(double) * nv, cudaMemcpyDeviceToHost, c->stream));
+  if (g_out) d2h_large(g_out, g, sizeof(double) * nv, c->stream);
   CK(cudaEventRecord(e1, c->stream));
   CK(cudaEventSynchronize(e1));
   float ms = 0;
@@ -3023,65 +3024,84 @@ int info_impl(rism3d_ctx *c, const double *T, rism3d_info_result *res, double *s
 
 // Device -> host copy of a large result into caller memory that is
 // pageable (a NumPy array, a PETSc Vec): the driver's pageable path runs at
-// a few GB/s there.  Here the copy is split into kLanes contiguous slices,
+// a few GB/s there.  Here the copy is split into up to kLanes contiguous slices,
 // each run by its own host thread on its own stream through two alternating
 // pinned pieces: the DMA of piece i of a slice runs while its thread copies
 // piece i-1 out, and the lanes run side by side, so the PCIe transfer and
 // the host copy (402 MB: 7 ms and, on 8 threads, 5.5 ms on the B200 hosts)
-// overlap instead of alternating.  The lane sets (kLanes streams and 2 x
-// kLanes pieces of kPiece bytes: 64 MB pinned) come from a process-wide free
-// list, one per concurrent caller, held until exit.  Copies below 32 MB take
-// the plain cudaMemcpy.
+// overlap instead of alternating.  The lane sets (at most kLanes streams and 2 x
+// kLanes pieces of kPiece bytes: 64 MB pinned; made as the copies need them)
+// come from a process-wide free list, one per concurrent caller, held until
+// exit.  Copies below 16 MB take the plain cudaMemcpy: g at 64^3 (6.3 MB) adds 0.5
+// ms to a call with it and 1.0 with the lanes' threads, t and g at 96^3 (2 x 21
+// MB, t both ways) 5.9 and 4.6.
 constexpr size_t kPiece = size_t(4) << 20;
 constexpr int kLanes = 8;
+constexpr size_t kStagedMin = size_t(16) << 20;
 struct LaneSet {
   void *buf[kLanes][2] = {};
+  size_t cap[kLanes][2] = {};
   cudaStream_t st[kLanes] = {};
   cudaEvent_t ev[kLanes][2] = {};
 };
 std::mutex g_stage_mu;
 std::vector<LaneSet *> g_stage_free;
 
-LaneSet *lane_set_new() {
-  auto *ls = new LaneSet;
+// How a copy is split: about a megabyte per lane and two pieces of it, up to
+// kLanes lanes of kPiece pieces.
+struct LanePlan {
+  int lanes;
+  size_t piece, slice;
+  explicit LanePlan(size_t bytes) {
+    lanes = (int)std::min<size_t>(kLanes, std::max<size_t>(1, bytes >> 20));
+    const size_t unit = size_t(256) << 10;
+    piece = std::min(kPiece, (bytes / (2 * (size_t)lanes) + unit - 1) / unit * unit);
+    slice = ((bytes + lanes - 1) / lanes + piece - 1) / piece * piece;
+  }
+};
+
+// Streams, events and pinned pieces of the plan's lanes, as far as the set does
+// not hold them yet.
+void lane_set_fit(LaneSet *ls, const LanePlan &p) {
+  for (int l = 0; l < p.lanes; ++l) {
+    for (int b = 0; b < 2; ++b) {
+      if (ls->cap[l][b] < p.piece) {
+        if (ls->buf[l][b]) CK(cudaFreeHost(ls->buf[l][b]));
+        ls->buf[l][b] = nullptr;
+        ls->cap[l][b] = 0;
+        CK(cudaHostAlloc(&ls->buf[l][b], p.piece, cudaHostAllocPortable));
+        ls->cap[l][b] = p.piece;
+      }
+      if (!ls->ev[l][b]) CK(cudaEventCreateWithFlags(&ls->ev[l][b], cudaEventDisableTiming));
+    }
+    if (!ls->st[l]) CK(cudaStreamCreateWithFlags(&ls->st[l], cudaStreamNonBlocking));
+  }
+}
+
+LaneSet *lane_set_take(const LanePlan &p) {
+  LaneSet *ls = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    if (!g_stage_free.empty()) {
+      ls = g_stage_free.back();
+      g_stage_free.pop_back();
+    }
+  }
+  if (!ls) ls = new LaneSet;
   try {
-    for (int l = 0; l < kLanes; ++l) {
-      for (int b = 0; b < 2; ++b) {
-        CK(cudaHostAlloc(&ls->buf[l][b], kPiece, cudaHostAllocPortable));
-        CK(cudaEventCreateWithFlags(&ls->ev[l][b], cudaEventDisableTiming));
-      }
-      CK(cudaStreamCreateWithFlags(&ls->st[l], cudaStreamNonBlocking));
-    }
-  } catch (...) {
-    for (int l = 0; l < kLanes; ++l) {
-      for (int b = 0; b < 2; ++b) {
-        if (ls->buf[l][b]) cudaFreeHost(ls->buf[l][b]);
-        if (ls->ev[l][b]) cudaEventDestroy(ls->ev[l][b]);
-      }
-      if (ls->st[l]) cudaStreamDestroy(ls->st[l]);
-    }
-    delete ls;
+    lane_set_fit(ls, p);
+  } catch (...) {  // keeps what it has; nothing is in flight on it
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    g_stage_free.push_back(ls);
     throw;
   }
   return ls;
 }
 
-LaneSet *lane_set_take() {
-  {
-    std::lock_guard<std::mutex> lk(g_stage_mu);
-    if (!g_stage_free.empty()) {
-      LaneSet *ls = g_stage_free.back();
-      g_stage_free.pop_back();
-      return ls;
-    }
-  }
-  return lane_set_new();
-}
-
-// Runs lane(l) for l < kLanes, lanes 1.. on their own threads.
-template <typename F> void run_lanes(F &&lane) {
+// Runs lane(l) for l < lanes, lanes 1.. on their own threads.
+template <typename F> void run_lanes(int lanes, F &&lane) {
   std::vector<std::thread> th;
-  for (int l = 1; l < kLanes; ++l) {
+  for (int l = 1; l < lanes; ++l) {
     try {
       th.emplace_back(lane, l);
     } catch (const std::system_error &) {  // no thread to be had: run the lane here
@@ -3095,7 +3115,8 @@ template <typename F> void run_lanes(F &&lane) {
 // The set goes back only once none of its streams can still be moving data.
 void lane_set_give(LaneSet *ls, bool failed) {
   bool clean = !failed;
-  for (int l = 0; l < kLanes; ++l) clean = clean && cudaStreamSynchronize(ls->st[l]) == cudaSuccess;
+  for (int l = 0; l < kLanes; ++l)
+    if (ls->st[l]) clean = clean && cudaStreamSynchronize(ls->st[l]) == cudaSuccess;
   if (clean) {
     std::lock_guard<std::mutex> lk(g_stage_mu);
     g_stage_free.push_back(ls);
@@ -3110,24 +3131,25 @@ void lane_set_give(LaneSet *ls, bool failed) {
 // lane copies a piece into pinned memory and moves it while it fills the
 // other; complete (and ordered before later work on st) on return.
 void h2d_large(void *dst, const void *src, size_t bytes, cudaStream_t st) {
-  if (bytes < (size_t(32) << 20)) {
+  if (bytes < kStagedMin) {
     CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
     CK(cudaStreamSynchronize(st));
     return;
   }
-  LaneSet *ls = lane_set_take();
+  const LanePlan plan(bytes);
+  LaneSet *ls = lane_set_take(plan);
   cudaEvent_t ready = nullptr;  // dst (stream-ordered on st) exists
   CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
   CK(cudaEventRecord(ready, st));
   std::atomic<int> failed{0};
-  const size_t slice = ((bytes + kLanes - 1) / kLanes + kPiece - 1) / kPiece * kPiece;
-  run_lanes([&](int l) {
+  const size_t slice = plan.slice, piece = plan.piece;
+  run_lanes(plan.lanes, [&](int l) {
     const size_t a = std::min(bytes, (size_t)l * slice), b = std::min(bytes, a + slice);
     if (a >= b) return;
     if (cudaStreamWaitEvent(ls->st[l], ready, 0) != cudaSuccess) { failed = 1; return; }
     size_t i = 0;
-    for (size_t off = a; off < b; off += kPiece, ++i) {
-      const size_t len = std::min(kPiece, b - off);
+    for (size_t off = a; off < b; off += piece, ++i) {
+      const size_t len = std::min(piece, b - off);
       // the DMA that last read this buffer (two pieces ago) has finished
       if (i >= 2 && cudaEventSynchronize(ls->ev[l][i & 1]) != cudaSuccess) { failed = 1; return; }
       std::memcpy(ls->buf[l][i & 1], static_cast<const char *>(src) + off, len);
@@ -3144,26 +3166,27 @@ void h2d_large(void *dst, const void *src, size_t bytes, cudaStream_t st) {
 }
 
 void d2h_large(void *dst, const void *src, size_t bytes, cudaStream_t st) {
-  if (bytes < (size_t(32) << 20)) {
+  if (bytes < kStagedMin) {
     CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     return;
   }
-  LaneSet *ls = lane_set_take();
+  const LanePlan plan(bytes);
+  LaneSet *ls = lane_set_take(plan);
   // the lanes' streams start once the source is complete on st
   cudaEvent_t ready = nullptr;
   CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
   CK(cudaEventRecord(ready, st));
   std::atomic<int> failed{0};
-  const size_t slice = ((bytes + kLanes - 1) / kLanes + kPiece - 1) / kPiece * kPiece;
+  const size_t slice = plan.slice, piece = plan.piece;
   auto lane = [&](int l) {
     const size_t a = std::min(bytes, (size_t)l * slice), b = std::min(bytes, a + slice);
     if (a >= b) return;
     if (cudaStreamWaitEvent(ls->st[l], ready, 0) != cudaSuccess) { failed = 1; return; }
     size_t prev_off = 0, prev_len = 0;
-    for (size_t off = a, i = 0;; off += kPiece, ++i) {
+    for (size_t off = a, i = 0;; off += piece, ++i) {
       const bool more = off < b;
-      const size_t len = more ? std::min(kPiece, b - off) : 0;
+      const size_t len = more ? std::min(piece, b - off) : 0;
       if (more) {
         if (cudaMemcpyAsync(ls->buf[l][i & 1], static_cast<const char *>(src) + off, len, cudaMemcpyDeviceToHost,
                             ls->st[l]) != cudaSuccess ||
@@ -3181,7 +3204,7 @@ void d2h_large(void *dst, const void *src, size_t bytes, cudaStream_t st) {
       prev_len = len;
     }
   };
-  run_lanes(lane);
+  run_lanes(plan.lanes, lane);
   cudaEventDestroy(ready);
   lane_set_give(ls, failed != 0);
 }
@@ -3286,23 +3309,24 @@ void cache_clear() {
   for (auto &e : all) delete e.ctx;
 }
 
-// Writes one byte into every page of [p, p + bytes) from a few host threads:
-// a caller's fresh result buffer (a NumPy array) takes its first-touch page
-// faults here, while the device solves, instead of inside the copy-out.
+// Rewrites one byte of every page of [p, p + bytes) with its own value from a
+// few host threads: a caller's fresh result buffer (a NumPy array) takes its
+// first-touch page faults here, while the device solves, instead of inside the
+// copy-out.
 struct PageToucher {
   std::vector<std::thread> th;
   PageToucher(void *p, size_t bytes) {
-    if (!p || bytes < (size_t(64) << 20)) return;
+    if (!p || bytes < kStagedMin) return;
     const long pg = 4096;
-    const int nthr = 4;
+    const int nthr = bytes < (size_t(64) << 20) ? 1 : 4;
     const size_t slice = (bytes / nthr + pg - 1) / pg * pg;
     for (int q = 0; q < nthr; ++q) {
-      const size_t a = std::min(bytes, q * slice), b = std::min(bytes, (q + 1) * slice);
+      const size_t a = std::min(bytes, q * slice), b = q + 1 == nthr ? bytes : std::min(bytes, (q + 1) * slice);
       if (a >= b) continue;
       try {
         th.emplace_back([=] {
           volatile char *c = static_cast<char *>(p);
-          for (size_t o = a; o < b; o += pg) c[o] = 0;
+          for (size_t o = a; o < b; o += pg) c[o] = c[o];
         });
       } catch (const std::system_error &) {
         break;  // no thread: the copy-out takes the faults
@@ -3324,13 +3348,14 @@ int solve_on(rism3d_ctx *ctx, double *t_inout, double *g_out, rism3d_result *out
   struct Free { double *a, *b; ~Free() { dfree(a); dfree(b); } } fr{T, g};
   if (t_inout) h2d_large(T, t_inout, bytes, ctx->stream);
   else CK(cudaMemsetAsync(T, 0, bytes, ctx->stream));
-  PageToucher touch(g_out, bytes);  // g_out is written in full below; its old contents do not matter
+  PageToucher touch(g_out, bytes), touch_t(t_inout, bytes);
   rism3d_result r{};
   int st = solve_impl(ctx, T, &r);
   observables_impl(ctx, T, g, &r);
   r.launches += 2;  // the observables' kernels
   r.status = st;
   touch.join();
+  touch_t.join();
   if (t_inout) d2h_large(t_inout, T, bytes, ctx->stream);
   if (g_out) d2h_large(g_out, g, bytes, ctx->stream);
   if (out) *out = r;
@@ -3566,10 +3591,12 @@ int rism3d_solvent_solve(const rism3d_problem *pd, int m, const rism3d_site *sol
       const size_t bytes = sizeof(double) * ctx->nvec;
       double *T = dalloc<double>(ctx->nvec);
       struct Free { double *a; ~Free() { dfree(a); } } fr{T};
-      if (t_in) CK(cudaMemcpy(T, t_in, bytes, cudaMemcpyHostToDevice));
+      if (t_in) h2d_large(T, t_in, bytes, ctx->stream);
       else solvent_guess(ctx, T);
+      const size_t nk = (size_t)ctx->g.Nh * ctx->g.N1 * ctx->g.N2;
+      PageToucher touch_t(t_out, bytes), touch_chi(chi_out, sizeof(double2) * ctx->m * nk), touch_g(g_out, bytes);
       const int st = solvent_solve_impl(ctx, T, chi_out, g_out, &res);
-      if (t_out) CK(cudaMemcpy(t_out, T, bytes, cudaMemcpyDeviceToHost));
+      if (t_out) d2h_large(t_out, T, bytes, ctx->stream);
       return st;
     });
     rism3d_ctx_destroy(ctx);
@@ -3669,15 +3696,15 @@ int rism3d_solute_grad(const rism3d_problem *pd, int m, const rism3d_site *solve
     const size_t bytes = sizeof(double) * ctx->nvec;
     double *T = dalloc<double>(ctx->nvec);
     struct Free { double *a; ~Free() { dfree(a); } } fr{T};
-    if (t_inout) CK(cudaMemcpy(T, t_inout, bytes, cudaMemcpyHostToDevice));
-    else CK(cudaMemset(T, 0, bytes));
+    if (t_inout) h2d_large(T, t_inout, bytes, ctx->stream);
+    else CK(cudaMemsetAsync(T, 0, bytes, ctx->stream));
     rism3d_result r{};
     int st = solve_impl(ctx, T, &r);
     observables_impl(ctx, T, nullptr, &r);
     r.status = st;
     if (st == RISM3D_OK) st = gradient_impl(ctx, T, grad);
     if (st == RISM3D_OK && grad->dx_reference) st = reference_gradient_impl(ctx, T, grad->dx_reference);
-    if (t_inout) CK(cudaMemcpy(t_inout, T, bytes, cudaMemcpyDeviceToHost));
+    if (t_inout) d2h_large(t_inout, T, bytes, ctx->stream);
     if (out) *out = r;
     return st;
   });
