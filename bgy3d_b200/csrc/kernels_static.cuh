@@ -320,8 +320,11 @@ template <typename V, int N, int B> __host__ __device__ constexpr bool tma_tile_
 }
 
 // y pass: one [N][B] tile (kx0 .. kx0+B-1 at fixed z, site) by TMA.
-// tm: W as {2 Nhp, N1, m N2} scalars, box {2B, N1, 1}.
-template <typename T, bool INV, int N, int B>
+// tm: W as {2 Nhp, N1, m N2} scalars, box {2B, N1, 1}.  ALONG_Z: the same
+// along z, at fixed y (box {2B, 1, N2}): the z transform alone, for the passes
+// whose work at a k point is a kernel of its own (k_oz, the forward transform
+// of the gradient).
+template <typename T, bool INV, int N, int B, bool ALONG_Z = false>
 __global__ void __launch_bounds__(SplitY<N>::R1 * B) k_y_s(Geo g, const __grid_constant__ CUtensorMap tm,
                                                          const typename Cx<T>::type *__restrict__ twg,
                                                          int *__restrict__ err) {
@@ -333,22 +336,24 @@ __global__ void __launch_bounds__(SplitY<N>::R1 * B) k_y_s(Geo g, const __grid_c
   V *tw = buf + N * B;
   uint64_t *bar = reinterpret_cast<uint64_t *>(tw + N);
   const int tid = threadIdx.x;
-  const int kx0 = blockIdx.x * B, z = blockIdx.y, site = blockIdx.z;
+  const int kx0 = blockIdx.x * B, f = blockIdx.y, site = blockIdx.z;  // f: the fixed z (or y)
   if (tid == 0) mbar_init(bar, 1);
   __syncthreads();
   if (tid == 0) {
     mbar_expect_tx(bar, (uint32_t)(N * B * sizeof(V)));
 #pragma unroll
-    for (int c = 0; c < N; c += tma_rows(N)) tma_load_3d(buf + c * B, &tm, bar, 2 * kx0, c, site * g.N2 + z);
+    for (int c = 0; c < N; c += tma_rows(N))
+      tma_load_3d(buf + c * B, &tm, bar, 2 * kx0, ALONG_Z ? f : c, site * g.N2 + (ALONG_Z ? c : f));
   }
   for (int q = tid; q < N; q += NTHR) tw[q] = twg[q];
-  if (!cta_wait_tile(bar, 0, kMbarPolls, err, 1)) return;
+  if (!cta_wait_tile(bar, 0, kMbarPolls, err, ALONG_Z ? 2 : 1)) return;
   fft2<N, B, NTHR, INV, true, LayCol<N, B>, SplitY<N>>(buf, tw);
   fence_proxy_async();
   __syncthreads();
   if (tid == 0) {
 #pragma unroll
-    for (int c = 0; c < N; c += tma_rows(N)) tma_store_3d(&tm, buf + c * B, 2 * kx0, c, site * g.N2 + z);
+    for (int c = 0; c < N; c += tma_rows(N))
+      tma_store_3d(&tm, buf + c * B, 2 * kx0, ALONG_Z ? f : c, site * g.N2 + (ALONG_Z ? c : f));
     tma_commit();
     tma_wait_read0();
   }

@@ -17,8 +17,8 @@ namespace rism {
 // every grid of 32 .. 512 points (even 2^a 3^b), along each axis.  The
 // runtime-length passes (one barrier pair per radix, indices divided at run
 // time) are several times slower at every one of them, so a shape is here if
-// its two-step split fits registers; the rest (below 32 points, more than
-// three solvent sites, a 3D chi) keeps them.  FP32 J.v, all five passes,
+// its two-step split fits registers; axes below 32 points keep them, and so
+// does the z pass of more than three solvent sites or a 3D chi.  FP32 J.v, all five passes,
 // runtime-length -> here, us: 32^3 48 -> 14, 54^3 98 -> 20, 108^3 373 -> 59,
 // 162^3 1265 -> 182, 288^3 6160 -> 822, 486^3 31100 -> 6060.
 #define RISM_X_LENS(X)                                                                                      \
@@ -70,6 +70,12 @@ template <typename T, int M> struct XPass {
 template <typename T, int N> struct YPass {
   using V = typename Cx<T>::type;
   static void run(bool inv, const Geo &g, const CUtensorMap &tm, const V *tw, int *err, cudaStream_t st);
+  static void kernels(std::vector<PassKernel> &k);
+};
+
+// The z transform alone (FP64, tiles of the y pass's width).
+template <int N> struct ZAxis {
+  static void run(bool inv, const Geo &g, const CUtensorMap &tm, const double2 *tw, int *err, cudaStream_t st);
   static void kernels(std::vector<PassKernel> &k);
 };
 

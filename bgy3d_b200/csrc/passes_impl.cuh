@@ -62,6 +62,19 @@ template <typename T, int N> void YPass<T, N>::kernels(std::vector<PassKernel> &
   k.push_back({(const void *)k_y_s<T, false, N, B>, ys_smem<T, N>()});
 }
 
+template <int N>
+void ZAxis<N>::run(bool inv, const Geo &g, const CUtensorMap &tm, const double2 *tw, int *err, cudaStream_t st) {
+  constexpr int B = static_B<double>();
+  const dim3 grid((g.Nh + B - 1) / B, g.N1, g.m);
+  if (inv) k_y_s<double, true, N, B, true><<<grid, SplitY<N>::R1 * B, ys_smem<double, N>(), st>>>(g, tm, tw, err);
+  else k_y_s<double, false, N, B, true><<<grid, SplitY<N>::R1 * B, ys_smem<double, N>(), st>>>(g, tm, tw, err);
+}
+template <int N> void ZAxis<N>::kernels(std::vector<PassKernel> &k) {
+  constexpr int B = static_B<double>();
+  k.push_back({(const void *)k_y_s<double, true, N, B, true>, ys_smem<double, N>()});
+  k.push_back({(const void *)k_y_s<double, false, N, B, true>, ys_smem<double, N>()});
+}
+
 template <typename T, int MODE, int N>
 void z_run(int B, bool persistent, const Geo &g, const CUtensorMap &tm, const typename Cx<T>::type *tw,
            const ZParams<T> &zp, int *err, cudaStream_t st) {
@@ -113,7 +126,8 @@ template <typename T, int N> void ZPass<T, N>::kernels(int m, std::vector<PassKe
   template struct XPass<double, M>;
 #define RISM_INST_Y(N)              \
   template struct YPass<float, N>; \
-  template struct YPass<double, N>;
+  template struct YPass<double, N>; \
+  template struct ZAxis<N>;
 #define RISM_INST_Z(N)              \
   template struct ZPass<float, N>; \
   template struct ZPass<double, N>;

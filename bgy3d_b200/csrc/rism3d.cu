@@ -287,9 +287,10 @@ struct rism3d_ctx {
   // shape-specialised passes: available per precision ([0] FP64, [1] FP32),
   // with TMA descriptors of W for the y and z tiles
   bool stat[2] = {false, false};
+  bool xy[2] = {false, false};  // ... of the x and y passes alone: more sites, a 3D chi
   int zb[2] = {4, 8};  // z tile width of the shape-specialised z pass ([0] FP64, [1] FP32: 8 or 4)
   bool zpers[2] = {false, false};  // that z pass from persistent double-buffered CTAs
-  CUtensorMap tmy[2], tmz[2];
+  CUtensorMap tmy[2], tmz[2], tmza;  // tmza: ZAxis
   int *d_err = nullptr;  // set by a kernel whose bounded wait timed out
 
   ~rism3d_ctx() {
@@ -448,7 +449,7 @@ void make_tmap(rism3d_ctx *c, CUtensorMap *tm, bool fp64, int B, int by, int bz)
 template <typename T, bool INV> void launch_y(rism3d_ctx *c) {
   TimeScope ts(c, TK_Y, sizeof(T) == 8 ? 0 : 1);
   auto *W = c->work<T>();
-  if (c->stat[sizeof(T) == 8 ? 0 : 1]) {
+  if (c->xy[sizeof(T) == 8 ? 0 : 1]) {
     const CUtensorMap &tm = c->tmy[sizeof(T) == 8 ? 0 : 1];
     const auto *tw = static_cast<const typename Cx<T>::type *>(c->plan<T>(1).tw);
     switch (c->g.N1) {
@@ -474,6 +475,20 @@ void allow_smem(const void *fn, size_t need);
 unsigned persistent_grid(const void *fn, size_t smem, unsigned work, int threads);
 int optin_limit();
 
+// The z transform alone, shape-specialised (c->xy), FP64.
+void launch_zaxis(rism3d_ctx *c, bool inv) {
+  const auto *tw = static_cast<const double2 *>(c->plan<double>(2).tw);
+  switch (c->g.N2) {
+#define ZA_CASE(N)                                                       \
+  case N:                                                                \
+    ZAxis<N>::run(inv, c->g, c->tmza, tw, c->d_err, c->stream);          \
+    break;
+    RISM_YZ_LENS(ZA_CASE)
+#undef ZA_CASE
+  }
+  CKL();
+}
+
 // z pass of a pure-solvent context (solvent.cuh), FP64, for MS solvent sites.
 template <int MODE, int MS> void launch_oz_ms(rism3d_ctx *c) {
   PureParams<MS> pp{};
@@ -485,10 +500,18 @@ template <int MODE, int MS> void launch_oz_ms(rism3d_ctx *c) {
     pp.q2[p] = c->pq2[p];
     pp.wr[p] = c->pwr[p];
   }
+  auto *W = c->work<double>();
+  if (c->xy[0]) {
+    if (MODE != MODE_VL) launch_zaxis(c, false);
+    const long long np = (long long)c->g.Nh * c->g.N1 * c->g.N2;
+    k_oz<MODE, MS><<<(unsigned)((np + 127) / 128), 128, 0, c->stream>>>(c->g, W, pp);
+    CKL();
+    launch_zaxis(c, true);
+    return;
+  }
   const int B = c->tl<double>().BZ;
   dim3 grid((c->g.Nh + B - 1) / B, c->g.N1);
   const size_t sm = zsmem<double>(c);
-  auto *W = c->work<double>();
   if (B == 16) k_z_oz<MODE, 16, MS><<<grid, 256, sm, c->stream>>>(c->g, c->plan<double>(2), W, pp);
   else if (B == 8) k_z_oz<MODE, 8, MS><<<grid, 256, sm, c->stream>>>(c->g, c->plan<double>(2), W, pp);
   else k_z_oz<MODE, 4, MS><<<grid, 256, sm, c->stream>>>(c->g, c->plan<double>(2), W, pp);
@@ -574,7 +597,7 @@ template <typename T, int MODE>
 int pipeline(rism3d_ctx *c, const T *A, const T *Bv, T p, T sub, T *out, bool norms = true, const T *t = nullptr) {
   const int rows = c->g.N1 * c->g.N2;
   auto *W = c->work<T>();
-  const bool st = c->stat[sizeof(T) == 8 ? 0 : 1];
+  const bool st = c->xy[sizeof(T) == 8 ? 0 : 1];
   const int RX = st ? x_rows(sizeof(T) == 8, c->g.M) : c->tl<T>().RX;
   dim3 gx((rows + RX - 1) / RX, c->m);
   const auto *twx = static_cast<const typename Cx<T>::type *>(c->plan<T>(0).tw);
@@ -902,7 +925,7 @@ template <typename TS, typename TJ> void closure_slope(rism3d_ctx *c, const TS *
 // FP64 product at 256^3).
 template <typename T> int jacobian_product(rism3d_ctx *c, const T *x, const T *dx, T *out) {
   const int pr = sizeof(T) == 8 ? 0 : 1;
-  if (c->stat[pr] && !c->pure) {
+  if (c->xy[pr] && !c->pure) {
     pipeline<T, MODE_S>(c, dx, vfield<T>(c), (T)c->pd.beta, (T)1, out, false, x);
     if (pr == 0) c->jv_evals++; else c->jv32_evals++;
   } else {
@@ -990,7 +1013,7 @@ bool fx_usable(const rism3d_ctx *c) {
   if (dense && dense[0] == '1') return false;
   return c->tC && static_len_x(c->g.M) && c->Nc[0] % 2 == 0 && c->Nc[0] / 2 < c->g.M;
 }
-// Both sides by FFT (twogrid_fx2.cu) where the coarse half row also has a
+// Both sides by FFT (twogrid_fx2.cuh) where the coarse half row also has a
 // shape-specialised transform; RISM3D_DENSE_TRANSFERS=2 keeps the (K+1) x Nc
 // table product on the coarse side (tests compare the two).
 bool fx2_usable(const rism3d_ctx *c) {
@@ -1803,12 +1826,13 @@ void fwd3d(rism3d_ctx *c, const double *A) {
   k_xfwd<double, MODE_FWD><<<gx, 256, xsmem<double>(c), c->stream>>>(G, c->plan<double>(0), t.RX, A, A, 1.0,
                                                                      c->pd.closure, W, postw<double>(c));
   CKL();
-  dim3 gy((G.Nh + t.BY - 1) / t.BY, G.N2, c->m);
-  const size_t sy = ysmem<double>(c);
-  if (t.BY == 16) k_y<double, false, 16><<<gy, 256, sy, c->stream>>>(G, c->plan<double>(1), W);
-  else if (t.BY == 8) k_y<double, false, 8><<<gy, 256, sy, c->stream>>>(G, c->plan<double>(1), W);
-  else k_y<double, false, 4><<<gy, 256, sy, c->stream>>>(G, c->plan<double>(1), W);
-  CKL();
+  c->timer.launches[TK_XFWD]++;
+  launch_y<double, false>(c);
+  c->timer.launches[TK_Z]++;
+  if (c->xy[0]) {
+    launch_zaxis(c, false);
+    return;
+  }
   dim3 gz((G.Nh + t.BZ - 1) / t.BZ, G.N1);
   const size_t sz = zsmem<double>(c);
   const ZParams<double> zp = zparams<double>(c, false);
@@ -1816,7 +1840,6 @@ void fwd3d(rism3d_ctx *c, const double *A) {
   else if (t.BZ == 8) k_z<double, MODE_FWD, 8><<<gz, 256, sz, c->stream>>>(G, c->plan<double>(2), W, zp);
   else k_z<double, MODE_FWD, 4><<<gz, 256, sz, c->stream>>>(G, c->plan<double>(2), W, zp);
   CKL();
-  c->timer.launches[TK_XFWD] += 3;
 }
 
 // out = K v = (chi - 1) * v (the OZ convolution alone): the J.v passes with
@@ -2127,7 +2150,7 @@ void bind_solute(rism3d_ctx *c, int n, const rism3d_site *solute) {
 // column by column.  RISM3D_AUTOTUNE=0 keeps the register / occupancy rule.
 struct TuneVal {
   TileShape t[2];
-  bool stat[2];
+  bool stat[2], xy[2];
   int zb[2];
   bool zpers[2];
 };
@@ -2165,8 +2188,8 @@ template <typename T> void tune_precision(rism3d_ctx *c, const T *A, const T *Bv
   const size_t cs = sizeof(typename Cx<T>::type);
   const long long lim = optin_limit();
   const int reps = G.Nr >= (1LL << 22) ? 2 : 5;
-  const bool had_stat = c->stat[pr];
-  c->stat[pr] = false;
+  const bool had_stat = c->stat[pr], had_xy = c->xy[pr];
+  c->stat[pr] = c->xy[pr] = false;
   auto run = [&] { pipeline<T, MODE_J>(c, A, Bv, (T)1, (T)1, out, false); };
   const int cand[4] = {4, 8, 16, 32};
   // one axis at a time, the others held
@@ -2196,22 +2219,23 @@ template <typename T> void tune_precision(rism3d_ctx *c, const T *A, const T *Bv
     }
     *fields[axis] = best;
   }
-  if (had_stat) {
+  if (had_xy) {
     const float g_ms = time_ms(c, run, reps);
-    c->stat[pr] = true;
+    c->xy[pr] = true;
+    c->stat[pr] = had_stat;
     float s_ms = time_ms(c, run, reps);
     // the specialised z pass: wide tiles, or half as wide (twice the CTAs
     // in flight per SM)
     const int wide = c->zb[pr];
     float n_ms = 1e30f;
-    if (pr == 1 && z_has_variants(G.N2)) {  // FP32 only: 64-byte rows (FP64 would drop to 32-thread CTAs)
+    if (pr == 1 && had_stat && z_has_variants(G.N2)) {  // FP32 only: 64-byte rows (FP64 would drop to 32-thread CTAs)
       c->zb[pr] = wide / 2;
       make_tmap(c, &c->tmz[pr], pr == 0, c->zb[pr], 1, G.N2);
       n_ms = time_ms(c, run, reps);
     }
     if (n_ms < 0.95f * s_ms) {
       s_ms = n_ms;
-    } else if (z_has_variants(G.N2)) {
+    } else if (had_stat && z_has_variants(G.N2)) {
       c->zb[pr] = wide;
       make_tmap(c, &c->tmz[pr], pr == 0, wide, 1, G.N2);
       // persistent double-buffered CTAs for the wide tiles
@@ -2220,7 +2244,8 @@ template <typename T> void tune_precision(rism3d_ctx *c, const T *A, const T *Bv
       if (p_ms < 0.97f * s_ms) s_ms = p_ms;
       else c->zpers[pr] = false;
     }
-    c->stat[pr] = s_ms <= 1.05f * g_ms;  // keep the specialised passes unless clearly slower
+    c->xy[pr] = s_ms <= 1.05f * g_ms;  // keep the specialised passes unless clearly slower
+    c->stat[pr] = had_stat && c->xy[pr];
   }
 }
 
@@ -2254,6 +2279,7 @@ void autotune(rism3d_ctx *c) {
     if (it != g_tune.end()) {
       for (int pr = 0; pr < 2; ++pr) {
         c->tiles[pr] = it->second.t[pr];
+        c->xy[pr] = c->xy[pr] && it->second.xy[pr];
         c->stat[pr] = c->stat[pr] && it->second.stat[pr];
         c->zpers[pr] = c->stat[pr] && it->second.zpers[pr];
         if (c->stat[pr] && c->zb[pr] != it->second.zb[pr]) {
@@ -2283,6 +2309,7 @@ void autotune(rism3d_ctx *c) {
   for (int pr = 0; pr < 2; ++pr) {
     v.t[pr] = c->tiles[pr];
     v.stat[pr] = c->stat[pr];
+    v.xy[pr] = c->xy[pr];
     v.zb[pr] = c->zb[pr];
     v.zpers[pr] = c->zpers[pr];
   }
@@ -2405,6 +2432,52 @@ size_t generic_smem(rism3d_ctx *c) {
                    zsmem<float>(c)})
     need = std::max(need, b);
   return need;
+}
+
+// Selects the shape-specialised passes (TMA tiles) where all three lengths
+// have them: x and y for any fields, the z pass of a solute for up to three
+// sites and a radial chi (zs).  RISM3D_GENERIC_PASSES=1 keeps the
+// runtime-length passes everywhere.
+void specialise(rism3d_ctx *c, bool zs) {
+  const Geo &G = c->g;
+  const char *gen = std::getenv("RISM3D_GENERIC_PASSES");
+  if (!static_len_x(G.M) || !static_len_yz(G.N1) || !static_len_yz(G.N2) || (gen && gen[0] == '1')) return;
+  for (int pr = 0; pr < 2; ++pr) {
+    const int B = pr == 0 ? static_B<double>() : static_B<float>();
+    make_tmap(c, &c->tmy[pr], pr == 0, B, G.N1, 1);
+    if (zs) make_tmap(c, &c->tmz[pr], pr == 0, c->zb[pr], 1, G.N2);
+    c->xy[pr] = true;
+    c->stat[pr] = zs;
+  }
+  make_tmap(c, &c->tmza, true, static_B<double>(), 1, G.N2);
+  std::vector<PassKernel> ks;
+  switch (G.M) {
+#define ALLOW_X(M)                    \
+  case M:                             \
+    XPass<double, M>::kernels(ks);    \
+    XPass<float, M>::kernels(ks);     \
+    break;
+    RISM_X_LENS(ALLOW_X)
+#undef ALLOW_X
+  }
+#define ALLOW_Y(N)                    \
+  case N:                             \
+    YPass<double, N>::kernels(ks);    \
+    YPass<float, N>::kernels(ks);     \
+    break;
+  switch (G.N1) { RISM_YZ_LENS(ALLOW_Y) }
+#undef ALLOW_Y
+#define ALLOW_Z(N)                                \
+  case N:                                         \
+    ZAxis<N>::kernels(ks);                        \
+    if (zs) {                                     \
+      ZPass<double, N>::kernels(c->m, ks);        \
+      ZPass<float, N>::kernels(c->m, ks);         \
+    }                                             \
+    break;
+  switch (G.N2) { RISM_YZ_LENS(ALLOW_Z) }
+#undef ALLOW_Z
+  for (const PassKernel &k : ks) allow_smem(k.fn, k.smem);
 }
 
 // Opt-in for the runtime-length x and y passes (every context uses them).
@@ -2534,18 +2607,7 @@ int create_impl(const rism3d_problem *pd, int m, const rism3d_site *solvent, int
     c->L32 = dalloc<float2>((size_t)G.Nc);
     bind_solute(c, n, solute);
     init_work(c);
-    // shape-specialised passes (TMA tiles) for the lengths they are built for;
-    // RISM3D_GENERIC_PASSES=1 selects the runtime-length passes everywhere
-    const char *gen = std::getenv("RISM3D_GENERIC_PASSES");
-    if (static_len_x(G.M) && static_len_yz(G.N1) && static_len_yz(G.N2) && m <= 3 && !chi3 &&
-        !(gen && gen[0] == '1')) {
-      for (int pr = 0; pr < 2; ++pr) {
-        const int B = pr == 0 ? static_B<double>() : static_B<float>();
-        make_tmap(c, &c->tmy[pr], pr == 0, B, G.N1, 1);
-        make_tmap(c, &c->tmz[pr], pr == 0, c->zb[pr], 1, G.N2);
-        c->stat[pr] = true;
-      }
-    }
+    specialise(c, m <= 3 && !chi3);
     size_t need = generic_smem(c);
     allow_xy(need);
     auto allow = [&](const void *fn) { allow_smem(fn, need); };
@@ -2562,33 +2624,6 @@ int create_impl(const rism3d_problem *pd, int m, const rism3d_site *solvent, int
     OPTIN_Z(double)
     OPTIN_Z(float)
 #undef OPTIN_Z
-    if (c->stat[0]) {
-      std::vector<PassKernel> ks;
-      switch (G.M) {
-#define ALLOW_X(M)                      \
-  case M:                               \
-    XPass<double, M>::kernels(ks);      \
-    XPass<float, M>::kernels(ks);       \
-    break;
-        RISM_X_LENS(ALLOW_X)
-#undef ALLOW_X
-      }
-#define ALLOW_Y(N)                      \
-  case N:                               \
-    YPass<double, N>::kernels(ks);      \
-    YPass<float, N>::kernels(ks);       \
-    break;
-      switch (G.N1) { RISM_YZ_LENS(ALLOW_Y) }
-#undef ALLOW_Y
-#define ALLOW_Z(N)                      \
-  case N:                               \
-    ZPass<double, N>::kernels(m, ks);   \
-    ZPass<float, N>::kernels(m, ks);    \
-    break;
-      switch (G.N2) { RISM_YZ_LENS(ALLOW_Z) }
-#undef ALLOW_Z
-      for (const PassKernel &k : ks) allow_smem(k.fn, k.smem);
-    }
     autotune(c);
     // two-grid preconditioner: a copy of the problem on a coarse grid.  The
     // spacing coarse_h is taken when its grid has at most half the fine
@@ -2726,6 +2761,7 @@ int solvent_create_impl(const rism3d_problem *pd, int ms, const rism3d_site *sol
     c->ck = dalloc<double2>((size_t)np * G.Nc);
     CK(cudaMemsetAsync(c->ck, 0, sizeof(double2) * (size_t)np * G.Nc, c->stream));
     init_work(c);
+    specialise(c, false);
     const size_t need = generic_smem(c);
     allow_xy(need);
     allow_smem((const void *)k_z<double, MODE_FWD, 16>, need);

@@ -101,62 +101,26 @@ __device__ __forceinline__ void lu_solve(const double2 (&A)[MS][MS], const int (
 
 __device__ __forceinline__ double sinc(double x) { return x == 0.0 ? 1.0 : sin(x) / x; }
 
-// z pass of the pure solvent: forward z transform of the NP pair fields of a
-// tile, the per-k OZ solve (MODE_F) or its differential (MODE_J), inverse z
-// transform.  MODE_VL ignores the input and writes the long-range term
-// -beta q2 v_L(k) / h^3 (centred) for the inverse transform.  Output in the
-// units the x-inverse pass expects: t_centre(k) / h^3.
-template <int MODE, int B, int MS>
-__global__ void __launch_bounds__(256) k_z_oz(Geo g, AxisPlan pz, double2 *__restrict__ W, PureParams<MS> pp) {
+// The OZ step at one k point: q[pair], the transformed pair fields at the grid's
+// centre, becomes t_centre(k) / h^3 (MODE_F, which also writes C(k)), its
+// differential (MODE_J) or the long-range term -beta q2 v_L(k) / h^3 (MODE_VL,
+// which ignores q).
+template <int MODE, int MS>
+__device__ __forceinline__ void oz_point(const Geo &g, const PureParams<MS> &pp, int kx, int ky, int kz, long long o,
+                                         double2 (&q)[MS * (MS + 1) / 2]) {
   using V = double2;
   constexpr int NP = MS * (MS + 1) / 2;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  V *tw = reinterpret_cast<V *>(smem_raw);
-  V *buf = tw + pz.n;
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const int kx0 = blockIdx.x * B;
-  const int y = blockIdx.y;
-  const int bw = min(B, g.Nh - kx0);
-  const int N2 = g.N2;
-  const V *twg = reinterpret_cast<const V *>(pz.tw);
-  for (int q = tid; q < pz.n; q += nthr) tw[q] = twg[q];
-  const long long zstride = (long long)g.N1 * g.Nhp;
-  const long long col = (long long)y * g.Nhp + kx0;
-  constexpr int mB = NP * B;
-  if (MODE != MODE_VL) {
-    for (int e = tid; e < N2 * mB; e += nthr) {
-      const int z = e / mB, r = e - z * mB;
-      const int s = r / B, b = r - s * B;
-      V v = make_double2(0.0, 0.0);
-      if (b < bw) v = W[(long long)s * g.Nc + z * zstride + col + b];
-      buf[e] = v;
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int s = 0; s < NP; ++s) fft_tile<false, true>(buf + s * B, pz, B, mB, 1, tw);
-  } else {
-    __syncthreads();
-  }
-  const int ky = kfreq(y, g.N1);
-  const double k1 = ky * g.dk1;
   const double h3 = pp.h3, rho = pp.rho, beta = pp.beta;
-  for (int e = tid; e < N2 * B; e += nthr) {
-    const int z = e / B, b = e - z * B;
-    if (b >= bw) continue;
-    const int kx = kx0 + b;
-    const int kz = kfreq(z, N2);
-    const double k0 = kx * g.dk0, k2 = kz * g.dk2;
-    const double kk = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(k0, k0), __dmul_rn(k1, k1)), __dmul_rn(k2, k2)));
-    const double kq = kk * kk;
-    // coulomb_long_fourier(k, 1, G) (bgy3d-force.h:139-148)
-    const double clf = kq == 0.0 ? 0.0 : (4 * M_PI * kEps0Inv) * exp(-kq / (4 * kG * kG)) / kq;
-    const double sg = ((kx + ky + kz) & 1) ? -1.0 : 1.0;  // centre <-> corner
-    const long long o = z * zstride + col + b;
-    if (MODE == MODE_VL) {
+  const double k0 = kx * g.dk0, k1 = ky * g.dk1, k2 = kz * g.dk2;
+  const double kk = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(k0, k0), __dmul_rn(k1, k1)), __dmul_rn(k2, k2)));
+  const double kq = kk * kk;
+  // coulomb_long_fourier(k, 1, G) (bgy3d-force.h:139-148)
+  const double clf = kq == 0.0 ? 0.0 : (4 * M_PI * kEps0Inv) * exp(-kq / (4 * kG * kG)) / kq;
+  const double sg = ((kx + ky + kz) & 1) ? -1.0 : 1.0;  // centre <-> corner
+  if constexpr (MODE == MODE_VL) {
 #pragma unroll
-      for (int p = 0; p < NP; ++p) buf[(z * NP + p) * B + b] = make_double2(-beta * pp.q2[p] * clf * sg / h3, 0.0);
-      continue;
-    }
+    for (int p = 0; p < NP; ++p) q[p] = make_double2(-beta * pp.q2[p] * clf * sg / h3, 0.0);
+  } else {
     const double sqn = sqrt((double)(kx * kx + ky * ky + kz * kz));
     double Wm[MS][MS];
     V C[MS][MS], A[MS][MS], X[MS][MS], D[MS][MS];
@@ -166,7 +130,7 @@ __global__ void __launch_bounds__(256) k_z_oz(Geo g, AxisPlan pz, double2 *__res
       for (int j = 0; j <= i; ++j) {
         const int p = i * (i + 1) / 2 + j;
         Wm[i][j] = Wm[j][i] = (i == j) ? 1.0 : sinc(pp.wr[p] * sqn);
-        const V in = buf[(z * NP + p) * B + b];
+        const V in = q[p];
         if (MODE == MODE_F) {
           // C = [FFT(c) h^3 - beta v_L] at the corner (hnc3d.c:382-405)
           const V cc = make_double2(in.x * h3 * sg - beta * pp.q2[p] * clf, in.y * h3 * sg);
@@ -209,7 +173,7 @@ __global__ void __launch_bounds__(256) k_z_oz(Geo g, AxisPlan pz, double2 *__res
           const int p = i * (i + 1) / 2 + j;
           // back to the centre, long range out (hnc3d.c:411-437)
           const double tr = R[i][j].x - C[i][j].x - beta * pp.q2[p] * clf, ti = R[i][j].y - C[i][j].y;
-          buf[(z * NP + p) * B + b] = make_double2(tr * sg / h3, ti * sg / h3);
+          q[p] = make_double2(tr * sg / h3, ti * sg / h3);
         }
     } else {
       // Q = W + rho X (into X), Y = W dC Q (into A's row buffer via R2)
@@ -243,9 +207,58 @@ __global__ void __launch_bounds__(256) k_z_oz(Geo g, AxisPlan pz, double2 *__res
         for (int j = 0; j <= i; ++j) {
           const int p = i * (i + 1) / 2 + j;
           const double tr = R[i][j].x - D[i][j].x, ti = R[i][j].y - D[i][j].y;
-          buf[(z * NP + p) * B + b] = make_double2(tr * sg / h3, ti * sg / h3);
+          q[p] = make_double2(tr * sg / h3, ti * sg / h3);
         }
     }
+  }
+}
+
+// z pass of the pure solvent: forward z transform of the NP pair fields of a
+// tile, the per-k OZ solve (MODE_F) or its differential (MODE_J), inverse z
+// transform.  MODE_VL ignores the input and writes the long-range term
+// -beta q2 v_L(k) / h^3 (centred) for the inverse transform.  Output in the
+// units the x-inverse pass expects: t_centre(k) / h^3.
+template <int MODE, int B, int MS>
+__global__ void __launch_bounds__(256) k_z_oz(Geo g, AxisPlan pz, double2 *__restrict__ W, PureParams<MS> pp) {
+  using V = double2;
+  constexpr int NP = MS * (MS + 1) / 2;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  V *tw = reinterpret_cast<V *>(smem_raw);
+  V *buf = tw + pz.n;
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int kx0 = blockIdx.x * B;
+  const int y = blockIdx.y;
+  const int bw = min(B, g.Nh - kx0);
+  const int N2 = g.N2;
+  const V *twg = reinterpret_cast<const V *>(pz.tw);
+  for (int q = tid; q < pz.n; q += nthr) tw[q] = twg[q];
+  const long long zstride = (long long)g.N1 * g.Nhp;
+  const long long col = (long long)y * g.Nhp + kx0;
+  constexpr int mB = NP * B;
+  if (MODE != MODE_VL) {
+    for (int e = tid; e < N2 * mB; e += nthr) {
+      const int z = e / mB, r = e - z * mB;
+      const int s = r / B, b = r - s * B;
+      V v = make_double2(0.0, 0.0);
+      if (b < bw) v = W[(long long)s * g.Nc + z * zstride + col + b];
+      buf[e] = v;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int s = 0; s < NP; ++s) fft_tile<false, true>(buf + s * B, pz, B, mB, 1, tw);
+  } else {
+    __syncthreads();
+  }
+  const int ky = kfreq(y, g.N1);
+  for (int e = tid; e < N2 * B; e += nthr) {
+    const int z = e / B, b = e - z * B;
+    if (b >= bw) continue;
+    V q[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) q[p] = MODE == MODE_VL ? V{} : buf[(z * NP + p) * B + b];
+    oz_point<MODE, MS>(g, pp, kx0 + b, ky, kfreq(z, N2), z * zstride + col + b, q);
+#pragma unroll
+    for (int p = 0; p < NP; ++p) buf[(z * NP + p) * B + b] = q[p];
   }
   __syncthreads();
 #pragma unroll 1
@@ -255,6 +268,28 @@ __global__ void __launch_bounds__(256) k_z_oz(Geo g, AxisPlan pz, double2 *__res
     const int s = r / B, b = r - s * B;
     if (b < bw) W[(long long)s * g.Nc + z * zstride + col + b] = buf[e];
   }
+}
+
+// The OZ step alone, on the k grid in place, between the shape-specialised z
+// transforms (one thread per point).  A z pass that keeps its NP tiles in
+// shared memory around the step, as the solute's does, has few threads per SM
+// (NP = 6 FP64 tiles) for a step that wants them: 3 x 3 complex factorisations
+// with their divisions, a sine per bond.  With the specialised x and y passes beside
+// it a 96^3 water solve went from 135 to 98 ms.
+template <int MODE, int MS> __global__ void __launch_bounds__(128) k_oz(Geo g, double2 *__restrict__ W, PureParams<MS> pp) {
+  constexpr int NP = MS * (MS + 1) / 2;
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int kx = (int)(e % g.Nh);
+  const long long r = e / g.Nh;
+  const int y = (int)(r % g.N1), z = (int)(r / g.N1);
+  if (z >= g.N2) return;
+  const long long o = ((long long)z * g.N1 + y) * g.Nhp + kx;
+  double2 q[NP];
+#pragma unroll
+  for (int p = 0; p < NP; ++p) q[p] = MODE == MODE_VL ? double2{} : W[p * g.Nc + o];
+  oz_point<MODE, MS>(g, pp, kx, kfreq(y, g.N1), kfreq(z, g.N2), o, q);
+#pragma unroll
+  for (int p = 0; p < NP; ++p) W[p * g.Nc + o] = q[p];
 }
 
 // Site-site short-range potentials on the centred grid (bgy3d_pair_potential,
