@@ -106,8 +106,32 @@ static __global__ void k_grad_weights(Geo g, const double *__restrict__ t, const
   B[p] = rhoh3 * bsum;
 }
 
+// The short- and long-range Coulomb functions and their derivatives over x at
+// one x: cscap0, cscap1s, cl0, cl1s from one erfc and one exponential.  From
+// x = 1 on (every point but those within 0.83 A of the site) erf is 1 - erfc,
+// whose error is then a fifth of erfc's own.
+__device__ __forceinline__ void coulomb_pair(double x, double &s0, double &s1, double &l0, double &l1) {
+  if (x < 1.0) {
+    s0 = cscap0(x);
+    s1 = cscap1s(x);
+    l0 = cl0(x);
+    l1 = cl1s(x);
+    return;
+  }
+  const double ix = 1.0 / x, ix2 = ix * ix, ec = erfc(x), er = 1.0 - ec;
+  const double ge = (2 / sqrt(M_PI)) * x * exp(-x * x);
+  s0 = ec * ix;
+  s1 = -(ec + ge) * ix2 * ix;
+  l0 = er * ix;
+  l1 = (ge - er) * ix2 * ix;
+}
+
 // Real-space sums for solute site u = blockIdx.y over this block's grid
 // points: part[(u * gridDim.x + blockIdx.x) * 6 + {q, sigma, eps, x, y, z}].
+// FP64 arithmetic bounds it (n error functions per point): the Coulomb terms
+// are evaluated once per point and solute site, not per solvent site too, the
+// pair constants sit in shared memory and (sigma / r)^6 takes no division.
+// 128^3, 12 solute and 3 solvent sites: 2.98 -> 0.70 ms.
 static __global__ void __launch_bounds__(256) k_grad_real(Geo g, double h0, double h1, double h2, double L0,
                                                           double L1, double L2, const SiteP *__restrict__ solvent,
                                                           const SiteP *__restrict__ solute,
@@ -115,29 +139,54 @@ static __global__ void __launch_bounds__(256) k_grad_real(Geo g, double h0, doub
                                                           double *__restrict__ part) {
   const int u = blockIdx.y;
   const SiteP su = solute[u];
+  // per solvent site: eps_iu, sigma_iu^2, the LJ cap's r^2, the derivative
+  // factors of sigma_u and eps_u, the Coulomb prefactor
+  __shared__ double ce[kMaxSites], cs2[kMaxSites], cr2[kMaxSites], csg[kMaxSites], cde[kMaxSites], cq[kMaxSites];
+  if (threadIdx.x < g.m) {
+    const SiteP a = solvent[threadIdx.x];
+    const double eab = sqrt(a.epsilon * su.epsilon), sab = 0.5 * (a.sigma + su.sigma);
+    ce[threadIdx.x] = eab;
+    cs2[threadIdx.x] = sab * sab;
+    cr2[threadIdx.x] = 0.2 * sab * (0.2 * sab);
+    csg[threadIdx.x] = -0.5 * eab / sab;
+    cde[threadIdx.x] = eab > 0 ? a.epsilon / (2 * eab) : 0.0;
+    cq[threadIdx.x] = a.charge * kEps0Inv;
+  }
+  __syncthreads();
+  const double uq = kG * kG * kG * su.charge;
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < g.Nr;
-       p += (long long)gridDim.x * blockDim.x) {
-    const int i0 = (int)(p % g.N0);
-    const int i1 = (int)((p / g.N0) % g.N1);
-    const int i2 = (int)(p / ((long long)g.N0 * g.N1));
+  for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < (unsigned)g.Nr; p += gridDim.x * blockDim.x) {
+    const unsigned row = p / (unsigned)g.N0;
+    const int i0 = (int)(p - row * g.N0);
+    const int i2 = (int)(row / (unsigned)g.N1), i1 = (int)(row - (unsigned)i2 * g.N1);
     const double dx = i0 * h0 - L0 / 2 - su.x, dy = i1 * h1 - L1 / 2 - su.y, dz = i2 * h2 - L2 / 2 - su.z;
-    const double r = sqrt(dx * dx + dy * dy + dz * dz);
+    const double r2 = dx * dx + dy * dy + dz * dz, r = sqrt(r2), ir2 = 1.0 / r2;
+    double s0, s1, l0, l1;
+    coulomb_pair(kG * r, s0, s1, l0, l1);
+    const double csr = kG * s0, csd = uq * s1;
     double gr = 0.0;  // (1/r) d/dr of sum_i A_i v_iu
     for (int s = 0; s < g.m; ++s) {
-      const SiteP a = solvent[s];
       const double w = A[(long long)s * g.Nr + p];
-      const double eab = sqrt(a.epsilon * su.epsilon), sab = 0.5 * (a.sigma + su.sigma);
-      const double sv = r / sab;
-      const double qq = a.charge * kEps0Inv;  // times q_u: short-range Coulomb prefactor
-      acc[0] += w * qq * kG * cscap0(kG * r);
-      acc[1] += w * eab * ljcap1(sv) * (-sv / sab) * 0.5;
-      if (eab > 0) acc[2] += w * (a.epsilon / (2 * eab)) * ljcap0(sv);
-      gr += w * (eab * ljcap1s(sv) / (sab * sab) + qq * su.charge * kG * kG * kG * cscap1s(kG * r));
+      acc[0] += w * cq[s] * csr;
+      double e0, d1;  // LJ value / eps, and s d/ds of it
+      if (r2 >= cr2[s]) {
+        const double i2 = cs2[s] * ir2, p6 = i2 * i2 * i2;
+        e0 = 4 * p6 * (p6 - 1);
+        d1 = 4 * p6 * (6 - 12 * p6);
+        gr += w * ce[s] * d1 * ir2;
+      } else {
+        const double sv = r / sqrt(cs2[s]);
+        e0 = ljcap0(sv);
+        d1 = ljcap1(sv) * sv;
+        gr += w * ce[s] * ljcap1s(sv) / cs2[s];
+      }
+      acc[1] += w * csg[s] * d1;
+      acc[2] += w * cde[s] * e0;
+      gr += w * cq[s] * csd;
     }
     const double bw = B[p];
-    acc[0] += bw * kEps0Inv * kG * cl0(kG * r);
-    gr += bw * kEps0Inv * su.charge * kG * kG * kG * cl1s(kG * r);
+    acc[0] += bw * kEps0Inv * kG * l0;
+    gr += bw * kEps0Inv * uq * l1;
     // d/dR_u = -(r - R_u) / r d/dr
     acc[3] -= gr * dx;
     acc[4] -= gr * dy;
