@@ -13,7 +13,9 @@
 // half-length complex FFT of the x passes plus the r2c untangle, and the
 // coarse side is a (K+1) x Nc table product.  Transforms run in FP32.
 #pragma once
-#include "fft_static.cuh"
+#include <type_traits>
+
+#include "kernels_static.cuh"
 
 namespace rism {
 
@@ -282,10 +284,6 @@ __global__ void __launch_bounds__(256) k_prolong_fx(long long rows, int Nc, int 
 #undef FX_LOAD
 }
 
-}  // namespace rism
-
-namespace rism {
-
 // ---- both sides by FFT: the coarse side as a packed row transform of
 // length Nc = 2 MC instead of the (K+1) x Nc table product (K = MC).
 //
@@ -296,237 +294,271 @@ namespace rism {
 // Prolongation: X_k = f_k r2c_Nc(y)_k from the MC-point forward FFT of the
 // coarse row and its untangle, then the fine packed c2r as before.
 // twc / postc: the twiddles of the MC-point transform and exp(-2 pi i k / Nc),
-// k in [0, MC] (the coarse grid's own x tables).  The coarse row tile
-// aliases the fine one (it is only live while the fine one is not).
-template <int M, int MC, int RX> __host__ __device__ constexpr int fx2_words() {
-  return M + fx_buf<M, RX>() + RX * (MC + 1) + MC;
+// k in [0, MC] (the coarse grid's own x tables).
+//
+// Bound by latency (a chain of barriers over 10 KB of rows), so as the x
+// passes: small CTAs of one batch each, a thread's loads all in flight, both
+// transforms in the order of their two steps (perm_pos), the untangling of one
+// side and the packing of the other in one step between the two tiles, and the
+// last step's outputs from its registers: five CTA barriers instead of twelve.
+// us, persistent CTAs of 256 threads with whole transforms -> here: 162 -> 54
+// points FP32, restriction 62 -> 34, prolongation 79 -> 63; 128 -> 48 FP64 37 ->
+// 19 and 57 -> 27.
+constexpr int kFx2Threads = 128;
+template <int M, int MC, int RX> __host__ __device__ constexpr size_t fx2_smem() {
+  return sizeof(float2) * (size_t)(M + MC + RX * (LayRow<M, SplitRow<M>::R2>::RS + LayRow<MC, SplitRow<MC>::R2>::RS));
 }
-template <int M, int MC, int RX> inline size_t fx2_smem() { return sizeof(float2) * (size_t)fx2_words<M, MC, RX>(); }
 
-// z-pack of a Hermitian half spectrum X_0..X_K (row stride K1) for the packed
-// c2r of length 2 MM (K >= MM: only X_0..X_MM are read; K < MM: zero above
-// K).  Writes the MM packed values of every row into buf (layout L).
-template <int MM, int RX, class L>
-__device__ __forceinline__ void fx_pack_c2r(const float2 *X, int K, int K1, const float2 *post, float2 *buf) {
-  constexpr int H = MM / 2 + 1;
-  for (int e = threadIdx.x; e < RX * H; e += 256) {
-    const int row = e / H, k = e - row * H;
-    float2 xk = make_float2(0.f, 0.f), xm = make_float2(0.f, 0.f);
-    if (k <= K) xk = X[row * K1 + k];
-    if (MM - k <= K) xm = X[row * K1 + (MM - k)];
-    if (k == 0) { xk.y = 0.f; xm.y = 0.f; }
-    float2 Aa, Dd;
-    Aa.x = xk.x + xm.x; Aa.y = xk.y - xm.y;
-    Dd.x = xk.x - xm.x; Dd.y = xk.y + xm.y;
-    const float2 Pp = cmul(Dd, cconj(post[k]));
-    float2 zk, zm;
-    zk.x = Aa.x - Pp.y; zk.y = Aa.y + Pp.x;
-    zm.x = Aa.x + Pp.y; zm.y = -(Aa.y - Pp.x);
-    buf[L::at(k, row)] = zk;
-    if (k != 0 && MM - k != k) buf[L::at(MM - k, row)] = zm;
+// The two steps of a forward transform of RX rows in place, spectrum in
+// permuted order; ends synchronised.
+template <int M, int RX, class S, class Lay> __device__ __forceinline__ void fx2_fwd(float2 *buf, const float2 *tw) {
+#pragma unroll
+  for (int q = threadIdx.x; q < RX * S::R2; q += kFx2Threads) {
+    const int row = q / S::R2, n2 = q % S::R2;
+    float2 u[S::R1];
+#pragma unroll
+    for (int n1 = 0; n1 < S::R1; ++n1) u[n1] = buf[Lay::at(S::R2 * n1 + n2, row)];
+    fwd_step1<S>(u, n2, tw);
+#pragma unroll
+    for (int k1 = 0; k1 < S::R1; ++k1) buf[Lay::at(S::R2 * k1 + n2, row)] = u[k1];
   }
+  __syncthreads();
+#pragma unroll
+  for (int q = threadIdx.x; q < RX * S::R1; q += kFx2Threads) {
+    const int row = q / S::R1, k1 = q % S::R1;
+    float2 u[S::R2];
+#pragma unroll
+    for (int n2 = 0; n2 < S::R2; ++n2) u[n2] = buf[Lay::at(S::R2 * k1 + n2, row)];
+    fwd_step2<S>(u, tw);
+#pragma unroll
+    for (int k2 = 0; k2 < S::R2; ++k2) buf[Lay::at(S::R2 * k1 + k2, row)] = u[k2];
+  }
+  __syncthreads();
+}
+// The first step of the inverse transform in place; ends synchronised.
+template <int M, int RX, class S, class Lay> __device__ __forceinline__ void fx2_inv1(float2 *buf, const float2 *tw) {
+#pragma unroll
+  for (int q = threadIdx.x; q < RX * S::R1; q += kFx2Threads) {
+    const int row = q / S::R1, k1 = q % S::R1;
+    float2 u[S::R2];
+#pragma unroll
+    for (int k2 = 0; k2 < S::R2; ++k2) u[k2] = buf[Lay::at(S::R2 * k1 + k2, row)];
+    inv_step1<S>(u, k1, tw);
+#pragma unroll
+    for (int n2 = 0; n2 < S::R2; ++n2) buf[Lay::at(S::R2 * k1 + n2, row)] = u[n2];
+  }
+  __syncthreads();
 }
 
-// 128-point half rows at 3 CTAs per SM (80 registers, no spills; the
-// unbounded choice of 128 allows 2): the batches are latency chains, so
-// resident CTAs set the throughput.
+// X_k of the row transform of length 2 M from its packed transform (k <= M),
+// and the packed pair (Z_k, Z_{M-k}) of the inverse from (X_k, X_{M-k}).
+template <int M, class S, class Lay>
+__device__ __forceinline__ float2 fx2_untangle(const float2 *buf, int row, int k, const float2 *post) {
+  const float2 zk = buf[Lay::at(perm_pos<S>(k == M ? 0 : k), row)];
+  const float2 zm = buf[Lay::at(perm_pos<S>(k == 0 || k == M ? 0 : M - k), row)];
+  const float2 E = make_float2((zk.x + zm.x) * 0.5f, (zk.y - zm.y) * 0.5f);
+  const float2 O = make_float2((zk.y + zm.y) * 0.5f, -(zk.x - zm.x) * 0.5f);
+  return cadd(E, cmul(post[k], O));
+}
+template <int M, class S, class Lay>
+__device__ __forceinline__ void fx2_pack(float2 *buf, int row, int k, float2 xk, float2 xm, const float2 *post) {
+  if (k == 0) { xk.y = 0.f; xm.y = 0.f; }
+  const float2 Aa = make_float2(xk.x + xm.x, xk.y - xm.y), Dd = make_float2(xk.x - xm.x, xk.y + xm.y);
+  const float2 Pp = cmul(Dd, cconj(post[k]));
+  buf[Lay::at(perm_pos<S>(k), row)] = make_float2(Aa.x - Pp.y, Aa.y + Pp.x);
+  if (k != 0 && M - k != k) buf[Lay::at(perm_pos<S>(M - k), row)] = make_float2(Aa.x + Pp.y, -(Aa.y - Pp.x));
+}
+
 template <typename TI, int M, int MC, int RX>
-__global__ void __launch_bounds__(256, M == 128 ? 3 : 1) k_restrict_fx2(long long rows, const TI *__restrict__ in, float s,
-                                                      const float2 *__restrict__ post, const float2 *__restrict__ twg,
-                                                      const float2 *__restrict__ postc,
-                                                      const float2 *__restrict__ twcg, float *__restrict__ out) {
-  using V = float2;
-  using Lay = LayRow<M, SplitRow<M>::R2>;
-  using LayC = LayRow<MC, SplitRow<MC>::R2>;
-  using Q = typename Quad<TI>::type;
-  static_assert(MC < M && fx_buf<MC, RX>() <= fx_buf<M, RX>(), "coarse row tile must fit the fine one");
-  constexpr int N0 = 2 * M, Nc = 2 * MC, K = MC, K1 = MC + 1;
-  // a batch of rows is one run of memory: RX M / 2 pairs of complex values,
-  // whose rows may end inside a pair (odd M), and RX MC / 2 output float4
-  static_assert(RX % 2 == 0, "a batch holds whole pairs");
-  constexpr int NQ = RX * M / 2, CNT = (NQ + 255) / 256;
-  constexpr int NC = RX * MC / 2;
+__global__ void __launch_bounds__(kFx2Threads) k_restrict_fx2(long long rows, const TI *__restrict__ in, float s,
+                                                              const float2 *__restrict__ post, const float2 *__restrict__ twg,
+                                                              const float2 *__restrict__ postc,
+                                                              const float2 *__restrict__ twcg, float *__restrict__ out) {
+  using S = SplitRow<M>;
+  using SC = SplitRow<MC>;
+  using Lay = LayRow<M, S::R2>;
+  using LayC = LayRow<MC, SC::R2>;
+  using VEC = typename VecW<TI, M>::vec;
+  static_assert(MC < M, "the coarse row is the shorter one");
+  constexpr int THR = kFx2Threads, VW = VecW<TI, M>::n, PER_ROW = M / VW, CNT = (RX * PER_ROW + THR - 1) / THR;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  V *tw = reinterpret_cast<V *>(smem_raw);
-  V *buf = tw + M;
-  V *X = buf + fx_buf<M, RX>();
-  V *twc = X + RX * K1;
+  float2 *tw = reinterpret_cast<float2 *>(smem_raw);
+  float2 *twc = tw + M;
+  float2 *buf = twc + MC;
+  float2 *bc = buf + RX * Lay::RS;
   const int tid = threadIdx.x;
-  const long long nbat = (rows + RX - 1) / RX;
-  const float inv_n0 = 1.0f / (float)N0;
-  long long bat = blockIdx.x;
-  Q ra[CNT];
-#define FX2_LOAD_ROWS(BAT)                                                                          \
-  {                                                                                                 \
-    const long long r0 = (BAT) * RX;                                                                \
-    _Pragma("unroll") for (int it = 0; it < CNT; ++it) {                                            \
-      const int e = tid + it * 256;                                                                 \
-      if (e < NQ && e < (rows - r0) * M / 2) ra[it] = *reinterpret_cast<const Q *>(in + r0 * N0 + 4 * e); \
-    }                                                                                               \
-  }
-  if (bat < nbat) FX2_LOAD_ROWS(bat)
-  for (int q = tid; q < M; q += 256) tw[q] = twg[q];
-  for (int q = tid; q < MC; q += 256) twc[q] = twcg[q];
-  for (; bat < nbat; bat += gridDim.x) {
-    const long long row0 = bat * RX;
+  const long long row0 = (long long)blockIdx.x * RX;
+  VEC ra[CNT];
 #pragma unroll
-    for (int it = 0; it < CNT; ++it) {
-      const int e = tid + it * 256;
-      if (e >= NQ) break;
-      V a = make_float2(0.f, 0.f), b = a;
-      if (e < (rows - row0) * M / 2) {
-        Quad<TI>::split(ra[it], a, b);
-        a.x *= s; a.y *= s; b.x *= s; b.y *= s;
-      }
-      buf[Lay::at((2 * e) % M, (2 * e) / M)] = a;
-      buf[Lay::at((2 * e + 1) % M, (2 * e + 1) / M)] = b;
-    }
-    if (bat + gridDim.x < nbat) FX2_LOAD_ROWS(bat + gridDim.x)
-    __syncthreads();
-    fft2<M, RX, 256, false, false, Lay, SplitRow<M>>(buf, tw);
-    for (int e = tid; e < RX * K1; e += 256) {
-      const int row = e / K1, k = e - row * K1;
-      const V zk = buf[Lay::at(k, row)];
-      const V zm = buf[Lay::at(k == 0 ? 0 : M - k, row)];
-      V E, O;
-      E.x = (zk.x + zm.x) * 0.5f;
-      E.y = (zk.y - zm.y) * 0.5f;
-      O.x = (zk.y + zm.y) * 0.5f;
-      O.y = -(zk.x - zm.x) * 0.5f;
-      X[row * K1 + k] = cadd(E, cmul(post[k], O));
-    }
-    __syncthreads();
-    fx_pack_c2r<MC, RX, LayC>(X, K, K1, postc, buf);
-    __syncthreads();
-    fft2<MC, RX, 256, true, false, LayC, SplitRow<MC>>(buf, twc);
-    for (int e = tid; e < NC; e += 256) {
-      if (e >= (rows - row0) * MC / 2) break;
-      const V za = buf[LayC::at((2 * e) % MC, (2 * e) / MC)], zb = buf[LayC::at((2 * e + 1) % MC, (2 * e + 1) / MC)];
-      *reinterpret_cast<float4 *>(out + row0 * Nc + 4 * e) =
-          make_float4(za.x * inv_n0, za.y * inv_n0, zb.x * inv_n0, zb.y * inv_n0);
-    }
-    __syncthreads();
+  for (int it = 0; it < CNT; ++it) {
+    const int e = tid + it * THR;
+    if (e < RX * PER_ROW && row0 + e / PER_ROW < rows)
+      ra[it] = *reinterpret_cast<const VEC *>(in + (row0 + e / PER_ROW) * (2 * M) + 2 * VW * (e % PER_ROW));
   }
-#undef FX2_LOAD_ROWS
+  for (int q = tid; q < M; q += THR) tw[q] = twg[q];
+  for (int q = tid; q < MC; q += THR) twc[q] = twcg[q];
+#pragma unroll
+  for (int it = 0; it < CNT; ++it) {
+    const int e = tid + it * THR;
+    if (e >= RX * PER_ROW) break;
+    const int row = e / PER_ROW, jj = (e % PER_ROW) * VW;
+    const TI *v = reinterpret_cast<const TI *>(&ra[it]);
+    const bool in_range = row0 + row < rows;
+#pragma unroll
+    for (int w = 0; w < VW; ++w)
+      buf[Lay::at(jj + w, row)] =
+          in_range ? make_float2((float)v[2 * w] * s, (float)v[2 * w + 1] * s) : make_float2(0.f, 0.f);
+  }
+  __syncthreads();
+  fx2_fwd<M, RX, S, Lay>(buf, tw);
+  constexpr int H = MC / 2 + 1;
+#pragma unroll 2
+  for (int e = tid; e < RX * H; e += THR) {
+    const int row = e / H, k = e % H;
+    fx2_pack<MC, SC, LayC>(bc, row, k, fx2_untangle<M, S, Lay>(buf, row, k, post),
+                           fx2_untangle<M, S, Lay>(buf, row, MC - k, post), postc);
+  }
+  __syncthreads();
+  fx2_inv1<MC, RX, SC, LayC>(bc, twc);
+  const float inv_n0 = 1.0f / (float)(2 * M);
+#pragma unroll
+  for (int q = tid; q < RX * SC::R2; q += THR) {
+    const int row = q / SC::R2, n2 = q % SC::R2;
+    float2 u[SC::R1];
+#pragma unroll
+    for (int k1 = 0; k1 < SC::R1; ++k1) u[k1] = bc[LayC::at(SC::R2 * k1 + n2, row)];
+    inv_step2<SC>(u, twc);
+    if (row0 + row >= rows) continue;
+    float2 *o = reinterpret_cast<float2 *>(out + (row0 + row) * (2 * MC)) + n2;
+#pragma unroll
+    for (int n1 = 0; n1 < SC::R1; ++n1) o[SC::R2 * n1] = make_float2(u[n1].x * inv_n0, u[n1].y * inv_n0);
+  }
 }
 
-// 128-point half rows (the 256^3 grid) at 3 CTAs per SM: at the compiler's
-// unbounded choice of 128 registers only 2 fit; the bound costs a few spilled
-// words there (more at 256-point rows, which keep the unbounded choice)
+// The subtracted term s r is taken in r's precision.  The last step's outputs
+// leave from its registers where its lanes cover whole sectors (R2 complex
+// values in a row), else through shared memory.
 template <typename TO, typename TR, int M, int MC, int RX>
-__global__ void __launch_bounds__(256, M == 128 ? (RX >= 32 ? 2 : 3) : 1) k_prolong_fx2(long long rows, const float *__restrict__ y,
-                                                     const float2 *__restrict__ post, const float2 *__restrict__ twg,
-                                                     const float2 *__restrict__ postc,
-                                                     const float2 *__restrict__ twcg, const TR *__restrict__ r,
-                                                     double s, TO *__restrict__ out) {
-  using V = float2;
-  using Lay = LayRow<M, SplitRow<M>::R2>;
-  using LayC = LayRow<MC, SplitRow<MC>::R2>;
-  using QR = typename Quad<TR>::type;
-  static_assert(MC < M && fx_buf<MC, RX>() <= fx_buf<M, RX>(), "coarse row tile must fit the fine one");
-  constexpr int N0 = 2 * M, Nc = 2 * MC, K = MC, K1 = MC + 1;
-  static_assert(RX % 2 == 0, "a batch holds whole pairs");
-  constexpr int NQ = RX * M / 2, CNT = (NQ + 255) / 256;  // pairs of complex values of a batch, as above
-  constexpr int YC = (RX * MC + 255) / 256;  // coarse pairs per thread
+__global__ void __launch_bounds__(kFx2Threads) k_prolong_fx2(long long rows, const float *__restrict__ y,
+                                                             const float2 *__restrict__ post, const float2 *__restrict__ twg,
+                                                             const float2 *__restrict__ postc,
+                                                             const float2 *__restrict__ twcg, const TR *__restrict__ r,
+                                                             double s, TO *__restrict__ out) {
+  using S = SplitRow<M>;
+  using SC = SplitRow<MC>;
+  using Lay = LayRow<M, S::R2>;
+  using LayC = LayRow<MC, SC::R2>;
+  static_assert(std::is_same<TO, TR>::value && MC < M, "one field type; the coarse row is the shorter one");
+  constexpr int THR = kFx2Threads;
+  constexpr bool direct = S::R2 * 2 * sizeof(TR) % 32 == 0;
+  constexpr int VW = direct ? 1 : VecW<TR, M>::n;
+  using C2 = typename Cx<TR>::type;
+  using VEC = std::conditional_t<direct, C2, typename VecW<TR, M>::vec>;
+  constexpr int PER_ROW = M / VW;
+  constexpr int ITEMS = (RX * S::R2 + THR - 1) / THR;
+  constexpr int CNT = direct ? ITEMS * S::R1 : (RX * PER_ROW + THR - 1) / THR;
+  constexpr int YC = (RX * MC + THR - 1) / THR;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  V *tw = reinterpret_cast<V *>(smem_raw);
-  V *buf = tw + M;
-  V *X = buf + fx_buf<M, RX>();
-  V *twc = X + RX * K1;
+  float2 *tw = reinterpret_cast<float2 *>(smem_raw);
+  float2 *twc = tw + M;
+  float2 *buf = twc + MC;
+  float2 *bc = buf + RX * Lay::RS;
   const int tid = threadIdx.x;
-  const long long nbat = (rows + RX - 1) / RX;
-  const float fk = 1.0f / (float)Nc;
-  long long bat = blockIdx.x;
-  QR rr[CNT], rn[CNT];
-  V yv[YC];
-#define FX2_LOAD(BAT, RR)                                                                           \
-  {                                                                                                 \
-    const long long r0 = (BAT) * RX;                                                                \
-    _Pragma("unroll") for (int it = 0; it < CNT; ++it) {                                            \
-      const int e = tid + it * 256;                                                                 \
-      if (e < NQ && e < (rows - r0) * M / 2) RR[it] = *reinterpret_cast<const QR *>(r + r0 * N0 + 4 * e); \
-    }                                                                                               \
-    _Pragma("unroll") for (int q = 0; q < YC; ++q) {                                                \
-      const int e = tid + q * 256;                                                                  \
-      yv[q] = (e < RX * MC && r0 + e / MC < rows) ? *reinterpret_cast<const float2 *>(y + r0 * Nc + 2 * e) \
-                                                 : make_float2(0.f, 0.f);                          \
-    }                                                                                               \
-  }
-  if (bat < nbat) FX2_LOAD(bat, rr)
-  for (int q = tid; q < M; q += 256) tw[q] = twg[q];
-  for (int q = tid; q < MC; q += 256) twc[q] = twcg[q];
-  for (; bat < nbat; bat += gridDim.x) {
-    const long long row0 = bat * RX;
+  const long long row0 = (long long)blockIdx.x * RX;
+  // element `it` of this thread: (row, complex index), or row < 0
+  auto where = [&](int it, int &row, int &jj) {
+    if (direct) {
+      const int q = tid + (it / S::R1) * THR;
+      row = q < RX * S::R2 ? q / S::R2 : -1;
+      jj = S::R2 * (it % S::R1) + q % S::R2;
+    } else {
+      const int e = tid + it * THR;
+      row = e < RX * PER_ROW ? e / PER_ROW : -1;
+      jj = (e % PER_ROW) * VW;
+    }
+    if (row0 + row >= rows) row = -1;
+  };
+  float2 yv[YC];
 #pragma unroll
-    for (int q = 0; q < YC; ++q) {
-      const int e = tid + q * 256;
-      if (e < RX * MC) buf[LayC::at(e % MC, e / MC)] = yv[q];
+  for (int it = 0; it < YC; ++it) {
+    const int e = tid + it * THR;
+    yv[it] = e < RX * MC && row0 + e / MC < rows ? *reinterpret_cast<const float2 *>(y + row0 * (2 * MC) + 2 * e)
+                                                 : make_float2(0.f, 0.f);
+  }
+  VEC rin[CNT];
+#pragma unroll
+  for (int it = 0; it < CNT; ++it) {
+    int row, jj;
+    where(it, row, jj);
+    if (row >= 0) rin[it] = *reinterpret_cast<const VEC *>(r + (row0 + row) * (2 * M) + 2 * jj);
+  }
+  for (int q = tid; q < M; q += THR) tw[q] = twg[q];
+  for (int q = tid; q < MC; q += THR) twc[q] = twcg[q];
+#pragma unroll
+  for (int it = 0; it < YC; ++it) {
+    const int e = tid + it * THR;
+    if (e < RX * MC) bc[LayC::at(e % MC, e / MC)] = yv[it];
+  }
+  __syncthreads();
+  fx2_fwd<MC, RX, SC, LayC>(bc, twc);
+  // untangle to the Nc-point r2c with weights f_k (1/Nc, half at the Nyquist
+  // K, real there), zero above K, and pack for the fine side
+  constexpr float fk = 1.0f / (float)(2 * MC);
+  auto spec = [&](int row, int k) {
+    if (k > MC) return make_float2(0.f, 0.f);
+    const float2 x = fx2_untangle<MC, SC, LayC>(bc, row, k, postc);
+    return k == MC ? make_float2(x.x * (0.5f * fk), 0.f) : make_float2(x.x * fk, x.y * fk);
+  };
+  constexpr int H = M / 2 + 1;
+#pragma unroll 2
+  for (int e = tid; e < RX * H; e += THR) {
+    const int row = e / H, k = e % H;
+    fx2_pack<M, S, Lay>(buf, row, k, spec(row, k), spec(row, M - k), post);
+  }
+  __syncthreads();
+  fx2_inv1<M, RX, S, Lay>(buf, tw);
+  const TR sr = (TR)s;
+  auto put = [&](int it, int row, int jj, const float2 *z) {
+    if (row < 0) return;
+    const TR *rr = reinterpret_cast<const TR *>(&rin[it]);
+    VEC o;
+    TR *oo = reinterpret_cast<TR *>(&o);
+#pragma unroll
+    for (int w = 0; w < VW; ++w) {
+      oo[2 * w] = (TR)z[w].x - sr * rr[2 * w];
+      oo[2 * w + 1] = (TR)z[w].y - sr * rr[2 * w + 1];
     }
-    const bool more = bat + gridDim.x < nbat;
-    if (more) FX2_LOAD(bat + gridDim.x, rn)
-    __syncthreads();
-    fft2<MC, RX, 256, false, false, LayC, SplitRow<MC>>(buf, twc);
-    // untangle to the Nc-point r2c, weights f_k (1/Nc, half at the Nyquist K)
-    for (int e = tid; e < RX * K1; e += 256) {
-      const int row = e / K1, k = e - row * K1;
-      V xk;
-      if (k == K) {
-        const V z0 = buf[LayC::at(0, row)];
-        xk = make_float2((z0.x - z0.y) * 0.5f * fk, 0.f);
-      } else {
-        const V zk = buf[LayC::at(k, row)];
-        const V zm = buf[LayC::at(k == 0 ? 0 : MC - k, row)];
-        V E, O;
-        E.x = (zk.x + zm.x) * 0.5f;
-        E.y = (zk.y - zm.y) * 0.5f;
-        O.x = (zk.y + zm.y) * 0.5f;
-        O.y = -(zk.x - zm.x) * 0.5f;
-        xk = cadd(E, cmul(postc[k], O));
-        xk.x *= fk; xk.y *= fk;
-      }
-      X[row * K1 + k] = xk;
+    *reinterpret_cast<VEC *>(out + (row0 + row) * (2 * M) + 2 * jj) = o;
+  };
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const int q = tid + i * THR;
+    if (q >= RX * S::R2) break;
+    const int row = q / S::R2, n2 = q % S::R2;
+    float2 u[S::R1];
+#pragma unroll
+    for (int k1 = 0; k1 < S::R1; ++k1) u[k1] = buf[Lay::at(S::R2 * k1 + n2, row)];
+    inv_step2<S>(u, tw);
+#pragma unroll
+    for (int n1 = 0; n1 < S::R1; ++n1) {
+      if constexpr (direct)
+        put(i * S::R1 + n1, row0 + row < rows ? row : -1, S::R2 * n1 + n2, &u[n1]);
+      else
+        buf[Lay::at(S::R2 * n1 + n2, row)] = u[n1];
     }
+  }
+  if constexpr (!direct) {
     __syncthreads();
-    fx_pack_c2r<M, RX, Lay>(X, K, K1, post, buf);
-    __syncthreads();
-    fft2<M, RX, 256, true, false, Lay, SplitRow<M>>(buf, tw);
 #pragma unroll
     for (int it = 0; it < CNT; ++it) {
-      const int e = tid + it * 256;
-      if (e >= NQ || e >= (rows - row0) * M / 2) break;
-      V ra, rb;
-      Quad<TR>::split(rr[it], ra, rb);
-      const V za = buf[Lay::at((2 * e) % M, (2 * e) / M)], zb = buf[Lay::at((2 * e + 1) % M, (2 * e + 1) / M)];
-      TO *o = out + row0 * N0 + 4 * e;  // 4 consecutive outputs, 4-element aligned
-      const TR *rx = r + row0 * N0 + 4 * e;
-      if constexpr (sizeof(TR) == 8) {
-        // the subtracted term in the output precision (r kept exact for FP64)
-        const double2 r01 = *reinterpret_cast<const double2 *>(rx), r23 = *reinterpret_cast<const double2 *>(rx + 2);
-        const double o0 = (double)za.x - s * r01.x, o1 = (double)za.y - s * r01.y;
-        const double o2 = (double)zb.x - s * r23.x, o3 = (double)zb.y - s * r23.y;
-        if constexpr (sizeof(TO) == 8) {
-          *reinterpret_cast<double2 *>(o) = make_double2(o0, o1);
-          *reinterpret_cast<double2 *>(o + 2) = make_double2(o2, o3);
-        } else {
-          o[0] = (TO)o0; o[1] = (TO)o1; o[2] = (TO)o2; o[3] = (TO)o3;
-        }
-      } else {
-        const float sf = (float)s;
-        const float o0 = za.x - sf * ra.x, o1 = za.y - sf * ra.y, o2 = zb.x - sf * rb.x, o3 = zb.y - sf * rb.y;
-        if constexpr (sizeof(TO) == 4) {
-          *reinterpret_cast<float4 *>(o) = make_float4(o0, o1, o2, o3);
-        } else {
-          o[0] = (TO)o0; o[1] = (TO)o1; o[2] = (TO)o2; o[3] = (TO)o3;
-        }
-      }
-    }
-    if (more) {
+      int row, jj;
+      where(it, row, jj);
+      float2 z[VW];
 #pragma unroll
-      for (int it = 0; it < CNT; ++it) rr[it] = rn[it];
+      for (int w = 0; w < VW; ++w) z[w] = row >= 0 ? buf[Lay::at(jj + w, row)] : float2{};
+      put(it, row, jj, z);
     }
-    __syncthreads();
   }
-#undef FX2_LOAD
 }
 
 }  // namespace rism

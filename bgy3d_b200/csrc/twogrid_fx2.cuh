@@ -3,8 +3,8 @@
 // per fine half row M over the coarse half rows MC that the coarse-grid rule
 // can pair with it: pairs without a kernel fall back to the (K+1) x Nc table
 // product (fine rows of the older shapes) or the dense tiles, at 162 -> 54
-// points 107 us per restriction and 153 us per prolongation against 62 and 80
-// here, at 64 -> 32 points 8.4 and 12.7 us against 5.7 and 7.1.  Instantiated by the twogrid_fx2*.cu translation units.
+// points 107 us per restriction and 153 us per prolongation against 34 and 63
+// here.  Instantiated by the twogrid_fx2*.cu translation units.
 #pragma once
 #include <cuda_runtime.h>
 
