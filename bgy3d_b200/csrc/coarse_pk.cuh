@@ -456,42 +456,6 @@ __device__ __forceinline__ void pk_z(const PkArgs &a, float2 *smem, const float2
   }
 }
 
-// Least squares of a k-step Arnoldi run, in place on the CTA's shared copy
-// of H (column j at H[j * (k + 1) + i], i <= j + 1) by Givens rotations:
-// y minimises |beta e1 - H y|; then y[0] += beta, so that sum y_j V_j = x +
-// r0.  By one warp, lane j the column j: rotation i comes from column i and is
-// applied to all later columns at once, and the back substitution takes each
-// y_i off every row above it at once (one thread took 10 us for 16 steps).
-__device__ __forceinline__ void pk_lsq(int k, double *H, double beta, double *y) {
-  const int ld = k + 1, lane = threadIdx.x & 31;
-  double g = lane == 0 ? beta : 0.0;  // entry `lane` of the rotated right-hand side
-  for (int i = 0; i < k; ++i) {
-    const double p = H[i * ld + i], q = H[i * ld + i + 1];  // the same words in every lane
-    const double r = hypot(p, q);
-    const double cs = r == 0.0 ? 1.0 : p / r, sn = r == 0.0 ? 0.0 : q / r;
-    __syncwarp();
-    if (lane >= i && lane < k) {
-      double *col = H + lane * ld;
-      const double u = col[i], v = col[i + 1];
-      col[i] = lane == i ? r : cs * u + sn * v;
-      col[i + 1] = lane == i ? 0.0 : -sn * u + cs * v;
-    }
-    const double gi = __shfl_sync(0xffffffffu, g, i);
-    if (lane == i) g = cs * gi;
-    if (lane == i + 1) g = -sn * gi;
-    __syncwarp();
-  }
-  double yi = 0.0;
-  for (int i = k - 1; i >= 0; --i) {
-    const double d = H[i * ld + i];
-    const double t = d != 0.0 ? __shfl_sync(0xffffffffu, g, i) / d : 0.0;
-    if (lane == i) yi = t;
-    if (lane < i) g -= H[i * ld + lane] * t;
-  }
-  if (lane < k) y[lane] = yi + (lane == 0 ? beta : 0.0);
-  __syncwarp();
-}
-
 // The end of a solve, by warp 0 of every CTA: CTA 0 writes H, s_0 and y out;
 // sY holds y_j / s_j.  The caller synchronises.
 __device__ __forceinline__ void pk_finish(const PkArgs &a, double *sH, const double *sS, double *sY) {

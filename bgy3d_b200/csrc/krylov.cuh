@@ -261,30 +261,34 @@ __global__ void __launch_bounds__(256) k_mdot_red(long long nw, const T *__restr
 }
 
 // k_maxpy_red: w -= sum_v h_v V_v (v < nv) and *hn = |w| reduced likewise.
-template <typename T>
+// A thread's loads are all issued before the first is used (16 vectors at a
+// time) and the last block's sum is a tree: beside other streams a sweep over
+// up to 16 vectors of a 48^3 grid took 17.5 us with its loads in turn and one
+// thread adding 256 values, 14 us here.
+template <typename T, int NVT>
 __global__ void __launch_bounds__(256) k_maxpy_red(long long nw, T *__restrict__ w, int nv, VecSet<T> vs,
                                                   const double *__restrict__ h, double *__restrict__ part,
                                                   unsigned *__restrict__ ticket, double *__restrict__ hn) {
   using VT = typename Wide<T>::type;
-  constexpr int WN = Wide<T>::n;
-  T c[kVecMax];
-#pragma unroll
-  for (int v = 0; v < kVecMax; ++v) c[v] = (T)(v < nv ? h[v] : 0.0);
+  constexpr int WN = Wide<T>::n, GV = NVT < 16 ? NVT : 16;
   double s2 = 0.0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nw; i += (long long)gridDim.x * blockDim.x) {
-    const VT a = reinterpret_cast<const VT *>(w)[i];
-    const T *ar = reinterpret_cast<const T *>(&a);
-    VT o;
+    VT o = reinterpret_cast<const VT *>(w)[i];
     T *r = reinterpret_cast<T *>(&o);
 #pragma unroll
-    for (int q = 0; q < WN; ++q) r[q] = ar[q];
+    for (int g = 0; g < NVT; g += GV) {
+      VT b[GV];
 #pragma unroll
-    for (int v = 0; v < kVecMax; ++v) {
-      if (v < nv) {
-        const VT b = reinterpret_cast<const VT *>(vs.p[v])[i];
-        const T *br = reinterpret_cast<const T *>(&b);
+      for (int v = 0; v < GV; ++v)
+        if (g + v < nv) b[v] = reinterpret_cast<const VT *>(vs.p[g + v])[i];
 #pragma unroll
-        for (int q = 0; q < WN; ++q) r[q] -= c[v] * br[q];
+      for (int v = 0; v < GV; ++v) {
+        if (g + v < nv) {
+          const T c = (T)h[g + v];
+          const T *br = reinterpret_cast<const T *>(&b[v]);
+#pragma unroll
+          for (int q = 0; q < WN; ++q) r[q] -= c * br[q];
+        }
       }
     }
     T sq = T(0);
@@ -303,21 +307,20 @@ __global__ void __launch_bounds__(256) k_maxpy_red(long long nw, T *__restrict__
     double a = 0.0;
     for (int q = 0; q < (int)(blockDim.x >> 5); ++q) a += sm[q];
     part[blockIdx.x] = a;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
-  __shared__ double red[256];
   double s = 0.0;
   for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s += part[b];
-  red[threadIdx.x] = s;
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) sm[wid] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
-    for (int q = 0; q < (int)blockDim.x; ++q) t += red[q];
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += sm[q];
     *hn = sqrt(t);
     *ticket = 0u;
   }
@@ -331,38 +334,51 @@ template <typename T> __global__ void k_scale_by(long long n, T *__restrict__ w,
     w[i] *= inv;
 }
 
-// Least squares of a k-step Arnoldi run, on one thread: min |beta e1 - H y|
-// with H's column j at H[j * (k + 1) + i], i <= j + 1; then y[0] += beta,
-// so that sum y_j V_j = x + r0 (the GMRES iterate plus its right-hand side).
-__global__ static void k_arnoldi_lsq(int k, const double *__restrict__ H, const double *__restrict__ beta,
-                                     double *__restrict__ y) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double R[kVecMax][kVecMax + 1];  // R[i][j], i <= j + 1
-  double g[kVecMax + 1], cs[kVecMax], sn[kVecMax];
-  for (int j = 0; j < k; ++j)
-    for (int i = 0; i <= j + 1; ++i) R[i][j] = H[j * (k + 1) + i];
-  for (int i = 0; i <= k; ++i) g[i] = 0.0;
-  g[0] = *beta;
-  for (int j = 0; j < k; ++j) {
-    for (int i = 0; i < j; ++i) {
-      const double a = R[i][j], b = R[i + 1][j];
-      R[i][j] = cs[i] * a + sn[i] * b;
-      R[i + 1][j] = -sn[i] * a + cs[i] * b;
+// Least squares of a k-step Arnoldi run, in place on a shared copy
+// of H (column j at H[j * (k + 1) + i], i <= j + 1) by Givens rotations:
+// y minimises |beta e1 - H y|; then y[0] += beta, so that sum y_j V_j = x +
+// r0.  By one warp, lane j the column j: rotation i comes from column i and is
+// applied to all later columns at once, and the back substitution takes each
+// y_i off every row above it at once (one thread took 10 us for 16 steps).
+__device__ __forceinline__ void pk_lsq(int k, double *H, double beta, double *y) {
+  const int ld = k + 1, lane = threadIdx.x & 31;
+  double g = lane == 0 ? beta : 0.0;  // entry `lane` of the rotated right-hand side
+  for (int i = 0; i < k; ++i) {
+    const double p = H[i * ld + i], q = H[i * ld + i + 1];  // the same words in every lane
+    const double r = hypot(p, q);
+    const double cs = r == 0.0 ? 1.0 : p / r, sn = r == 0.0 ? 0.0 : q / r;
+    __syncwarp();
+    if (lane >= i && lane < k) {
+      double *col = H + lane * ld;
+      const double u = col[i], v = col[i + 1];
+      col[i] = lane == i ? r : cs * u + sn * v;
+      col[i + 1] = lane == i ? 0.0 : -sn * u + cs * v;
     }
-    const double a = R[j][j], b = R[j + 1][j];
-    const double r = hypot(a, b);
-    cs[j] = r == 0.0 ? 1.0 : a / r;
-    sn[j] = r == 0.0 ? 0.0 : b / r;
-    R[j][j] = r;
-    g[j + 1] = -sn[j] * g[j];
-    g[j] = cs[j] * g[j];
+    const double gi = __shfl_sync(0xffffffffu, g, i);
+    if (lane == i) g = cs * gi;
+    if (lane == i + 1) g = -sn * gi;
+    __syncwarp();
   }
+  double yi = 0.0;
   for (int i = k - 1; i >= 0; --i) {
-    double s = g[i];
-    for (int l = i + 1; l < k; ++l) s -= R[i][l] * y[l];
-    y[i] = R[i][i] != 0.0 ? s / R[i][i] : 0.0;
+    const double d = H[i * ld + i];
+    const double t = d != 0.0 ? __shfl_sync(0xffffffffu, g, i) / d : 0.0;
+    if (lane == i) yi = t;
+    if (lane < i) g -= H[i * ld + lane] * t;
   }
-  if (k > 0) y[0] += *beta;
+  if (lane < k) y[lane] = yi + (lane == 0 ? beta : 0.0);
+  __syncwarp();
+}
+
+// The same as a kernel of one warp (k <= kVecMax): y from H and beta in global
+// memory.  One thread with its copy of H in local memory took 74 us for 16
+// steps.
+__global__ static void __launch_bounds__(32) k_arnoldi_lsq(int k, const double *__restrict__ H,
+                                                           const double *__restrict__ beta, double *__restrict__ y) {
+  __shared__ double sH[kVecMax * (kVecMax + 1)];
+  for (int q = threadIdx.x; q < k * (k + 1); q += 32) sH[q] = H[q];
+  __syncwarp();
+  pk_lsq(k, sH, *beta, y);
 }
 
 // Launch of the dot sweeps with the smallest accumulator bound NVT >= nv.
@@ -396,6 +412,16 @@ void launch_mdot_red(unsigned grid, cudaStream_t st, long long nw, const T *w, i
   else if (nv <= 8) k_mdot_red<T, 8><<<grid, 256, 0, st>>>(nw, w, nv, vs, part, ticket, h);
   else if (nv <= 16) k_mdot_red<T, 16><<<grid, 256, 0, st>>>(nw, w, nv, vs, part, ticket, h);
   else k_mdot_red<T, kVecMax><<<grid, 256, 0, st>>>(nw, w, nv, vs, part, ticket, h);
+}
+
+template <typename T>
+void launch_maxpy_red(unsigned grid, cudaStream_t st, long long nw, T *w, int nv, const VecSet<T> &vs, const double *h,
+                      double *part, unsigned *ticket, double *hn) {
+  if (nv <= 2) k_maxpy_red<T, 2><<<grid, 256, 0, st>>>(nw, w, nv, vs, h, part, ticket, hn);
+  else if (nv <= 4) k_maxpy_red<T, 4><<<grid, 256, 0, st>>>(nw, w, nv, vs, h, part, ticket, hn);
+  else if (nv <= 8) k_maxpy_red<T, 8><<<grid, 256, 0, st>>>(nw, w, nv, vs, h, part, ticket, hn);
+  else if (nv <= 16) k_maxpy_red<T, 16><<<grid, 256, 0, st>>>(nw, w, nv, vs, h, part, ticket, hn);
+  else k_maxpy_red<T, kVecMax><<<grid, 256, 0, st>>>(nw, w, nv, vs, h, part, ticket, hn);
 }
 
 }  // namespace rism

@@ -1164,7 +1164,7 @@ int coarse_steps(const rism3d_ctx *c) {
 // The coarse solve driven entirely on the device: k GMRES steps from zero
 // on J_H with an explicitly normalised basis, the dot products and norms
 // reduced into device memory, the small least-squares problem solved by one
-// thread, and tc_y = sum y_j V_j = J_H^-1 r + r written at the end.  On
+// warp, and tc_y = sum y_j V_j = J_H^-1 r + r written at the end.  On
 // entry the coarse basis vector 0 holds r; nothing here waits for the host,
 // so the whole sequence is captured once as a CUDA graph.
 void coarse_solve_dev(rism3d_ctx *c, int k) {
@@ -1189,11 +1189,11 @@ void coarse_solve_dev(rism3d_ctx *c, int k) {
     double *h = H + (size_t)j * (k + 1);
     // classical Gram-Schmidt, each sweep with its reduction fused in
     launch_mdot_red<float>(G, st, nw, B[j + 1], j + 1, vs, cc->dpart, c->cg_ticket, h);
-    k_maxpy_red<float><<<G, 256, 0, st>>>(nw, B[j + 1], j + 1, vs, h, cc->dpart, c->cg_ticket, h + j + 1);
+    launch_maxpy_red<float>(G, st, nw, B[j + 1], j + 1, vs, h, cc->dpart, c->cg_ticket, h + j + 1);
     k_scale_by<float><<<gv, 256, 0, st>>>(cc->nvec, B[j + 1], h + j + 1);
     CKL();
   }
-  k_arnoldi_lsq<<<1, 1, 0, st>>>(k, H, beta, y);
+  k_arnoldi_lsq<<<1, 32, 0, st>>>(k, H, beta, y);
   VecSet<float> vs{};
   for (int i = 0; i < kVecMax; ++i) vs.p[i] = B[i < k ? i : 0];
   launch_maxpyv<float>(G, st, nw, c->tc_y, 0.0, k, vs, mone, y, nullptr);
@@ -2142,10 +2142,13 @@ void bind_solute(rism3d_ctx *c, int n, const rism3d_site *solute) {
 }
 
 // ------------------------------------------------------------ autotuner
-// The batch sizes of the runtime-length passes (x rows, y and z columns per
-// CTA) and, where shape-specialised passes exist, the choice between them and
-// the runtime-length ones are timed on the context's own buffers the first
-// time a (grid, fields) shape is seen in the process; the winners are cached.
+// The forms of the specialised z pass or, where the passes are runtime-length,
+// their batch sizes (x rows, y and z columns per CTA) are timed on the
+// context's own buffers the first time a (grid, fields) shape is seen in the
+// process; the winners are cached.  The specialised passes are not timed
+// against the others: they are the faster ones at every length, by 1.5 times
+// and more, and timings made beside the streams of a batch once kept a whole
+// process on the slower ones for a shape.
 // Only the scheduling changes: every candidate computes the same transforms
 // column by column.  RISM3D_AUTOTUNE=0 keeps the register / occupancy rule.
 struct TuneVal {
@@ -2188,13 +2191,30 @@ template <typename T> void tune_precision(rism3d_ctx *c, const T *A, const T *Bv
   const size_t cs = sizeof(typename Cx<T>::type);
   const long long lim = optin_limit();
   const int reps = G.Nr >= (1LL << 22) ? 2 : 5;
-  const bool had_stat = c->stat[pr], had_xy = c->xy[pr];
-  c->stat[pr] = c->xy[pr] = false;
   auto run = [&] { pipeline<T, MODE_J>(c, A, Bv, (T)1, (T)1, out, false); };
+  if (c->pure && c->xy[pr]) return;
+  if (c->stat[pr]) {
+    if (!z_has_variants(G.N2)) return;
+    const float s_ms = time_ms(c, run, reps);
+    // the specialised z pass: wide tiles, or half as wide (twice the CTAs
+    // in flight per SM)
+    const int wide = c->zb[pr];
+    if (pr == 1) {  // FP32 only: 64-byte rows (FP64 would drop to 32-thread CTAs)
+      c->zb[pr] = wide / 2;
+      make_tmap(c, &c->tmz[pr], pr == 0, c->zb[pr], 1, G.N2);
+      if (time_ms(c, run, reps) < 0.95f * s_ms) return;
+      c->zb[pr] = wide;
+      make_tmap(c, &c->tmz[pr], pr == 0, wide, 1, G.N2);
+    }
+    // persistent double-buffered CTAs for the wide tiles
+    c->zpers[pr] = true;
+    c->zpers[pr] = time_ms(c, run, reps) < 0.97f * s_ms;
+    return;
+  }
   const int cand[4] = {4, 8, 16, 32};
-  // one axis at a time, the others held
+  // one axis at a time, the others held (z only beside specialised x and y)
   int *fields[3] = {&t.RX, &t.BY, &t.BZ};
-  for (int axis = 0; axis < 3; ++axis) {
+  for (int axis = c->xy[pr] ? 2 : 0; axis < 3; ++axis) {
     int best = *fields[axis];
     float best_ms = time_ms(c, run, reps);
     for (int k : cand) {
@@ -2218,34 +2238,6 @@ template <typename T> void tune_precision(rism3d_ctx *c, const T *A, const T *Bv
       *fields[axis] = keep;
     }
     *fields[axis] = best;
-  }
-  if (had_xy) {
-    const float g_ms = time_ms(c, run, reps);
-    c->xy[pr] = true;
-    c->stat[pr] = had_stat;
-    float s_ms = time_ms(c, run, reps);
-    // the specialised z pass: wide tiles, or half as wide (twice the CTAs
-    // in flight per SM)
-    const int wide = c->zb[pr];
-    float n_ms = 1e30f;
-    if (pr == 1 && had_stat && z_has_variants(G.N2)) {  // FP32 only: 64-byte rows (FP64 would drop to 32-thread CTAs)
-      c->zb[pr] = wide / 2;
-      make_tmap(c, &c->tmz[pr], pr == 0, c->zb[pr], 1, G.N2);
-      n_ms = time_ms(c, run, reps);
-    }
-    if (n_ms < 0.95f * s_ms) {
-      s_ms = n_ms;
-    } else if (had_stat && z_has_variants(G.N2)) {
-      c->zb[pr] = wide;
-      make_tmap(c, &c->tmz[pr], pr == 0, wide, 1, G.N2);
-      // persistent double-buffered CTAs for the wide tiles
-      c->zpers[pr] = true;
-      const float p_ms = time_ms(c, run, reps);
-      if (p_ms < 0.97f * s_ms) s_ms = p_ms;
-      else c->zpers[pr] = false;
-    }
-    c->xy[pr] = s_ms <= 1.05f * g_ms;  // keep the specialised passes unless clearly slower
-    c->stat[pr] = had_stat && c->xy[pr];
   }
 }
 
