@@ -2791,6 +2791,8 @@ void long_range_field(rism3d_ctx *c, double *out) {
   TimeScope ts(c, TK_XINV, 0);
   const int RX = c->tl<double>().RX;
   dim3 gx((c->g.N1 * c->g.N2 + RX - 1) / RX, c->m);
+  // the pass subtracts 0 * out: fresh pool memory may hold NaN
+  CK(cudaMemsetAsync(out, 0, sizeof(double) * c->nvec, c->stream));
   k_xinv<double><<<gx, 256, xsmem<double>(c), c->stream>>>(c->g, c->plan<double>(0), RX, c->work<double>(), out, out,
                                                           1.0 / (double)c->g.Nr, 0.0, postw<double>(c), c->npart);
   CKL();

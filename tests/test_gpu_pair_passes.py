@@ -13,7 +13,7 @@ torch = pytest.importorskip("torch")
 
 pytestmark = pytest.mark.gpu
 
-from bgy3d_b200 import RismContext, find_molecule  # noqa: E402
+from bgy3d_b200 import RismContext, find_molecule, hnc3d_run_solvent  # noqa: E402
 
 
 def compare(make, monkeypatch, cases):
@@ -54,3 +54,17 @@ def test_five_sites(fixture_loader, N, monkeypatch):
     chi = np.ascontiguousarray(arr["chi"][np.ix_(i, i)])
     compare(lambda: RismContext(meta["solute"], [meta["solvent"][j] for j in i], s, chi), monkeypatch,
             [(torch.float64, 1e-12), (torch.float32, 2e-5)])
+
+
+def test_solvent_energy_ignores_stale_device_memory():
+    """The free energies after a context whose buffers were full of NaN is given back to the pool."""
+    w = find_molecule("water")
+    s = {"N": 48, "L": 10.0, "rho": 0.033427745, "beta": 1.6889, "norm-tol": 1e-12, "closure": "KH", "max-iter": 100}
+    want = hnc3d_run_solvent(w, s)["free-energy"]
+    for n in (48, 54, 64):
+        ctx = RismContext(None, w, dict(s, N=n), None)
+        ctx.jacobian_t1(torch.zeros(ctx.shape, device="cuda", dtype=torch.float64),
+                        torch.full(ctx.shape, float("nan"), device="cuda", dtype=torch.float64))
+        ctx.close()
+        got = hnc3d_run_solvent(w, s)["free-energy"]
+        assert abs(got - want) < 1e-8
