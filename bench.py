@@ -66,7 +66,8 @@ PLAIN_FP64 = {"precision": "fp64", "coarse-h": 0, "ew-forcing": 0, "krylov-resta
 # DRAM bytes (read + write) of the five FP32 passes of one Jacobian product at
 # 256^3 (x-forward 576.0, y 352.9, z 351.7, y-inverse 352.8, x-inverse
 # 574.1 MB), measured by ncu dram__bytes_read.sum + dram__bytes_write.sum on
-# the shape-specialised kernels.
+# the shape-specialised kernels; the z pass now also reads the 54 MB octant
+# table of chi - 1, which is not in this figure.
 JV_TRAFFIC = 2207.5e6
 
 
