@@ -2842,11 +2842,15 @@ template <int MS> void chi_out_launch(rism3d_ctx *c, double2 *out) {
   CKL();
 }
 
-// Newton-GMRES on the pair fields from T (device, in/out), then the
-// observables, chi - 1 on the k grid and g (host outputs, each optional).
 void d2h_large(void *dst, const void *src, size_t bytes, cudaStream_t st);
 
-int solvent_solve_impl(rism3d_ctx *c, double *T, double *chi_out, double *g_out, rism3d_solvent_result *res) {
+// Newton-GMRES on the pair fields from T (device, in/out), then the
+// observables, chi - 1 on the k grid and g (host outputs, each optional).
+// `before_copies` runs once the device has everything queued and before a byte
+// of a host output is written.
+template <typename F>
+int solvent_solve_impl(rism3d_ctx *c, double *T, double *chi_out, double *g_out, rism3d_solvent_result *res,
+                       F &&before_copies) {
   const rism3d_problem &pd = c->pd;
   *res = rism3d_solvent_result{};
   c->f_evals = c->jv_evals = 0;
@@ -2867,19 +2871,21 @@ int solvent_solve_impl(rism3d_ctx *c, double *T, double *chi_out, double *g_out,
   CKL();
   std::vector<double> hp((size_t)rb * 5);
   CK(cudaMemcpyAsync(hp.data(), part, sizeof(double) * hp.size(), cudaMemcpyDeviceToHost, c->stream));
+  double2 *dchi = nullptr;
+  const size_t chi_bytes = sizeof(double2) * (size_t)c->m * G.Nh * G.N1 * G.N2;
   if (chi_out) {
     fwd3d(c, h);
-    const long long nk = (long long)G.Nh * G.N1 * G.N2;
-    double2 *dchi = dalloc<double2>((size_t)c->m * nk);
+    dchi = dalloc<double2>(chi_bytes / sizeof(double2));
     switch (c->pure) {
       case 1: chi_out_launch<1>(c, dchi); break;
       case 2: chi_out_launch<2>(c, dchi); break;
       case 3: chi_out_launch<3>(c, dchi); break;
       default: chi_out_launch<4>(c, dchi); break;
     }
-    d2h_large(chi_out, dchi, sizeof(double2) * (size_t)c->m * nk, c->stream);
-    dfree(dchi);
   }
+  before_copies();
+  if (chi_out) d2h_large(chi_out, dchi, chi_bytes, c->stream);
+  dfree(dchi);
   if (g_out) d2h_large(g_out, g, sizeof(double) * nv, c->stream);
   CK(cudaEventRecord(e1, c->stream));
   CK(cudaEventSynchronize(e1));
@@ -3342,7 +3348,8 @@ void cache_clear() {
 // Rewrites one byte of every page of [p, p + bytes) with its own value from a
 // few host threads: a caller's fresh result buffer (a NumPy array) takes its
 // first-touch page faults here, while the device solves, instead of inside the
-// copy-out.
+// copy-out.  To be joined before anything else writes there: a value read
+// before that write and stored after it would undo it.
 struct PageToucher {
   std::vector<std::thread> th;
   PageToucher(void *p, size_t bytes) {
@@ -3625,7 +3632,11 @@ int rism3d_solvent_solve(const rism3d_problem *pd, int m, const rism3d_site *sol
       else solvent_guess(ctx, T);
       const size_t nk = (size_t)ctx->g.Nh * ctx->g.N1 * ctx->g.N2;
       PageToucher touch_t(t_out, bytes), touch_chi(chi_out, sizeof(double2) * ctx->m * nk), touch_g(g_out, bytes);
-      const int st = solvent_solve_impl(ctx, T, chi_out, g_out, &res);
+      const int st = solvent_solve_impl(ctx, T, chi_out, g_out, &res, [&] {
+        touch_t.join();
+        touch_chi.join();
+        touch_g.join();
+      });
       if (t_out) d2h_large(t_out, T, bytes, ctx->stream);
       return st;
     });
