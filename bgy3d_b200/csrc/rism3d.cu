@@ -588,16 +588,23 @@ void reduce_norms(rism3d_ctx *c, int nblk, double *resid) {
   resid[1] = std::sqrt(h[1]);
 }
 
+// Whether vectors at these addresses can be read and written 16 bytes at a time.
+template <typename... P> bool aligned16(const P *...p) {
+  return ((reinterpret_cast<uintptr_t>(p) | ... | uintptr_t(0)) & 15) == 0;
+}
+
 // The five passes of one residual (MODE_F: A = t, Bv = v, p = beta) or
 // Jacobian product (MODE_J: A = dt, Bv = d = c'(t), p = scale of dt);
 // out = (FFT^-1 ...) / N - sub * A.  Returns the number of norm partials (made
-// where `norms`).  MODE_S (shape-specialised passes only): a Jacobian product
-// with the slope at `t` (A = dt, Bv = v, p = beta).
+// where `norms`).  MODE_S (shape-specialised passes and aligned vectors only): a
+// Jacobian product with the slope at `t` (A = dt, Bv = v, p = beta).  The
+// specialised x passes move 16 bytes at a time; a caller's FP32 vectors on an
+// 8-byte boundary take the runtime-length ones, which move pairs of values.
 template <typename T, int MODE>
 int pipeline(rism3d_ctx *c, const T *A, const T *Bv, T p, T sub, T *out, bool norms = true, const T *t = nullptr) {
   const int rows = c->g.N1 * c->g.N2;
   auto *W = c->work<T>();
-  const bool st = c->xy[sizeof(T) == 8 ? 0 : 1];
+  const bool st = c->xy[sizeof(T) == 8 ? 0 : 1] && aligned16(A, Bv, out, t);
   const int RX = st ? x_rows(sizeof(T) == 8, c->g.M) : c->tl<T>().RX;
   dim3 gx((rows + RX - 1) / RX, c->m);
   const auto *twx = static_cast<const typename Cx<T>::type *>(c->plan<T>(0).tw);
@@ -922,10 +929,11 @@ template <typename TS, typename TJ> void closure_slope(rism3d_ctx *c, const TS *
 // One Jacobian product at x from scratch (the jacobian_t1 entry points).  The
 // shape-specialised x pass takes the slope from x and v as it goes, where a
 // slope field beforehand cost a write and a read of it (246 us of a 1256 us
-// FP64 product at 256^3).
+// FP64 product at 256^3); x may start at any element, and off 16 bytes goes
+// through the slope field, as a whole product does whose vectors are off them.
 template <typename T> int jacobian_product(rism3d_ctx *c, const T *x, const T *dx, T *out) {
   const int pr = sizeof(T) == 8 ? 0 : 1;
-  if (c->xy[pr] && !c->pure) {
+  if (c->xy[pr] && !c->pure && aligned16(x, dx, out)) {
     pipeline<T, MODE_S>(c, dx, vfield<T>(c), (T)c->pd.beta, (T)1, out, false, x);
     if (pr == 0) c->jv_evals++; else c->jv32_evals++;
   } else {
@@ -1006,7 +1014,8 @@ unsigned persistent_grid(const void *fn, size_t smem, unsigned work, int threads
 }
 
 // x-axis transfers by FFT (twogrid_fft.cuh) where the row length has a
-// shape-specialised transform; false: use the dense tiles.
+// shape-specialised transform and the fine fields are 16-byte aligned (a
+// caller's may not be); false: use the dense tiles, which take any element.
 constexpr int kFxRX = 16;
 bool fx_usable(const rism3d_ctx *c) {
   const char *dense = std::getenv("RISM3D_DENSE_TRANSFERS");  // 1: the dense tiles everywhere (tests)
@@ -1044,7 +1053,7 @@ bool fx2_prolong(int M, int MC, long long rows, const float *y, const float2 *po
   }
 }
 template <typename T> bool fx_restrict(rism3d_ctx *c, long long rows, const T *in, double s) {
-  if (!fx_usable(c)) return false;
+  if (!fx_usable(c) || !aligned16(in)) return false;
   const int K = c->Nc[0] / 2;
   const auto *post = postw<float>(c);
   const auto *tw = static_cast<const float2 *>(c->plan<float>(0).tw);
@@ -1072,7 +1081,7 @@ template <typename T> bool fx_restrict(rism3d_ctx *c, long long rows, const T *i
   return true;
 }
 template <typename T> bool fx_prolong(rism3d_ctx *c, long long rows, const T *r, double s, T *out) {
-  if (!fx_usable(c)) return false;
+  if (!fx_usable(c) || !aligned16(r, out)) return false;
   const int K = c->Nc[0] / 2;
   const auto *post = postw<float>(c);
   const auto *tw = static_cast<const float2 *>(c->plan<float>(0).tw);
@@ -3399,6 +3408,16 @@ int solve_on(rism3d_ctx *ctx, double *t_inout, double *g_out, rism3d_result *out
   return st;
 }
 
+// The passes read and write pairs of values at least.
+template <typename T, typename... P> void require_pairs(const T *a, const P *...rest) {
+  if (((reinterpret_cast<uintptr_t>(a) | ... | reinterpret_cast<uintptr_t>(rest)) & (2 * sizeof(T) - 1)) != 0)
+    throw ArgFail{RISM3D_ERR_ARG, "vectors must be aligned to two elements"};
+}
+template <typename T, typename... P> void require_elements(const T *a, const P *...rest) {
+  if (((reinterpret_cast<uintptr_t>(a) | ... | reinterpret_cast<uintptr_t>(rest)) & (sizeof(T) - 1)) != 0)
+    throw ArgFail{RISM3D_ERR_ARG, "vectors must be aligned to their elements"};
+}
+
 template <typename F> int guard(F &&f) {
   try {
     return f();
@@ -3463,6 +3482,7 @@ long long rism3d_ctx_size(const rism3d_ctx *ctx) { return ctx ? ctx->nvec : 0; }
 int rism3d_iterate_t1(rism3d_ctx *ctx, const double *T, double *dT, double *resid) {
   if (!ctx || !T || !dT) return RISM3D_ERR_ARG;
   return guard([&] {
+    require_pairs(T, dT);
     double r[2];
     eval_F<double>(ctx, T, dT, r);
     if (resid) resid[0] = r[0], resid[1] = r[1];
@@ -3474,6 +3494,8 @@ int rism3d_jacobian_t1(rism3d_ctx *ctx, const double *T, const double *dT, doubl
   if (!ctx || !T || !dT || !JdT) return RISM3D_ERR_ARG;
   if (ctx->pd.closure == RISM3D_PY) return RISM3D_ERR_UNSUPPORTED;
   return guard([&] {
+    require_elements(T);
+    require_pairs(dT, JdT);
     return jacobian_product<double>(ctx, T, dT, JdT);
   });
 }
@@ -3482,6 +3504,7 @@ int rism3d_iterate_t1_f32(rism3d_ctx *ctx, const float *T, float *dT, double *re
   if (!ctx || !T || !dT) return RISM3D_ERR_ARG;
   if (ctx->pure) return RISM3D_ERR_UNSUPPORTED;
   return guard([&] {
+    require_pairs(T, dT);
     double r[2];
     eval_F<float>(ctx, T, dT, r);
     if (resid) resid[0] = r[0], resid[1] = r[1];
@@ -3494,6 +3517,8 @@ int rism3d_jacobian_t1_f32(rism3d_ctx *ctx, const float *T, const float *dT, flo
   if (!ctx || !T || !dT || !JdT) return RISM3D_ERR_ARG;
   if (ctx->pd.closure == RISM3D_PY) return RISM3D_ERR_UNSUPPORTED;
   return guard([&] {
+    require_elements(T);
+    require_pairs(dT, JdT);
     return jacobian_product<float>(ctx, T, dT, JdT);
   });
 }
@@ -3758,6 +3783,7 @@ int rism3d_precondition(rism3d_ctx *ctx, const double *T, const double *v, doubl
   if (!ctx || !T || !v || !z) return RISM3D_ERR_ARG;
   if (!ctx->coarse) return RISM3D_ERR_UNSUPPORTED;
   return guard([&] {
+    require_elements(T, v, z);
     double *d = slopebuf<double>(ctx);
     closure_slope<double, double>(ctx, T, d);
     tg_prepare<double>(ctx, d);
@@ -3771,6 +3797,7 @@ int rism3d_precondition_f32(rism3d_ctx *ctx, const float *T, const float *v, flo
   if (!ctx || !T || !v || !z) return RISM3D_ERR_ARG;
   if (!ctx->coarse) return RISM3D_ERR_UNSUPPORTED;
   return guard([&] {
+    require_elements(T, v, z);
     float *d = slopebuf<float>(ctx);
     closure_slope<float, float>(ctx, T, d);
     tg_prepare<float>(ctx, d);

@@ -157,7 +157,8 @@ __global__ void __launch_bounds__(kPxThreads) k_prolong_x(long long rows, int N,
     __syncthreads();
   }
   const int c0 = col0 + tc * 8;
-  const bool full = c0 + 8 <= N && (N % 8) == 0;
+  const bool full = c0 + 8 <= N && (N % 8) == 0 &&
+                    ((reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
 #pragma unroll
   for (int a = 0; a < 8; ++a) {
     const long long row = row0 + tr * 8 + a;

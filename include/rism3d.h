@@ -238,7 +238,11 @@ long long rism3d_ctx_size(const rism3d_ctx *ctx);
 
 /* F(T) = (chi-1) * c(T) - beta/eps0 tau - T: the VecFunc1 iterate_t1
    (hnc3d.c:1183-1285).  T, dT: device pointers, FP64, [m][N2][N1][N0].
-   resid (optional, host, 2 doubles) receives ||dT||_inf and ||dT||_2. */
+   resid (optional, host, 2 doubles) receives ||dT||_inf and ||dT||_2.
+   Vectors on 16-byte boundaries (as cudaMalloc gives them) run fastest.  FP64
+   ones have to be on one, FP32 ones on an 8-byte boundary, except the state T
+   of the Jacobian products, which may start at any element; else
+   RISM3D_ERR_ARG. */
 int rism3d_iterate_t1(rism3d_ctx *ctx, const double *T, double *dT, double *resid);
 
 /* J(T) dT = (chi-1) * (c'(T) dT) - dT: the VecFunc2 jacobian_t1
@@ -271,7 +275,8 @@ const char *rism3d_last_error(void);
    M^-1 v = P (J_H^-1 + I) R v - v, where R / P are the band-limited
    transfers to / from the coarse grid, J_H the coarse Jacobian built from
    the restricted closure slope R c'(T), and J_H^-1 a coarse_steps-step
-   FP32 GMRES from zero.  Device pointers, FP64 [m][N2][N1][N0].  Returns
+   FP32 GMRES from zero.  Device pointers, FP64 [m][N2][N1][N0], from any
+   element (fastest on 16-byte boundaries).  Returns
    RISM3D_ERR_UNSUPPORTED when the context has no coarse grid. */
 int rism3d_precondition(rism3d_ctx *ctx, const double *T, const double *v, double *z);
 
