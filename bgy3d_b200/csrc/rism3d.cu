@@ -2162,7 +2162,6 @@ void bind_solute(rism3d_ctx *c, int n, const rism3d_site *solute) {
 // column by column.  RISM3D_AUTOTUNE=0 keeps the register / occupancy rule.
 struct TuneVal {
   TileShape t[2];
-  bool stat[2], xy[2];
   int zb[2];
   bool zpers[2];
 };
@@ -2266,23 +2265,23 @@ void force_z_persistent(rism3d_ctx *c) {
   }
 }
 
-// Applies the cached shapes of this context's (grid, fields) or times them.
+// Applies the cached shapes of this context's (grid, fields, pass family) or
+// times them; the family is the context's own (specialise), never the cache's.
 void autotune(rism3d_ctx *c) {
   struct Force { rism3d_ctx *c; ~Force() { force_z_persistent(c); } } force{c};
   const char *env = std::getenv("RISM3D_AUTOTUNE");
   if (env && env[0] == '0') return;
   const Geo &G = c->g;
   const int kind = c->pure ? 2 : (c->chi3_64 ? 1 : 0);  // the z pass differs per kind
-  const auto key = std::make_tuple(G.N0, G.N1, G.N2, G.m, kind);
+  const int family = (c->xy[0] ? 1 : 0) + (c->stat[0] ? 2 : 0);  // alike in both precisions
+  const auto key = std::make_tuple(G.N0, G.N1, G.N2, G.m, 4 * kind + family);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
     if (it != g_tune.end()) {
       for (int pr = 0; pr < 2; ++pr) {
         c->tiles[pr] = it->second.t[pr];
-        c->xy[pr] = c->xy[pr] && it->second.xy[pr];
-        c->stat[pr] = c->stat[pr] && it->second.stat[pr];
-        c->zpers[pr] = c->stat[pr] && it->second.zpers[pr];
+        c->zpers[pr] = it->second.zpers[pr];
         if (c->stat[pr] && c->zb[pr] != it->second.zb[pr]) {
           c->zb[pr] = it->second.zb[pr];
           make_tmap(c, &c->tmz[pr], pr == 0, c->zb[pr], 1, G.N2);
@@ -2309,8 +2308,6 @@ void autotune(rism3d_ctx *c) {
   TuneVal v;
   for (int pr = 0; pr < 2; ++pr) {
     v.t[pr] = c->tiles[pr];
-    v.stat[pr] = c->stat[pr];
-    v.xy[pr] = c->xy[pr];
     v.zb[pr] = c->zb[pr];
     v.zpers[pr] = c->zpers[pr];
   }
