@@ -282,17 +282,19 @@ template <typename T> struct ZParams {
 // rows are 32-byte aligned and need no bounds check (the padding holds 0).
 __host__ __device__ __forceinline__ int oct_row(const Geo &g) { return (g.Nh + 7) & ~7; }
 
-// A radial table on the k grid: out[q][|ky|][|kz|][kx] = table q at |k|, by the
-// interpolation rule of the passes (nearest entry plus slope, in T).  |k| only
-// depends on |ky| and |kz|, so the octant 0 <= ky <= N1/2, 0 <= kz <= N2/2
-// holds every value of the half spectrum.  The shape-specialised z passes read
-// it in place of the FP64 square root and division and the gathered pairs that
-// the rule takes at every point: alone that changed nothing (their time was
-// barriers), but a tile's values become rows that can be staged beside it.
-// 54 MB per FP32 context at 256^3, m = 3.
+// Radial tables on the k grid: kt[q][|ky|][|kz|][kx] = table q of chi at |k|
+// (nchi of them) and ks likewise of s (ns), by the interpolation rule of the
+// passes (nearest entry plus slope, in T).  |k| only depends on |ky| and |kz|, so
+// the octant 0 <= ky <= N1/2, 0 <= kz <= N2/2 holds every value of the half
+// spectrum.  The shape-specialised z passes read it in place of the FP64 square
+// root and division and the gathered pairs that the rule takes at every point:
+// alone that changed nothing (their time was barriers), but a tile's values
+// become rows that can be staged beside it.  At 256^3, m = 3, 9 tables are 81 MB
+// in FP32 and 163 MB in FP64.
 template <typename T>
-__global__ void __launch_bounds__(256) k_octant(Geo g, const typename Vec2<T>::type *__restrict__ tab, int ntab, int nrad,
-                                                double dkr, T *__restrict__ out) {
+__global__ void __launch_bounds__(256) k_octant(Geo g, const typename Vec2<T>::type *__restrict__ chi, int nchi,
+                                                const typename Vec2<T>::type *__restrict__ s, int ns, int nrad,
+                                                double dkr, T *__restrict__ kt, T *__restrict__ ks) {
   const int H1 = g.N1 / 2 + 1, H2 = g.N2 / 2 + 1;
   const int OR = oct_row(g);
   const long long oct = (long long)H1 * H2 * OR;
@@ -306,9 +308,13 @@ __global__ void __launch_bounds__(256) k_octant(Geo g, const typename Vec2<T>::t
   int i = (int)(ix + 0.5);
   i = min(max(i, 0), nrad - 1);
   const T fr = T(ix - i);
-  for (int q = 0; q < ntab; ++q) {
-    const typename Vec2<T>::type t = tab[(long long)q * nrad + i];
-    out[q * oct + e] = kx < g.Nh ? t.x + t.y * fr : T(0);
+  for (int q = 0; q < nchi; ++q) {
+    const typename Vec2<T>::type t = chi[(long long)q * nrad + i];
+    kt[q * oct + e] = kx < g.Nh ? t.x + t.y * fr : T(0);
+  }
+  for (int q = 0; q < ns; ++q) {
+    const typename Vec2<T>::type t = s[(long long)q * nrad + i];
+    ks[q * oct + e] = kx < g.Nh ? t.x + t.y * fr : T(0);
   }
 }
 

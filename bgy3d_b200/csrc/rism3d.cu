@@ -220,7 +220,7 @@ struct rism3d_ctx {
   float2 *L32 = nullptr;
   double2 *chi64 = nullptr, *s64 = nullptr;
   float2 *chi32 = nullptr, *s32 = nullptr;
-  double *kt64 = nullptr, *ks64 = nullptr;  // the tables above on the octant of the k grid (made on first use)
+  double *kt64 = nullptr, *ks64 = nullptr;  // the tables above on the octant of the k grid
   float *kt32 = nullptr, *ks32 = nullptr;
   double2 *chi3_64 = nullptr;  // chi - 1 on the k grid (W layout, packed pairs), or null
   float2 *chi3_32 = nullptr;
@@ -347,42 +347,55 @@ struct TimeScope {
 
 long long octant_size(const Geo &g) { return (long long)(g.N1 / 2 + 1) * (g.N2 / 2 + 1) * oct_row(g); }
 
-// Radial tables on the octant of the k grid: made once per context and
-// precision, on the stream of the pass that first needs them (before any
-// capture: coarse_graph and coarse_pk_ready ask for theirs up front).
+// Radial tables on the octant of the k grid, chi - 1 and (lr) the long-range
+// factor, as far as they are not there: in one launch, on the context's stream.
 template <typename T>
-const T *octant_table(rism3d_ctx *c, const typename Vec2<T>::type *tab, int ntab, T **slot) {
-  if (!*slot && tab) {
-    const long long oct = octant_size(c->g);
-    T *p = dalloc<T>((size_t)ntab * oct);
-    k_octant<T><<<(unsigned)((oct + 255) / 256), 256, 0, c->stream>>>(c->g, tab, ntab, c->pd.nrad, c->dkr, p);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) dfree(p);
-    CK(e);
-    *slot = p;
+void octant_tables(rism3d_ctx *c, const typename Vec2<T>::type *chi, const typename Vec2<T>::type *s, bool lr, T **kt,
+                   T **ks) {
+  const int np = !*kt && chi ? c->m * (c->m + 1) / 2 : 0, ns = lr && !*ks && s && c->pd.renorm ? c->m : 0;
+  if (np + ns == 0) return;
+  const long long oct = octant_size(c->g);
+  T *a = nullptr, *b = nullptr;
+  try {
+    if (np) a = dalloc<T>((size_t)np * oct);
+    if (ns) b = dalloc<T>((size_t)ns * oct);
+    k_octant<T><<<(unsigned)((oct + 255) / 256), 256, 0, c->stream>>>(c->g, chi, np, s, ns, c->pd.nrad, c->dkr, a, b);
+    CKL();
+  } catch (...) {  // a table that was not filled is not kept
+    dfree(a);
+    dfree(b);
+    throw;
   }
-  return *slot;
+  if (np) *kt = a;
+  if (ns) *ks = b;
+}
+// A context makes the tables of its own arithmetic when it is made, so that its
+// first evaluation costs what later ones do; those of the other precision come
+// with the first pass that asks for them (never inside a capture: coarse_graph
+// and coarse_pk_ready ask for theirs up front).
+template <typename T> void octant_tables(rism3d_ctx *c, bool lr) {
+  if constexpr (sizeof(T) == 8) octant_tables<double>(c, c->chi64, c->s64, lr, &c->kt64, &c->ks64);
+  else octant_tables<float>(c, c->chi32, c->s32, lr, &c->kt32, &c->ks32);
 }
 
 template <typename T> ZParams<T> zparams(rism3d_ctx *c, bool full) {
   constexpr bool f64 = sizeof(T) == 8;
   ZParams<T> z{};
-  const int np = c->m * (c->m + 1) / 2;
-  const bool oct = c->stat[f64 ? 0 : 1];  // the shape-specialised z passes read the octant tables
+  if (c->stat[f64 ? 0 : 1]) octant_tables<T>(c, full);  // read by the shape-specialised z passes
   if constexpr (f64) {
     z.chi = c->chi64;
     z.chi3 = c->chi3_64;
     z.stab = (full && c->pd.renorm) ? c->s64 : nullptr;
     z.L = full ? c->L64 : nullptr;
-    if (oct) z.kt = octant_table<T>(c, c->chi64, np, &c->kt64);
-    if (oct && z.stab) z.ks = octant_table<T>(c, c->s64, c->m, &c->ks64);
+    z.kt = c->kt64;
+    z.ks = z.stab ? c->ks64 : nullptr;
   } else {
     z.chi = c->chi32;
     z.chi3 = c->chi3_32;
     z.stab = (full && c->pd.renorm) ? c->s32 : nullptr;
     z.L = full ? c->L32 : nullptr;
-    if (oct) z.kt = octant_table<T>(c, c->chi32, np, &c->kt32);
-    if (oct && z.stab) z.ks = octant_table<T>(c, c->s32, c->m, &c->ks32);
+    z.kt = c->kt32;
+    z.ks = z.stab ? c->ks32 : nullptr;
   }
   z.oct = octant_size(c->g);
   z.nrad = c->pd.nrad;
@@ -2503,8 +2516,10 @@ void allow_xy(size_t need) {
 // [m(m+1)/2][N2][N1][N0/2+1] (the --solvent-3d kernel); then chi is unused,
 // the long-range term takes the no-renorm form and the passes are the
 // runtime-length ones without the two-grid preconditioner.
+// coarse: the coarse problem of a preconditioner, which only evaluates FP32
+// Jacobian products.
 int create_impl(const rism3d_problem *pd, int m, const rism3d_site *solvent, int n, const rism3d_site *solute,
-                const double *chi, const double *chi3, rism3d_ctx **out) {
+                const double *chi, const double *chi3, rism3d_ctx **out, bool coarse = false) {
   if (!pd || !solvent || (!solute && n > 0) || (!chi && !chi3) || !out) throw ArgFail{RISM3D_ERR_ARG, "null argument"};
   if (m < 1 || m > kMaxSites) throw ArgFail{RISM3D_ERR_ARG, "solvent sites must be 1..6"};
   if (n < 0) throw ArgFail{RISM3D_ERR_ARG, "negative solute size"};
@@ -2606,6 +2621,8 @@ int create_impl(const rism3d_problem *pd, int m, const rism3d_site *solvent, int
     bind_solute(c, n, solute);
     init_work(c);
     specialise(c, m <= 3 && !chi3);
+    if (c->stat[0] && !coarse) octant_tables<double>(c, true);
+    if (c->stat[1] && (coarse || pd->precision != RISM3D_FP64)) octant_tables<float>(c, !coarse);
     size_t need = generic_smem(c);
     allow_xy(need);
     auto allow = [&](const void *fn) { allow_smem(fn, need); };
@@ -2651,7 +2668,7 @@ int create_impl(const rism3d_problem *pd, int m, const rism3d_site *solvent, int
         for (int a = 0; a < 3; ++a) pc.N[a] = nc[a];
         pc.coarse_h = 0;
         pc.verbosity = 0;
-        create_impl(&pc, m, solvent, n, solute, chi, nullptr, &c->coarse);
+        create_impl(&pc, m, solvent, n, solute, chi, nullptr, &c->coarse, true);
         for (int a = 0; a < 3; ++a) {
           const int nf = pd->N[a], ncs = nc[a];
           c->Nc[a] = ncs;
@@ -2706,6 +2723,8 @@ int create_impl(const rism3d_problem *pd, int m, const rism3d_site *solvent, int
         c->tc_y = dalloc<float>(c->coarse->nvec);
       }
     }
+    // the context may be used from another thread, on that thread's stream
+    if (!coarse) CK(cudaStreamSynchronize(c->stream));
   } catch (...) {
     delete c;
     throw;
