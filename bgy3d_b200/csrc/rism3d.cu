@@ -3085,13 +3085,13 @@ int info_impl(rism3d_ctx *c, const double *T, rism3d_info_result *res, double *s
 
 // Device -> host copy of a large result into caller memory that is
 // pageable (a NumPy array, a PETSc Vec): the driver's pageable path runs at
-// a few GB/s there.  Here the copy is split into up to kLanes contiguous slices,
+// a few GB/s there.  Here the copy is split into kLanes contiguous slices,
 // each run by its own host thread on its own stream through two alternating
 // pinned pieces: the DMA of piece i of a slice runs while its thread copies
 // piece i-1 out, and the lanes run side by side, so the PCIe transfer and
 // the host copy (402 MB: 7 ms and, on 8 threads, 5.5 ms on the B200 hosts)
-// overlap instead of alternating.  The lane sets (at most kLanes streams and 2 x
-// kLanes pieces of kPiece bytes: 64 MB pinned; made as the copies need them)
+// overlap instead of alternating.  The lane sets (kLanes streams and 2 x kLanes
+// pieces of up to kPiece bytes: 64 MB pinned at most; grown as the copies need them)
 // come from a process-wide free list, one per concurrent caller, held until
 // exit.  Copies below 16 MB take the plain cudaMemcpy: g at 64^3 (6.3 MB) adds 0.5
 // ms to a call with it and 1.0 with the lanes' threads, t and g at 96^3 (2 x 21
@@ -3108,23 +3108,20 @@ struct LaneSet {
 std::mutex g_stage_mu;
 std::vector<LaneSet *> g_stage_free;
 
-// How a copy is split: about a megabyte per lane and two pieces of it, up to
-// kLanes lanes of kPiece pieces.
+// How a copy is split: a slice per lane, in pieces of half a slice up to kPiece.
 struct LanePlan {
-  int lanes;
   size_t piece, slice;
   explicit LanePlan(size_t bytes) {
-    lanes = (int)std::min<size_t>(kLanes, std::max<size_t>(1, bytes >> 20));
     const size_t unit = size_t(256) << 10;
-    piece = std::min(kPiece, (bytes / (2 * (size_t)lanes) + unit - 1) / unit * unit);
-    slice = ((bytes + lanes - 1) / lanes + piece - 1) / piece * piece;
+    piece = std::min(kPiece, (bytes / (2 * (size_t)kLanes) + unit - 1) / unit * unit);
+    slice = ((bytes + kLanes - 1) / kLanes + piece - 1) / piece * piece;
   }
 };
 
-// Streams, events and pinned pieces of the plan's lanes, as far as the set does
-// not hold them yet.
+// Streams, events and pinned pieces of the lanes, as far as the set does not hold
+// them yet.
 void lane_set_fit(LaneSet *ls, const LanePlan &p) {
-  for (int l = 0; l < p.lanes; ++l) {
+  for (int l = 0; l < kLanes; ++l) {
     for (int b = 0; b < 2; ++b) {
       if (ls->cap[l][b] < p.piece) {
         if (ls->buf[l][b]) CK(cudaFreeHost(ls->buf[l][b]));
@@ -3159,10 +3156,10 @@ LaneSet *lane_set_take(const LanePlan &p) {
   return ls;
 }
 
-// Runs lane(l) for l < lanes, lanes 1.. on their own threads.
-template <typename F> void run_lanes(int lanes, F &&lane) {
+// Runs lane(l) for l < kLanes, lanes 1.. on their own threads.
+template <typename F> void run_lanes(F &&lane) {
   std::vector<std::thread> th;
-  for (int l = 1; l < lanes; ++l) {
+  for (int l = 1; l < kLanes; ++l) {
     try {
       th.emplace_back(lane, l);
     } catch (const std::system_error &) {  // no thread to be had: run the lane here
@@ -3204,7 +3201,7 @@ void h2d_large(void *dst, const void *src, size_t bytes, cudaStream_t st) {
   CK(cudaEventRecord(ready, st));
   std::atomic<int> failed{0};
   const size_t slice = plan.slice, piece = plan.piece;
-  run_lanes(plan.lanes, [&](int l) {
+  run_lanes([&](int l) {
     const size_t a = std::min(bytes, (size_t)l * slice), b = std::min(bytes, a + slice);
     if (a >= b) return;
     if (cudaStreamWaitEvent(ls->st[l], ready, 0) != cudaSuccess) { failed = 1; return; }
@@ -3265,7 +3262,7 @@ void d2h_large(void *dst, const void *src, size_t bytes, cudaStream_t st) {
       prev_len = len;
     }
   };
-  run_lanes(plan.lanes, lane);
+  run_lanes(lane);
   cudaEventDestroy(ready);
   lane_set_give(ls, failed != 0);
 }
