@@ -63,12 +63,11 @@ SETTINGS = {"L": 24.0, "rho": 0.0333295, "beta": 1.6889, "closure": "KH", "rmax"
 # scale the CPU samples.
 FP64_SOLVE_EVALS = {"f": 9, "jv": 464}
 PLAIN_FP64 = {"precision": "fp64", "coarse-h": 0, "ew-forcing": 0, "krylov-restart": 30}
-# DRAM bytes (read + write) of the five FP32 passes of one Jacobian product at
-# 256^3 (x-forward 576.0, y 352.9, z 351.7, y-inverse 352.8, x-inverse
-# 574.1 MB), measured by ncu dram__bytes_read.sum + dram__bytes_write.sum on
-# the shape-specialised kernels; the z pass now also reads the 54 MB octant
-# table of chi - 1, which is not in this figure.
-JV_TRAFFIC = 2207.5e6
+# DRAM bytes (read + write) of the five FP32 passes of one Jacobian product of a
+# solve at 256^3 (x-forward 575.3, y 352.9, z 407.0, y-inverse 353.0, x-inverse
+# 573.0 MB), measured by ncu dram__bytes_read.sum + dram__bytes_write.sum on the
+# shape-specialised kernels (the z pass reads its 54 MB table of chi - 1 too).
+JV_TRAFFIC = 2261.2e6
 
 
 def workload(grid=GRID):

@@ -21,9 +21,9 @@
 // The transforms leave out the reordering between their two steps (the x
 // untangling and the z phase index the permuted order instead), the steps next
 // to W move between registers and global memory directly, and the reductions
-// are one warp per value with its partials in flight together: XY and YXI have
-// five CTA barriers each instead of ten, Z five instead of ten, and nothing
-// spills.  16 steps, us, before -> after: 32^3 298 -> 204, 36^3 364 -> 209, 48^3
+// are one warp per value with its partials in flight together: an item of XY or
+// YXI has six CTA barriers, a round of Z tiles five, and the kernels up to 48^3
+// spill nothing, the others 60 to 252 bytes a thread.  16 steps, us, before -> after: 32^3 298 -> 204, 36^3 364 -> 209, 48^3
 // 489 -> 256, 54^3 532 -> 390, 64^3 628 -> 440, 72^3 1117 -> 630, 96^3 2056 ->
 // 1463.  What is left: the grid barrier (1.3 us, three per step), two or three
 // L2 round trips per phase, and above 48^3 the rest of the basis through L2 on

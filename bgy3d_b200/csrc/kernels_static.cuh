@@ -499,7 +499,7 @@ __device__ __forceinline__ void z_tile_g(const Geo &g, typename Cx<T>::type *buf
 // barriers and the latency behind them (2.4 of 6.5 TB/s), not by memory.
 // J / F passes before -> after, us: 256^3 FP32 169 / 234 -> 127 / 201, FP64
 // 341 / 474 -> 245 / 315; 96^3 FP32 21.9 / 26.0 -> 11.0 / 17.7, FP64 32.5 /
-// 42.0 -> 17.3 / 22.4; 512^3 FP32 1923 / 4195 -> 1426 / 2512.  What is left is
+// 42.0 -> 17.3 / 22.4; 512^3 FP32 1923 / 4195 -> 1426 / 2958 (half-width tiles).  What is left is
 // the FP64 units (FP64) and twelve resident warps per SM (FP32).
 template <typename T, int N> struct ZFused {
   // R2 bounds the registers of M (m R2 complex values): at most 18 in FP32, 9

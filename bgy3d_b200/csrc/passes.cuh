@@ -27,8 +27,15 @@ namespace rism {
 #define RISM_YZ_LENS(X)                                                                                        \
   X(32) X(36) X(48) X(54) X(64) X(72) X(96) X(108) X(128) X(144) X(162) X(192) X(216) X(256) X(288) X(324) X(384) \
   X(432) X(486) X(512)
-// ... and those with the half-width and the persistent z tile beside the
-// plain one, among which the context's creation chooses by timing.
+// ... and those with the half-width (FP32) and the persistent z tile beside the
+// wide one, among which the context's creation chooses by timing; the others have
+// the wide tile alone, and the two forms have not been tried there.  J pass at
+// m = 3, us, wide / half-width / persistent: 512^3 FP32 1685 / 1426 / 1934 (F 4130
+// / 2958 / 4598), where the wide tile is 98 KB.  Below that the wide tile is the
+// fastest or within the timing's margin of the half-width one (256^3 127 / - / 261,
+// 96^3 11.1 / - / 12.3, FP64 244 and 17.4 against 406 and 19.0 persistent; 48^3
+// coarse problems have been given either).  The persistent form was never chosen:
+// two tiles per CTA halve the CTAs of an SM.
 #define RISM_Z_VARIANT_LENS(X) X(48) X(64) X(72) X(96) X(128) X(144) X(192) X(256) X(512)
 
 #define RISM_IS(L) if (n == L) return true;

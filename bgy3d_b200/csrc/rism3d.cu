@@ -3093,9 +3093,9 @@ int info_impl(rism3d_ctx *c, const double *T, rism3d_info_result *res, double *s
 // overlap instead of alternating.  The lane sets (kLanes streams and 2 x kLanes
 // pieces of up to kPiece bytes: 64 MB pinned at most; grown as the copies need them)
 // come from a process-wide free list, one per concurrent caller, held until
-// exit.  Copies below 16 MB take the plain cudaMemcpy: g at 64^3 (6.3 MB) adds 0.5
-// ms to a call with it and 1.0 with the lanes' threads, t and g at 96^3 (2 x 21
-// MB, t both ways) 5.9 and 4.6.
+// exit.  Copies below 16 MB take the plain cudaMemcpy: g at 64^3 (6.3 MB, mapped
+// pages) adds 0.4 ms to a call with it and 1.0 with the lanes' threads, t and g at
+// 96^3 (2 x 21 MB, t both ways) 5.9 and 4.6.
 constexpr size_t kPiece = size_t(4) << 20;
 constexpr int kLanes = 8;
 constexpr size_t kStagedMin = size_t(16) << 20;

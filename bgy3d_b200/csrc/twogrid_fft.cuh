@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(256) k_prolong_fx(long long rows, int Nc, int 
 // passes: small CTAs of one batch each, a thread's loads all in flight, both
 // transforms in the order of their two steps (perm_pos), the untangling of one
 // side and the packing of the other in one step between the two tiles, and the
-// last step's outputs from its registers: five CTA barriers instead of twelve.
+// last step's outputs from its registers: five CTA barriers instead of ten.
 // us, persistent CTAs of 256 threads with whole transforms -> here: 162 -> 54
 // points FP32, restriction 62 -> 34, prolongation 79 -> 63; 128 -> 48 FP64 37 ->
 // 19 and 57 -> 27.

@@ -19,7 +19,7 @@
 // its two steps (fft_static.cuh); the third gathers the kept modes from there
 // and the last writes its rows to global memory.  One read and one write of
 // each field and four barriers; with whole transforms through shared memory
-// there were ten.  At 256^3, us per launch on average of y and z: 256 -> 64 points
+// there were eight.  At 256^3, us per launch on average of y and z: 256 -> 64 points
 // 24.3 -> 11.7, 64 -> 256 18.2 -> 10.3 (4.9 TB/s of the larger field along y).
 #include <cuda_runtime.h>
 
