@@ -63,5 +63,5 @@ def test_first_evaluation_makes_no_tables(fixture_loader, N, precision):
         assert before > 0
         ctx.jacobian_t1(T, T, out=out)
         ctx.iterate_t1(T, out=out)
-        assert pool.used() == before
+        assert pool.used() <= before  # less: a context of an earlier test, collected meanwhile
         ctx.close()
